@@ -41,8 +41,8 @@
 //                per record; the runs of adjacent hit bits of a warp's 64
 //                records (one key range each) are numbered and copied 32 at
 //                a time by the whole warp;
-//   k_unique_*   match_unique: per-query bitmap (small key spaces, output
-//                comes out sorted) or per-query block radix sort + unique.
+//   k_unique_*   match_unique: per-query bitmap, read out in order (small
+//                key spaces), or per-query block radix sort + unique.
 // Result overflow is exact: the record buffer is regrown and the batch re-run
 // (the reference truncates silently at 4,194,304 hits, gpu.cu:55).
 #include "match_kernels.cuh"
@@ -313,20 +313,24 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     // ---- match_unique ----
     s.ucount.reserve(nq);
     s.uoff.reserve(size_t(nq) + 1);
-    s.ukeys.reserve(std::max<uint64_t>(total, 1));
-    const uint64_t bitmap_words = (uint64_t(t.max_key) >> 5) + 1;
-    if (bitmap_words * 4 <= 48 * 1024) {
-        k_unique_bitmap<<<nq, kUniqThreads, bitmap_words * 4, st>>>(s.keys.p, s.qoff.p, uint32_t(bitmap_words), s.ukeys.p,
-                                                                     s.ucount.p);
+    if (unique_by_bitmap(t.max_key)) {
+        const uint32_t words = (t.max_key >> 5) + 1;
+        s.ukeys.reserve(size_t(nq) * bitmap_stride(words));
+        launch_unique_mark(s.keys.p, s.qoff.p, nq, words, s.ukeys.p, s.ucount.p, s.sm_count, st);
+        exclusive_scan<uint32_t, uint64_t>(s.ucount.p, s.uoff.p, nq, s.scr, st);
+        launch_unique_expand(s.ukeys.p, s.uoff.p, nq, words, s.keys.p, st);
+        bs.launches += 3 + scan_launches(nq);  // mark, expand, readback, scan
     } else {
-        k_unique_sort<<<nq, kUniqThreads, 0, st>>>(s.keys.p, s.qoff.p, s.ukeys.p, s.ucount.p);
+        s.ukeys.reserve(std::max<uint64_t>(total, 1));
+        // the offsets' buffer holds the list of long queries until the scan
+        launch_unique_sort(s.keys.p, s.qoff.p, nq, s.ukeys.p, s.ucount.p, reinterpret_cast<uint32_t *>(s.uoff.p), t.max_key,
+                           s.sm_count, st);
+        exclusive_scan<uint32_t, uint64_t>(s.ucount.p, s.uoff.p, nq, s.scr, st);
+        // compact into s.keys (unique prefix of every segment is <= its length)
+        k_compact<<<nq, 256, 0, st>>>(s.ukeys.p, s.qoff.p, s.uoff.p, nq, s.keys.p);
+        TM_CHECK_LAUNCH();
+        bs.launches += 4 + scan_launches(nq);  // two sorts, compact, readback, scan
     }
-    TM_CHECK_LAUNCH();
-    exclusive_scan<uint32_t, uint64_t>(s.ucount.p, s.uoff.p, nq, s.scr, st);
-    // compact into s.keys (unique prefix of every segment is <= its length)
-    k_compact<<<nq, 256, 0, st>>>(s.ukeys.p, s.qoff.p, s.uoff.p, nq, s.keys.p);
-    bs.launches += 3 + scan_launches(nq);  // unique, compact, readback, scan
-    TM_CHECK_LAUNCH();
     uint64_t utotal = 0;
     std::memcpy(&utotal, read_back(s, s.uoff.p + nq, 2, nullptr, 0, st), sizeof(uint64_t));
     *d_offsets = s.uoff.p;

@@ -28,7 +28,7 @@ struct MatchScratch {
     DevBuf<uint32_t> keys;        // [total keys] grouped by query
     DevBuf<uint32_t> ucount;      // [nq]
     DevBuf<uint64_t> uoff;        // [nq + 1]
-    DevBuf<uint32_t> ukeys;       // [total unique] (also radix temp)
+    DevBuf<uint32_t> ukeys;       // match_unique: [nq] bitmaps, or [total keys] of the sorting route
     MappedBuf<uint32_t> readback; // small device results read by the host (k_readback)
     std::vector<uint32_t> h_part_count, h_chunk_off, h_item_off;
     // work-queue order of the partitions (empty: id order); set by the

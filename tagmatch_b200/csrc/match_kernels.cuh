@@ -808,156 +808,275 @@ __global__ void __launch_bounds__(kFillThreads, TM_FILL_MIN_CTAS) k_key_fill(
 // ---------------------------------------------------------------------------
 // match_unique
 // ---------------------------------------------------------------------------
-constexpr int kUniqThreads = 256;
+// Two routes.  Keys of a small space [0, 32 * words) are marked in a bitmap
+// per query, which is then read out in order; others are sorted.
+constexpr uint32_t kBitmapMaxWords = 12288;  // 48 KB of shared memory
+constexpr int kExpandThreads = 256;
 
-// Key space [0, 32 * words): a bitmap per query in shared memory; the set
-// bits read in order are the sorted unique keys.
-__global__ void __launch_bounds__(kUniqThreads) k_unique_bitmap(const uint32_t *__restrict__ keys, const uint64_t *__restrict__ qoff,
-                                                                uint32_t words, uint32_t *__restrict__ ukeys,
-                                                                uint32_t *__restrict__ ucount) {
-    extern __shared__ uint32_t bm[];
+// Words between two queries' bitmaps (16-byte rows).
+__host__ __device__ inline uint32_t bitmap_stride(uint32_t words) { return (words + 3u) & ~3u; }
+
+// Marks a query's keys in a bitmap (built in shared memory, one CTA per
+// query), stores it and counts its bits.  Keeping the bitmap (8 KB per query
+// for 16-bit keys) lets the read-out write to the result's own place once
+// the counts are known, where writing keys per query and moving them
+// together afterwards took 428 us for 20,011 queries of 2,580 keys (mark,
+// read-out and move), and the two kernels here take 98 + 163 us: reading
+// the keys, the bitmaps' way out and back and the result are about 0.7 GB.
+// A block's time is the latency of its few steps, so a batch of many
+// queries wants small blocks, eight to an SM (256 threads: 98 us against 153
+// with 512 and 209 with 1,024); where all queries are resident at once, the
+// longest result is the kernel's time and wants many threads (500 queries
+// of the ten-million table: 89, 53 and 37 us).
+__global__ void __launch_bounds__(1024) k_unique_mark(const uint32_t *__restrict__ keys,
+                                                              const uint64_t *__restrict__ qoff, uint32_t words,
+                                                              uint32_t *__restrict__ bitmaps, uint32_t *__restrict__ ucount) {
+    extern __shared__ uint4 bm4[];
+    __shared__ uint32_t s_count;
+    uint32_t *bm = reinterpret_cast<uint32_t *>(bm4);
     const uint32_t q = blockIdx.x;
     const uint64_t b = qoff[q], e = qoff[q + 1];
-    if (e == b) {
+    if (e == b) {  // no bits, and no read-out
         if (threadIdx.x == 0) ucount[q] = 0;
         return;
     }
-    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) bm[i] = 0;
+    const uint32_t rows = bitmap_stride(words) >> 2;
+    for (uint32_t i = threadIdx.x; i < rows; i += blockDim.x) bm4[i] = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x == 0) s_count = 0;
     __syncthreads();
-    // four key loads in flight per thread
-    constexpr uint32_t kU = 4;
-    uint64_t i = b + threadIdx.x;
-    for (; i + (kU - 1) * blockDim.x < e; i += kU * blockDim.x) {
-        uint32_t k[kU];
-#pragma unroll
-        for (uint32_t u = 0; u < kU; ++u) k[u] = keys[i + u * blockDim.x];
-#pragma unroll
-        for (uint32_t u = 0; u < kU; ++u) atomicOr(&bm[k[u] >> 5], 1u << (k[u] & 31));
+    auto mark = [&](uint32_t k) { atomicOr(&bm[k >> 5], 1u << (k & 31)); };
+    auto mark4 = [&](const uint4 &v) {
+        mark(v.x);
+        mark(v.y);
+        mark(v.z);
+        mark(v.w);
+    };
+    // whole groups of four keys by 16-byte loads, two in flight per thread;
+    // the ragged ends one key at a time
+    const uint64_t b4 = min(e, (b + 3) & ~uint64_t(3)), e4 = max(b4, e & ~uint64_t(3));
+    if (b + threadIdx.x < b4) mark(keys[b + threadIdx.x]);
+    if (e4 + threadIdx.x < e) mark(keys[e4 + threadIdx.x]);
+    const uint4 *k4 = reinterpret_cast<const uint4 *>(keys);
+    uint64_t i = (b4 >> 2) + threadIdx.x;
+    for (; i + blockDim.x < (e4 >> 2); i += 2 * blockDim.x) {
+        const uint4 v0 = k4[i], v1 = k4[i + blockDim.x];
+        mark4(v0);
+        mark4(v1);
     }
-    for (; i < e; i += blockDim.x) {
-        const uint32_t k = keys[i];
-        atomicOr(&bm[k >> 5], 1u << (k & 31));
-    }
+    if (i < (e4 >> 2)) mark4(k4[i]);
     __syncthreads();
-    // read-out in order: warp w takes words [w * per, (w + 1) * per), 32 at
-    // a time (lane l word l); a prefix sum over the lanes' popcounts places
-    // the round's keys, which the warp then writes 32 consecutive keys per
-    // step (each lane finds the word holding its key by a 5-step shuffle
-    // search, then the bit by halving popcounts), so the stores coalesce
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const uint32_t per = ((words + nwarps - 1) / nwarps + 31) & ~31u;
-    const uint32_t w0 = min(words, warp * per), w1 = min(words, w0 + per);
+    uint4 *out = reinterpret_cast<uint4 *>(bitmaps + size_t(q) * (rows * 4));
     uint32_t c = 0;
-    for (uint32_t w = w0 + lane; w < w1; w += 32) c += __popc(bm[w]);
-    c = __reduce_add_sync(kFull, c);
-    uint32_t tot;
-    uint32_t pos = block_excl_scan<uint32_t>(lane == 0 ? c : 0u, tot);
-    pos = __shfl_sync(kFull, pos, 0);  // this warp's first output position
-    uint64_t d = b + pos;
-    for (uint32_t r0 = w0; r0 < w1; r0 += 32) {
-        const uint32_t w = r0 + lane;
-        const uint32_t x = w < w1 ? bm[w] : 0u;
-        const uint32_t cnt = __popc(x);
-        uint32_t incl = cnt;
-#pragma unroll
-        for (int s = 1; s < 32; s <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFull, incl, s);
-            if (lane >= (unsigned)s) incl += v;
-        }
-        const uint32_t total = __shfl_sync(kFull, incl, 31);
-        for (uint32_t j0 = 0; j0 < total; j0 += 32) {
-            const uint32_t j = j0 + lane;
-            uint32_t owner = 0;
-#pragma unroll
-            for (int step = 16; step >= 1; step >>= 1) {
-                const uint32_t v = __shfl_sync(kFull, incl, owner + step - 1);
-                if (v <= j) owner += step;
-            }
-            const uint32_t oincl = __shfl_sync(kFull, incl, owner), ocnt = __shfl_sync(kFull, cnt, owner);
-            uint32_t ox = __shfl_sync(kFull, x, owner);
-            if (j < total) {
-                uint32_t rk = j - (oincl - ocnt), bit = 0;  // rank of the key's bit within the word
-#pragma unroll
-                for (int s = 16; s >= 1; s >>= 1) {
-                    const uint32_t lowc = __popc(ox & ((1u << s) - 1u));
-                    if (rk >= lowc) {
-                        rk -= lowc;
-                        ox >>= s;
-                        bit += s;
-                    }
-                }
-                ukeys[d + j] = (r0 + owner) * 32 + bit;
-            }
-        }
-        d += total;
+    for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) {
+        const uint4 v = bm4[r];
+        out[r] = v;
+        c += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
     }
-    if (threadIdx.x == 0) ucount[q] = tot;
+    c = __reduce_add_sync(kFull, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&s_count, c);
+    __syncthreads();
+    if (threadIdx.x == 0) ucount[q] = s_count;
 }
 
-// General key space: block LSD radix sort of the query's keys (4-bit digits,
-// stable per-thread ranges) through ukeys as the ping-pong buffer, then
-// unique.  Sorted keys end in ukeys[b..e); the unique prefix is compacted in
-// place.
-constexpr int kRadixBits = 4;
-constexpr int kRadixBuckets = 1 << kRadixBits;
-
-__global__ void __launch_bounds__(kUniqThreads) k_unique_sort(uint32_t *__restrict__ keys, const uint64_t *__restrict__ qoff,
-                                                              uint32_t *__restrict__ ukeys, uint32_t *__restrict__ ucount) {
-    __shared__ uint32_t s_hist[kRadixBuckets * kUniqThreads];
+// Reads a query's bitmap out in order into its place of the result (one CTA
+// per query).  Warp w takes words [w * per, (w + 1) * per), 64 at a time,
+// two per lane: a prefix sum over the lanes' popcounts places each lane's
+// keys in a per-warp buffer (11-bit positions in the round's 2,048), which
+// the warp then writes out 32 consecutive keys per store.
+__global__ void __launch_bounds__(kExpandThreads) k_unique_expand(const uint32_t *__restrict__ bitmaps,
+                                                                  const uint64_t *__restrict__ uoff, uint32_t words,
+                                                                  uint32_t *__restrict__ out) {
+    constexpr int kWarps = kExpandThreads / 32;
+    __shared__ uint16_t s_stage[kWarps][2048];
+    __shared__ uint32_t s_sum[kWarps];
     const uint32_t q = blockIdx.x;
-    const uint64_t b = qoff[q], e = qoff[q + 1];
-    const uint64_t n = e - b;
+    const uint64_t o = uoff[q];
+    if (uoff[q + 1] == o) return;
+    // rows of two words; the stride is even and its padding words are zero
+    const uint32_t rows = bitmap_stride(words) >> 1;
+    const uint2 *bm = reinterpret_cast<const uint2 *>(bitmaps) + size_t(q) * rows;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t per = ((rows + kWarps - 1) / kWarps + 31) & ~31u;
+    const uint32_t r0 = min(rows, warp * per), r1 = min(rows, r0 + per);
+    uint32_t c = 0;
+    for (uint32_t r = r0 + lane; r < r1; r += 32) {
+        const uint2 v = bm[r];
+        c += __popc(v.x) + __popc(v.y);
+    }
+    c = __reduce_add_sync(kFull, c);
+    if (lane == 0) s_sum[warp] = c;
+    __syncthreads();
+    uint32_t *d = out + o;
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k)
+        if (k < int(warp)) d += s_sum[k];
+    uint16_t *stage = s_stage[warp];
+    for (uint32_t r = r0; r < r1; r += 32) {
+        const uint2 v = r + lane < r1 ? bm[r + lane] : make_uint2(0u, 0u);
+        const uint32_t cnt = __popc(v.x) + __popc(v.y);
+        const uint32_t incl = warp_incl_scan(cnt);
+        const uint32_t total = __shfl_sync(kFull, incl, 31);
+        // from the highest key down: one find per key (two words per lane
+        // even out the lanes' counts: 163 us against 187 with one)
+        uint16_t *at = stage + incl, *end = at - cnt;
+        uint32_t x = v.y, next = v.x, base = lane * 64 + 32;
+        while (at != end) {
+            if (x == 0) {
+                x = next;
+                base -= 32;
+            }
+            const uint32_t bit = 31u - __clz(x);
+            x ^= 1u << bit;
+            *--at = uint16_t(base + bit);
+        }
+        __syncwarp();
+        for (uint32_t j = lane; j < total; j += 32) d[j] = r * 64 + stage[j];
+        __syncwarp();  // the buffer is rewritten by the next round
+        d += total;
+    }
+}
+
+// The sorting route: a stable LSD radix sort of each query's keys, 8 bits
+// per pass, one CTA per query; then the first of each run of equal keys goes
+// to ukeys[b ..).  Queries of up to SMEM_KEYS keys ping-pong between two
+// buffers in shared memory, longer ones between keys and ukeys.  Warp w
+// holds the w-th stretch of the keys, so ranks come from per-warp digit
+// counts (a prefix sum over digits, then warps) and, within 32 keys, from
+// the lanes that hold the same digit.  Most results are short, and a small
+// block per query keeps many of them resident; the queries above
+// kSortSmallKeys keys are put on a list, and a second kernel gives them 1,024
+// threads each.  Both are bound by the shared-memory steps of the ranking:
+// 2,000 queries of 1,070 32-bit keys take 82 + 83 us (the few long results),
+// where one thread per stretch with 4-bit digits in global memory took 650.
+constexpr int kSortSmallThreads = 256, kSortLargeThreads = 1024;
+constexpr uint32_t kSortSmallKeys = 4096, kSortLargeKeys = 22528;
+template <int THREADS, uint32_t SMEM_KEYS>
+constexpr int kSortSmem = int(sizeof(uint32_t)) * (THREADS / 32 * 256 + 2 * int(SMEM_KEYS));
+
+template <int THREADS, uint32_t SMEM_KEYS>
+__device__ __forceinline__ void sort_query(uint32_t *keys, uint64_t b, uint32_t n, uint32_t *ukeys, uint32_t *ucount,
+                                           int key_bits) {
+    constexpr int kWarps = THREADS / 32;
+    extern __shared__ uint32_t s_dyn[];
+    uint32_t *s_cnt = s_dyn;                 // [kWarps][256] digit counts, then output positions
+    uint32_t *s_key = s_dyn + kWarps * 256;  // [2][SMEM_KEYS]
+    __shared__ uint32_t s_part[kWarps];
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool local = n <= SMEM_KEYS;
+    uint32_t *src = keys + b, *dst = ukeys + b;
+    if (local) {
+        for (uint32_t i = tid; i < n; i += THREADS) s_key[i] = src[i];
+        src = s_key;
+        dst = s_key + SMEM_KEYS;
+    }
+    // the warp's stretch: whole groups of 32 keys
+    const uint32_t per = ((n + kWarps - 1) / kWarps + 31) & ~31u;
+    const uint32_t r0 = min(uint64_t(n), uint64_t(warp) * per), r1 = min(uint64_t(n), uint64_t(r0) + per);
+    uint32_t *cnt = s_cnt + warp * 256;
+    for (int shift = 0; shift < key_bits; shift += 8) {
+        for (int i = lane; i < 256; i += 32) cnt[i] = 0;
+        __syncthreads();  // also: the keys are in place
+        for (uint32_t i = r0 + lane; i < r1; i += 32) atomicAdd(&cnt[(src[i] >> shift) & 255u], 1u);
+        __syncthreads();
+        // positions: thread t holds digit t (256 threads); a digit that
+        // holds every key leaves the order as it is
+        uint32_t tot = 0;
+        if (tid < 256) {
+            for (int w = 0; w < kWarps; ++w) tot += s_cnt[w * 256 + tid];
+        }
+        if (__syncthreads_or(tid < 256 && tot == n)) continue;
+        uint32_t incl = 0;
+        if (tid < 256) {
+            incl = warp_incl_scan(tot);
+            if (lane == 31) s_part[warp] = incl;
+        }
+        __syncthreads();
+        if (tid < 256) {
+            uint32_t at = incl - tot;
+            for (unsigned w = 0; w < warp; ++w) at += s_part[w];
+            for (int w = 0; w < kWarps; ++w) {
+                const uint32_t c = s_cnt[w * 256 + tid];
+                s_cnt[w * 256 + tid] = at;
+                at += c;
+            }
+        }
+        __syncthreads();
+        for (uint32_t g = r0; g < r1; g += 32) {
+            const bool have = g + lane < r1;
+            const uint32_t k = have ? src[g + lane] : 0u;
+            const uint32_t d = have ? (k >> shift) & 255u : 256u + lane;  // absent lanes match no one
+            const uint32_t same = __match_any_sync(kFull, d);
+            const uint32_t below = __popc(same & ((1u << lane) - 1u));
+            uint32_t at = 0;
+            if (have) at = cnt[d];
+            __syncwarp();
+            if (have && below == 0) cnt[d] = at + __popc(same);
+            __syncwarp();
+            if (have) dst[at + below] = k;
+        }
+        __syncthreads();
+        uint32_t *t = src;
+        src = dst;
+        dst = t;
+    }
+    __syncthreads();  // key_bits may be 0 (all keys 0)
+    // first of each run of equal keys; in global memory an odd number of
+    // passes leaves the sorted keys in ukeys itself, so they go back first
+    if (!local && src != keys + b) {
+        for (uint32_t i = tid; i < n; i += THREADS) dst[i] = src[i];
+        src = dst;
+        __syncthreads();
+    }
+    uint32_t c = 0;
+    for (uint32_t g = r0; g < r1; g += 32) {
+        const uint32_t i = g + lane;
+        const bool first = i < r1 && (i == 0 || src[i] != src[i - 1]);
+        c += __popc(__ballot_sync(kFull, first));
+    }
+    if (lane == 0) s_part[warp] = c;
+    __syncthreads();
+    uint32_t at = 0, total = 0;
+    for (int w = 0; w < kWarps; ++w) {
+        if (w == int(warp)) at = total;
+        total += s_part[w];
+    }
+    for (uint32_t g = r0; g < r1; g += 32) {
+        const uint32_t i = g + lane;
+        const bool first = i < r1 && (i == 0 || src[i] != src[i - 1]);
+        const uint32_t m = __ballot_sync(kFull, first);
+        if (first) ukeys[b + at + __popc(m & ((1u << lane) - 1u))] = src[i];
+        at += __popc(m);
+    }
+    if (tid == 0) *ucount = total;
+}
+
+// long_list: [0] number of long queries (zeroed by the caller), [1 ..] the queries.
+__global__ void __launch_bounds__(kSortSmallThreads) k_unique_sort(uint32_t *keys, const uint64_t *__restrict__ qoff,
+                                                                   uint32_t *ukeys, uint32_t *__restrict__ ucount,
+                                                                   uint32_t *long_list, int key_bits) {
+    const uint32_t q = blockIdx.x;
+    const uint64_t b = qoff[q], n = qoff[q + 1] - b;  // a query's keys are counted in 32 bits
+    if (n > kSortSmallKeys) {
+        if (threadIdx.x == 0) long_list[1 + atomicAdd(&long_list[0], 1u)] = q;
+        return;
+    }
     if (n == 0) {
         if (threadIdx.x == 0) ucount[q] = 0;
         return;
     }
-    const uint64_t per = (n + blockDim.x - 1) / blockDim.x;
-    const uint64_t r0 = min(n, threadIdx.x * per), r1 = min(n, r0 + per);
-    uint32_t *src = keys + b, *dst = ukeys + b;
-    for (int shift = 0; shift < 32; shift += kRadixBits) {
-        uint32_t h[kRadixBuckets];
-#pragma unroll
-        for (int d = 0; d < kRadixBuckets; ++d) h[d] = 0;
-        for (uint64_t i = r0; i < r1; ++i) h[(src[i] >> shift) & (kRadixBuckets - 1)]++;
-#pragma unroll
-        for (int d = 0; d < kRadixBuckets; ++d) s_hist[d * kUniqThreads + threadIdx.x] = h[d];
-        __syncthreads();
-        // exclusive scan over (digit, thread) order: each thread scans a
-        // contiguous run of kRadixBuckets entries
-        uint32_t run[kRadixBuckets];
-        uint32_t sum = 0;
-#pragma unroll
-        for (int d = 0; d < kRadixBuckets; ++d) {
-            run[d] = s_hist[threadIdx.x * kRadixBuckets + d];
-            sum += run[d];
-        }
-        uint32_t tot;
-        uint32_t pre = block_excl_scan<uint32_t>(sum, tot);
-#pragma unroll
-        for (int d = 0; d < kRadixBuckets; ++d) {
-            s_hist[threadIdx.x * kRadixBuckets + d] = pre;
-            pre += run[d];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int d = 0; d < kRadixBuckets; ++d) h[d] = s_hist[d * kUniqThreads + threadIdx.x];
-        for (uint64_t i = r0; i < r1; ++i) {
-            const uint32_t k = src[i];
-            dst[h[(k >> shift) & (kRadixBuckets - 1)]++] = k;
-        }
-        __syncthreads();
-        uint32_t *tmp = src;
-        src = dst;
-        dst = tmp;
+    sort_query<kSortSmallThreads, kSortSmallKeys>(keys, b, uint32_t(n), ukeys, &ucount[q], key_bits);
+}
+
+__global__ void __launch_bounds__(kSortLargeThreads) k_unique_sort_long(uint32_t *keys, const uint64_t *__restrict__ qoff,
+                                                                        uint32_t *ukeys, uint32_t *__restrict__ ucount,
+                                                                        const uint32_t *long_list, int key_bits) {
+    const uint32_t count = long_list[0];
+    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+        const uint32_t q = long_list[1 + i];
+        const uint64_t b = qoff[q];
+        sort_query<kSortLargeThreads, kSortLargeKeys>(keys, b, uint32_t(qoff[q + 1] - b), ukeys, &ucount[q], key_bits);
+        __syncthreads();  // the shared buffers are rewritten for the next query
     }
-    // 8 passes: the sorted keys are back in keys[b..e); unique into ukeys.
-    uint32_t c = 0;
-    for (uint64_t i = r0; i < r1; ++i) c += (i == 0 || src[i] != src[i - 1]);
-    uint32_t tot;
-    uint32_t pos = block_excl_scan<uint32_t>(c, tot);
-    for (uint64_t i = r0; i < r1; ++i)
-        if (i == 0 || src[i] != src[i - 1]) ukeys[b + pos++] = src[i];
-    if (threadIdx.x == 0) ucount[q] = tot;
 }
 
 __global__ void k_compact(const uint32_t *__restrict__ ukeys, const uint64_t *__restrict__ qoff,
@@ -975,6 +1094,40 @@ __global__ void k_compact(const uint32_t *__restrict__ ukeys, const uint64_t *__
         for (int u = 0; u < 4; ++u) out[dst + i + u * blockDim.x] = v[u];
     }
     for (; i < n; i += blockDim.x) out[dst + i] = ukeys[src + i];
+}
+
+// Whether match_unique marks bitmaps: the key space fits one.
+inline bool unique_by_bitmap(uint32_t max_key) { return (max_key >> 5) + 1 <= kBitmapMaxWords; }
+
+inline void launch_unique_mark(const uint32_t *keys, const uint64_t *qoff, uint32_t nq, uint32_t words, uint32_t *bitmaps,
+                               uint32_t *ucount, int sm_count, cudaStream_t st) {
+    // the bitmap and the count may together exceed the default 48 KB
+    TM_CUDA(cudaFuncSetAttribute(k_unique_mark, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBitmapMaxWords * 4)));
+    const unsigned threads = nq <= 4u * unsigned(sm_count) ? 1024 : 256;
+    k_unique_mark<<<nq, threads, bitmap_stride(words) * 4, st>>>(keys, qoff, words, bitmaps, ucount);
+    TM_CHECK_LAUNCH();
+}
+
+inline void launch_unique_expand(const uint32_t *bitmaps, const uint64_t *uoff, uint32_t nq, uint32_t words, uint32_t *out,
+                                 cudaStream_t st) {
+    k_unique_expand<<<nq, kExpandThreads, 0, st>>>(bitmaps, uoff, words, out);
+    TM_CHECK_LAUNCH();
+}
+
+// Sorts every query's keys and leaves the different ones in ukeys[qoff ..).
+// long_list: scratch of nq + 1 words.
+inline void launch_unique_sort(uint32_t *keys, const uint64_t *qoff, uint32_t nq, uint32_t *ukeys, uint32_t *ucount,
+                               uint32_t *long_list, uint32_t max_key, int sm_count, cudaStream_t st) {
+    int key_bits = 0;
+    while (key_bits < 32 && (max_key >> key_bits)) ++key_bits;
+    constexpr int small = kSortSmem<kSortSmallThreads, kSortSmallKeys>, large = kSortSmem<kSortLargeThreads, kSortLargeKeys>;
+    TM_CUDA(cudaFuncSetAttribute(k_unique_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, large));
+    TM_CUDA(cudaMemsetAsync(long_list, 0, sizeof(uint32_t), st));
+    k_unique_sort<<<nq, kSortSmallThreads, small, st>>>(keys, qoff, ukeys, ucount, long_list, key_bits);
+    TM_CHECK_LAUNCH();
+    k_unique_sort_long<<<std::min<uint32_t>(nq, uint32_t(sm_count)), kSortLargeThreads, large, st>>>(keys, qoff, ukeys, ucount,
+                                                                                                     long_list, key_bits);
+    TM_CHECK_LAUNCH();
 }
 
 // Copies na words at a, then nb words at b, into mapped pinned host memory

@@ -223,24 +223,26 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
         TM_CUDA(cudaStreamSynchronize(st));
         return;
     }
-    // match_unique: keys into one arena buffer, de-duplicated into a second
-    // one (the hit records' space when it is large enough: they are no
-    // longer read once the keys are filled), then compacted into the
-    // caller's output
-    const uint64_t bitmap_words = (uint64_t(t.max_key) >> 5) + 1;
-    const bool bitmap = bitmap_words * 4 <= 48 * 1024;
+    // match_unique: keys into one arena buffer; the bitmaps, or the sorting
+    // route's second key buffer, into another (the hit records' space when
+    // it is large enough: they are no longer read once the keys are filled).
+    // Bitmaps that fit nowhere leave the sorting route, whose buffer is as
+    // long as the keys.
     uint32_t *keys = ar.take<uint32_t>(std::max<uint64_t>(total, 1), "match_unique keys");
-    uint32_t *ukeys = std::max<uint64_t>(total, 1) * sizeof(uint32_t) <= hc[1] * sizeof(HitRec)
-                          ? reinterpret_cast<uint32_t *>(recs)
-                          : ar.take<uint32_t>(std::max<uint64_t>(total, 1), "match_unique keys");
+    const uint32_t words = (t.max_key >> 5) + 1;
+    const size_t bitmap_bytes = size_t(nq) * bitmap_stride(words) * sizeof(uint32_t);
+    const size_t key_bytes = std::max<uint64_t>(total, 1) * sizeof(uint32_t), rec_bytes = hc[1] * sizeof(HitRec);
+    const bool bitmap = unique_by_bitmap(t.max_key) && bitmap_bytes <= std::max(rec_bytes, ar.left());
+    const size_t second_bytes = bitmap ? bitmap_bytes : key_bytes;
+    uint32_t *second = second_bytes <= rec_bytes ? reinterpret_cast<uint32_t *>(recs)
+                                                 : ar.take<uint32_t>(second_bytes / sizeof(uint32_t), "match_unique keys");
     k_key_fill<<<gblocks, kFillThreads, 0, st>>>(recs, counters, t.slot_key_off.p, t.tile_keys.p, t.keys.p, qoff, qcursor, keys);
     TM_CHECK_LAUNCH();
     if (bitmap) {
-        k_unique_bitmap<<<nq, kUniqThreads, bitmap_words * 4, st>>>(keys, qoff, uint32_t(bitmap_words), ukeys, ucount);
+        launch_unique_mark(keys, qoff, nq, words, second, ucount, sms, st);
     } else {
-        k_unique_sort<<<nq, kUniqThreads, 0, st>>>(keys, qoff, ukeys, ucount);
+        launch_unique_sort(keys, qoff, nq, second, ucount, reinterpret_cast<uint32_t *>(d_out_offsets), t.max_key, sms, st);
     }
-    TM_CHECK_LAUNCH();
     scan_fixed<uint32_t, uint64_t>(ucount, d_out_offsets, nq, sums, offs, st);
     uint64_t utotal = 0;
     TM_CUDA(cudaMemcpyAsync(&utotal, d_out_offsets + nq, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
@@ -248,8 +250,12 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     *n_keys = utotal;
     if (utotal > capacity)
         throw Error(TM_ERR_CAPACITY, "output key buffer too small: " + std::to_string(utotal) + " keys needed");
-    k_compact<<<nq, 256, 0, st>>>(ukeys, qoff, d_out_offsets, nq, d_out_keys);
-    TM_CHECK_LAUNCH();
+    if (bitmap) {
+        launch_unique_expand(second, d_out_offsets, nq, words, d_out_keys, st);
+    } else {
+        k_compact<<<nq, 256, 0, st>>>(second, qoff, d_out_offsets, nq, d_out_keys);
+        TM_CHECK_LAUNCH();
+    }
     TM_CUDA(cudaStreamSynchronize(st));
 }
 
