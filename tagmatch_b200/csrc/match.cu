@@ -12,16 +12,18 @@
 //
 // Here the whole path runs on the device for a batch of queries:
 //   k_route      one thread per query tests the partition masks (held in
-//                shared memory); CTA-local counts reserve queue space with
-//                one global atomic per (CTA, partition); queue records are
-//                32 bytes (6 query words, query id, pad);
-//   host plan    work items = (partition, group of four 256-query chunks,
-//                segment of the partition's tiles), offsets computed on the
-//                host from the per-partition counts, partitions in id order
-//                or in the order the learned cost model gives;
-//   k_slices     per 256-query chunk, bit-sliced "lacks bit b" masks:
-//                Z[b] bit j set when query j of the chunk lacks bit b
-//                (192 x 256 bits, ballot per bit);
+//                shared memory): a vote per (partition, 32 queries) gives
+//                the routing matrix, a bit per (partition, query), and the
+//                partitions' counts;
+//   k_plan       queue, chunk and work item offsets from the counts; work
+//                items = (partition, group of four 256-query chunks, segment
+//                of the partition's tiles), partitions in id order or in the
+//                order the learned cost model gives;
+//   k_fill_queues  each partition's queue from its row of the matrix:
+//                records of 32 bytes (6 query words, query id, pad) and, per
+//                256-query chunk, bit-sliced "lacks bit b" masks: Z[b] bit j
+//                set when query j of the chunk lacks bit b (192 x 256 bits,
+//                bit transposes of the query words);
 //   k_match      persistent CTAs take items from an atomic counter.  Each
 //                item's query records are staged into shared memory by bulk
 //                TMA copies (cp.async.bulk + mbarrier), one per chunk; the
@@ -55,20 +57,17 @@ namespace tmb {
 MatchScratch &MatchScratch::operator=(MatchScratch &&o) noexcept {
     if (this == &o) return *this;
     queries = std::move(o.queries);
-    part_count = std::move(o.part_count);
+    zeroed = std::move(o.zeroed);
+    rows = std::move(o.rows);
     part_off = std::move(o.part_off);
-    part_cursor = std::move(o.part_cursor);
     queue = std::move(o.queue);
     item_off = std::move(o.item_off);
     chunk_off = std::move(o.chunk_off);
     slices = std::move(o.slices);
     work = std::move(o.work);
     keys16 = std::move(o.keys16);
-    counters = std::move(o.counters);
     recs = std::move(o.recs);
-    qkeys = std::move(o.qkeys);
     qoff = std::move(o.qoff);
-    qcursor = std::move(o.qcursor);
     keys = std::move(o.keys);
     ucount = std::move(o.ucount);
     uoff = std::move(o.uoff);
@@ -115,20 +114,32 @@ const uint16_t *narrow_keys(const uint32_t *d_keys, uint64_t n, MatchScratch &s,
     return s.keys16.p;
 }
 
-// Reads na words at a and nb words at b (device memory) into s.readback
+// Reads na words at a, nb at b and nc at c (device memory) into s.readback
 // and waits for them: a kernel writes them to mapped host memory, so the
 // read does not wait for copies that other streams have queued on the copy
 // engines (the host pipeline keeps multi-GB result copies in flight while
 // the next batch is matched).
-const uint32_t *read_back(MatchScratch &s, const void *a, uint32_t na, const void *b, uint32_t nb, cudaStream_t st) {
-    s.readback.reserve(size_t(na) + nb);
-    const unsigned blocks = std::min(64u, (na + nb + 255) / 256);
-    k_readback<<<std::max(blocks, 1u), 256, 0, st>>>(static_cast<const uint32_t *>(a), na,
-                                                     static_cast<const uint32_t *>(b), nb, s.readback.d);
+const uint32_t *read_back(MatchScratch &s, const void *a, uint32_t na, const void *b, uint32_t nb, const void *c, uint32_t nc,
+                          cudaStream_t st) {
+    const uint32_t n = na + nb + nc;
+    s.readback.reserve(n);
+    const unsigned blocks = std::min(64u, (n + 255) / 256);
+    k_readback<<<std::max(blocks, 1u), 256, 0, st>>>(static_cast<const uint32_t *>(a), na, static_cast<const uint32_t *>(b), nb,
+                                                     static_cast<const uint32_t *>(c), nc, s.readback.d);
     TM_CHECK_LAUNCH();
     TM_CUDA(cudaStreamSynchronize(st));
     return s.readback.h;
 }
+
+// Queues and slices are allocated by their exact sizes, which takes a wait
+// for the partitions' counts in the middle of the batch; when even every
+// query in every partition would need no more than this, that is allocated
+// and the wait saved (it is paid by small batches: about 10 us of 180 for
+// one query).
+constexpr size_t kQueueAheadBytes = size_t(256) << 20;
+// Largest routing matrix kept at once; larger ones are made in windows of
+// partitions, twice.
+constexpr size_t kRowWords = size_t(64) << 18;
 
 MatchScratch::~MatchScratch() {
     if (ev_begin) cudaEventDestroy(ev_begin);
@@ -145,9 +156,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     }
     const uint32_t P = t.n_parts;
     BatchStats bs;
-    s.qkeys.reserve(std::max<uint32_t>(nq, 1));
     s.qoff.reserve(size_t(nq) + 1);
-    s.counters.reserve(4);
     if (nq == 0 || P == 0 || t.n_tiles == 0) {
         TM_CUDA(cudaMemsetAsync(s.qoff.p, 0, (size_t(nq) + 1) * sizeof(uint64_t), st));
         TM_CUDA(cudaStreamSynchronize(st));
@@ -160,92 +169,85 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
         return;
     }
     // ---- routing ----
-    s.part_count.reserve(P);
-    s.part_off.reserve(size_t(P) + 1);
-    s.part_cursor.reserve(P);
-    TM_CUDA(cudaMemsetAsync(s.part_count.p, 0, P * sizeof(uint32_t), st));
-    TM_CUDA(cudaMemsetAsync(s.part_cursor.p, 0, P * sizeof(uint32_t), st));
-    const unsigned rblocks = blocks_for(nq, kRouteThreads);
-    for (uint32_t p0 = 0; p0 < P; p0 += kMaxRouteParts) {
-        const uint32_t pw = std::min(kMaxRouteParts, P - p0);
-        const size_t smem = size_t(pw) * (kWords + 2) * sizeof(uint32_t);
-        k_route<false><<<rblocks, kRouteThreads, smem, st>>>(d_queries, nq, t.part_mask.p, p0, pw, s.part_count.p, nullptr,
-                                                            nullptr, nullptr);
-        TM_CHECK_LAUNCH();
-    }
-    exclusive_scan<uint32_t, uint32_t>(s.part_count.p, s.part_off.p, P, s.scr, st);
-    s.h_part_count.resize(P);
-    const uint32_t *rb = read_back(s, s.part_count.p, P, s.part_off.p + P, 1, st);
-    std::copy(rb, rb + P, s.h_part_count.begin());
-    const uint32_t routed = rb[P];
-    bs.routed = routed;
-    for (uint32_t p = 0; p < P; ++p) bs.dense += uint64_t(s.h_part_count[p]) * t.h_part_size[p];
-    const uint32_t windows = (P + kMaxRouteParts - 1) / kMaxRouteParts;
-    bs.launches += 2 * windows + 3 + scan_launches(P);  // route x2, readback, slices, match, scan
-    s.queue.reserve(size_t(std::max<uint32_t>(routed, 1)) * kQueueWords + kChunk * kQueueWords);
-    for (uint32_t p0 = 0; p0 < P; p0 += kMaxRouteParts) {
-        const uint32_t pw = std::min(kMaxRouteParts, P - p0);
-        const size_t smem = size_t(pw) * (kWords + 2) * sizeof(uint32_t);
-        k_route<true><<<rblocks, kRouteThreads, smem, st>>>(d_queries, nq, t.part_mask.p, p0, pw, nullptr, s.part_off.p,
-                                                           s.part_cursor.p, s.queue.p);
-        TM_CHECK_LAUNCH();
-    }
-    // ---- plan: chunks and work items per partition (host, from the counts) ----
-    s.h_chunk_off.resize(size_t(P) + 1);
-    s.h_item_off.resize(size_t(P) + 1);
-    uint32_t chunks = 0, items = 0;
-    for (uint32_t p = 0; p < P; ++p) {
-        s.h_chunk_off[p] = chunks;
-        chunks += (s.h_part_count[p] + kChunk - 1) / kChunk;
-    }
-    // work items in the queue order: partition id order, or the order the
-    // learned cost model gives (most expensive items first)
+    // everything that starts at zero, cleared together
+    const uint32_t groups = route_groups(nq);
+    const size_t n_zero = 8 + size_t(P) * (1 + groups) + 2 * size_t(nq);
+    s.zeroed.reserve(n_zero);
+    unsigned long long *counters = reinterpret_cast<unsigned long long *>(s.zeroed.p);
+    uint32_t *qkeys = s.zeroed.p + 8, *qcursor = qkeys + nq, *part_count = qcursor + nq, *group_count = part_count + P;
+    TM_CUDA(cudaMemsetAsync(s.zeroed.p, 0, n_zero * sizeof(uint32_t), st));
+    const uint32_t window = route_window(P, nq, kRowWords), windows = (P + window - 1) / window;
+    s.rows.reserve(size_t(window) * route_row_words(nq));
+    for (uint32_t p0 = 0; p0 < P; p0 += window)
+        launch_route(true, d_queries, nq, t, p0, std::min(P, p0 + window), s.rows.p, part_count, group_count, st);
+    // ---- plan: queue positions, chunks and work items ----
     const bool ordered = s.part_order.size() == P;
-    for (uint32_t pos = 0; pos < P; ++pos) {
-        const uint32_t p = ordered ? s.part_order[pos] : pos;
-        s.h_item_off[pos] = items;
-        // an item: kItemChunks chunks of the partition x one tile segment
-        const uint32_t ng = (s.h_part_count[p] + kItemQueries - 1) / kItemQueries;
-        const uint32_t nt = t.h_part_tiles[p + 1] - t.h_part_tiles[p];
-        items += ng * ((nt + s.seg_tiles - 1) / s.seg_tiles);
-    }
-    s.h_chunk_off[P] = chunks;
-    s.h_item_off[P] = items;
     if (ordered) {
         s.d_part_order.reserve(P);
         TM_CUDA(cudaMemcpyAsync(s.d_part_order.p, s.part_order.data(), size_t(P) * 4, cudaMemcpyHostToDevice, st));
     }
-    s.item_off.reserve(size_t(P) + 1);
+    const uint32_t *order = ordered ? s.d_part_order.p : nullptr;
+    s.part_off.reserve(size_t(P) + 1);
     s.chunk_off.reserve(size_t(P) + 1);
-    TM_CUDA(cudaMemcpyAsync(s.item_off.p, s.h_item_off.data(), (size_t(P) + 1) * 4, cudaMemcpyHostToDevice, st));
-    TM_CUDA(cudaMemcpyAsync(s.chunk_off.p, s.h_chunk_off.data(), (size_t(P) + 1) * 4, cudaMemcpyHostToDevice, st));
-    s.slices.reserve(size_t(std::max<uint32_t>(chunks, 1)) * kSliceWords);
-    if (chunks) {
-        k_slices<<<chunks, kChunk, 0, st>>>(s.queue.p, s.part_off.p, s.part_count.p, s.chunk_off.p, P, s.slices.p);
-        TM_CHECK_LAUNCH();
+    s.item_off.reserve(size_t(P) + 1);
+    k_plan<<<1, kPlanThreads, 0, st>>>(part_count, t.part_tile_begin.p, order, P, s.seg_tiles, s.part_off.p, s.chunk_off.p,
+                                       s.item_off.p);
+    TM_CHECK_LAUNCH();
+    // the host's copy of the plan, once the counts are back
+    uint32_t items = 0, chunks = 0;
+    auto host_plan = [&](const uint32_t *counts) {
+        s.h_part_count.assign(counts, counts + P);
+        s.h_item_off.resize(size_t(P) + 1);
+        for (uint32_t pos = 0; pos < P; ++pos) {
+            bs.routed += counts[pos];
+            bs.dense += uint64_t(counts[pos]) * t.h_part_size[pos];
+            chunks += (counts[pos] + kChunk - 1) / kChunk;
+            // work items in the queue order: partition id order, or the order
+            // the learned cost model gives (most expensive items first)
+            const uint32_t p = ordered ? s.part_order[pos] : pos;
+            s.h_item_off[pos] = items;
+            // an item: kItemChunks chunks of the partition x one tile segment
+            const uint32_t ng = (counts[p] + kItemQueries - 1) / kItemQueries;
+            const uint32_t nt = t.h_part_tiles[p + 1] - t.h_part_tiles[p];
+            items += ng * ((nt + s.seg_tiles - 1) / s.seg_tiles);
+        }
+        s.h_item_off[P] = items;
+        bs.items = items;
+    };
+    size_t queue_len = size_t(nq) * P, slice_len = size_t(P) * blocks_for(nq, kChunk);
+    const bool ahead = !s.record_items && queue_len * kQueueWords * 4 + slice_len * kSliceWords * 4 <= kQueueAheadBytes;
+    if (!ahead) {
+        host_plan(read_back(s, part_count, P, nullptr, 0, nullptr, 0, st));
+        queue_len = bs.routed;
+        slice_len = chunks;
     }
-    bs.items = items;
+    s.queue.reserve((queue_len + kChunk) * kQueueWords);
+    s.slices.reserve(std::max<size_t>(slice_len, 1) * kSliceWords);
+    launch_fill_queues(d_queries, nq, t, window, s.rows.p, part_count, group_count, s.part_off.p, s.chunk_off.p, s.queue.p,
+                       s.slices.p, st);
+    // route, queues (both again per window), plan, match, scan, readback
+    bs.launches += windows * (windows > 1 ? 3 : 2) + 3 + scan_launches(nq) + (ahead ? 0u : 1u);
     // ---- match (regrow and re-run on pair overflow) ----
     if (s.rec_cap_hint == 0) s.rec_cap_hint = size_t(nq) * 512 + (1u << 20);
     s.recs.reserve(s.rec_cap_hint);
     unsigned long long hc[4] = {0, 0, 0, 0};
+    uint64_t total = 0;
     for (int attempt = 0;; ++attempt) {
-        TM_CUDA(cudaMemsetAsync(s.counters.p, 0, 4 * sizeof(unsigned long long), st));
+        // counters and the per-query key totals, which the subset test sums
+        // itself, are zero at first
+        if (attempt) TM_CUDA(cudaMemsetAsync(s.zeroed.p, 0, (8 + size_t(nq)) * sizeof(uint32_t), st));
         static const bool work_counters = std::getenv("TM_WORK_COUNTERS") != nullptr;
         if (work_counters) {
             s.work.reserve(8);
             TM_CUDA(cudaMemsetAsync(s.work.p, 0, 8 * sizeof(unsigned long long), st));
         }
-        // per-query key totals are summed by the subset test itself
-        TM_CUDA(cudaMemsetAsync(s.qkeys.p, 0, nq * sizeof(uint32_t), st));
         if (s.record_items) {
             s.item_stats.reserve(2 * size_t(std::max<uint32_t>(items, 1)));
             TM_CUDA(cudaMemsetAsync(s.item_stats.p, 0, 2 * size_t(items) * sizeof(unsigned long long), st));
         }
-        MatchArgs a{t.tile_words.p, t.tile_info.p, t.tile_keys.p, t.slot_key_off.p, t.part_tile_begin.p, s.part_count.p,
-                    s.part_off.p, s.item_off.p, s.chunk_off.p, s.queue.p, s.slices.p, P, s.seg_tiles, s.counters.p,
-                    s.recs.p, (unsigned long long)s.recs.cap, s.qkeys.p, fpl_trip_cost(),
-                    ordered ? s.d_part_order.p : nullptr, s.record_items ? s.item_stats.p : nullptr,
+        MatchArgs a{t.tile_words.p, t.tile_info.p, t.tile_keys.p, t.slot_key_off.p, t.part_tile_begin.p, part_count,
+                    s.part_off.p, s.item_off.p, s.chunk_off.p, s.queue.p, s.slices.p, P, s.seg_tiles, counters,
+                    s.recs.p, (unsigned long long)s.recs.cap, qkeys, fpl_trip_cost(), order, s.record_items ? s.item_stats.p : nullptr,
                     work_counters ? s.work.p : nullptr};
         if (match_begin && attempt == 0) TM_CUDA(cudaEventRecord(match_begin, st));
         if (s.profile) {
@@ -260,7 +262,11 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
         TM_CHECK_LAUNCH();
         if (s.profile) TM_CUDA(cudaEventRecord(s.ev_end, st));
         if (match_end) TM_CUDA(cudaEventRecord(match_end, st));
-        std::memcpy(hc, read_back(s, s.counters.p, 8, nullptr, 0, st), 4 * sizeof(unsigned long long));
+        exclusive_scan<uint32_t, uint64_t>(qkeys, s.qoff.p, nq, s.scr, st);
+        const uint32_t *rb = read_back(s, counters, 8, s.qoff.p + nq, 2, part_count, ahead && !attempt ? P : 0u, st);
+        std::memcpy(hc, rb, sizeof(hc));
+        std::memcpy(&total, rb + 8, sizeof(total));
+        if (ahead && !attempt) host_plan(rb + 10);
         if (hc[2]) throw Error(TM_ERR_TIMEOUT, "match kernel: bounded wait for the query copy expired");
         if (work_counters) {
             unsigned long long w[8];
@@ -290,16 +296,11 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     }
     // ---- keys ----
     const unsigned gblocks = std::max(1u, std::min(blocks_for(hc[1], kFillThreads * kFillPerLane), unsigned(s.sm_count) * 16));
-    // record-count readback, fill, key-total readback; each retry: match + readback
-    bs.launches += 3 + scan_launches(nq) + 2 * uint32_t(bs.retries);
-    exclusive_scan<uint32_t, uint64_t>(s.qkeys.p, s.qoff.p, nq, s.scr, st);
-    uint64_t total = 0;
-    std::memcpy(&total, read_back(s, s.qoff.p + nq, 2, nullptr, 0, st), sizeof(uint64_t));
+    // fill; each retry: match, scan, readback
+    bs.launches += 1 + (2 + scan_launches(nq)) * uint32_t(bs.retries);
     bs.pairs = hc[3];
     s.keys.reserve(std::max<uint64_t>(total, 1));
-    s.qcursor.reserve(nq);
-    TM_CUDA(cudaMemsetAsync(s.qcursor.p, 0, nq * sizeof(uint32_t), st));
-    k_key_fill<<<gblocks, kFillThreads, 0, st>>>(s.recs.p, s.counters.p, t.slot_key_off.p, t.tile_keys.p, t.keys.p, s.qoff.p, s.qcursor.p, s.keys.p);
+    k_key_fill<<<gblocks, kFillThreads, 0, st>>>(s.recs.p, counters, t.slot_key_off.p, t.tile_keys.p, t.keys.p, s.qoff.p, qcursor, s.keys.p);
     TM_CHECK_LAUNCH();
     if (!unique) {
         TM_CUDA(cudaStreamSynchronize(st));
@@ -332,7 +333,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
         bs.launches += 4 + scan_launches(nq);  // two sorts, compact, readback, scan
     }
     uint64_t utotal = 0;
-    std::memcpy(&utotal, read_back(s, s.uoff.p + nq, 2, nullptr, 0, st), sizeof(uint64_t));
+    std::memcpy(&utotal, read_back(s, s.uoff.p + nq, 2, nullptr, 0, nullptr, 0, st), sizeof(uint64_t));
     *d_offsets = s.uoff.p;
     *d_keys = s.keys.p;
     *n_keys = utotal;

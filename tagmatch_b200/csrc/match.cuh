@@ -11,26 +11,26 @@ constexpr int kSegTiles = 128;  // default tiles per work item (tm_autotune may 
 // Device scratch for one in-flight batch (grow-only).
 struct MatchScratch {
     DevBuf<uint32_t> queries;     // [nq][6] staged host input
-    DevBuf<uint32_t> part_count;  // [P]
+    // what a batch needs zeroed: [8] counters (as 64 bits: [0] work item, [1]
+    // hit records, [2] error flags, [3] pairs), [nq] key totals, [nq] key
+    // cursors, [P] queries per partition, [P][groups] the same per group
+    DevBuf<uint32_t> zeroed;
+    DevBuf<uint32_t> rows;        // routing matrix: [P][nq / 32] bits
     DevBuf<uint32_t> part_off;    // [P + 1]
-    DevBuf<uint32_t> part_cursor; // [P]
     DevBuf<uint32_t> queue;       // [routed][8]
     DevBuf<uint32_t> item_off;    // [P + 1] work items per partition (prefix)
     DevBuf<uint32_t> chunk_off;   // [P + 1] 256-query chunks per partition (prefix)
     DevBuf<uint32_t> slices;      // [chunks][192][8] bit-sliced "lacks bit" masks
     DevBuf<unsigned long long> work;  // optional kernel work counters
     DevBuf<uint16_t> keys16;          // keys narrowed for the host transfer
-    DevBuf<unsigned long long> counters;  // [0] work item, [1] hit records, [2] error flags, [3] pairs
     DevBuf<HitRec> recs;          // hit records of the subset test
-    DevBuf<uint32_t> qkeys;       // [nq]
     DevBuf<uint64_t> qoff;        // [nq + 1]
-    DevBuf<uint32_t> qcursor;     // [nq]
     DevBuf<uint32_t> keys;        // [total keys] grouped by query
     DevBuf<uint32_t> ucount;      // [nq]
     DevBuf<uint64_t> uoff;        // [nq + 1]
     DevBuf<uint32_t> ukeys;       // match_unique: [nq] bitmaps, or [total keys] of the sorting route
     MappedBuf<uint32_t> readback; // small device results read by the host (k_readback)
-    std::vector<uint32_t> h_part_count, h_chunk_off, h_item_off;
+    std::vector<uint32_t> h_part_count, h_item_off;
     // work-queue order of the partitions (empty: id order); set by the
     // engine from the learned cost model
     std::vector<uint32_t> part_order;

@@ -9,14 +9,12 @@
 namespace tmb {
 namespace {
 
-constexpr int kRouteThreads = 256;
 constexpr int kMatchThreads = 256;
 constexpr int kMatchWarps = kMatchThreads / 32;
 constexpr int kWarpRecs = 64;  // staged hit records per warp (1 KB)
 constexpr int kQuad = 1;       // tiles a warp selects candidates for at once (for all chunks of its item)
 constexpr int kTileLanes = 32 / kQuad;  // lanes per tile in the selection: 8 words x kItemChunks chunks
 static_assert(kTileLanes == 8 * kItemChunks, "selection lanes");
-constexpr uint32_t kMaxRouteParts = 1536;  // partition masks per routing window (48 KB of shared memory)
 constexpr unsigned long long kSpinLimit = 1ull << 26;
 
 inline unsigned blocks_for(size_t n, unsigned t) { return unsigned((n + t - 1) / t); }
@@ -24,93 +22,239 @@ inline unsigned blocks_for(size_t n, unsigned t) { return unsigned((n + t - 1) /
 // ---------------------------------------------------------------------------
 // Routing
 // ---------------------------------------------------------------------------
-template <bool FILL>
+constexpr int kSliceRows = kBits + 1;  // 192 bit rows + the all-zero padding row
+constexpr int kSliceWords = kSliceRows * 8;  // 193 x 256 bits
+
+constexpr int kRouteThreads = 256;        // queries per routing CTA
+constexpr uint32_t kRouteParts = 64;      // partition masks per routing CTA
+constexpr uint32_t kGroupQueries = 8192;  // queries per count group: 256 words of a partition's routing row
+constexpr uint32_t kFillRanks = 2048;     // queue positions per queue-filling CTA (8 chunks)
+constexpr int kPlanThreads = 1024;
+
+// Words of one partition's routing row (a bit per query, whole CTAs).
+__host__ __device__ inline uint32_t route_row_words(uint32_t nq) { return (nq + kRouteThreads - 1) / kRouteThreads * 8; }
+// Count groups per partition (0: the partition's count is enough).
+__host__ __device__ inline uint32_t route_groups(uint32_t nq) {
+    return nq <= kGroupQueries ? 0u : (nq + kGroupQueries - 1) / kGroupQueries;
+}
+
+// Routing matrix of partitions [p0, p1): bit l of rows[p - p0][w] is set when
+// partition p's mask is a subset of query 32 w + l.  Lane = query; the masks
+// are read from shared memory, one vote per (partition, 32 queries).  COUNT
+// adds each partition's queries to part_count (and to the partition's count
+// of every kGroupQueries queries), zeroed by the caller.  Queries x
+// partitions spread over the grid, so that a few queries or a few
+// partitions still make enough CTAs: testing all partitions in one CTA per
+// 256 queries, twice, took 500 of the 1,390 us of 4,096 queries on 2,082
+// partitions.
+template <bool COUNT>
 __global__ void __launch_bounds__(kRouteThreads) k_route(const uint32_t *__restrict__ queries, uint32_t nq,
-                                                         const uint32_t *__restrict__ part_mask, uint32_t p0, uint32_t pw,
-                                                         uint32_t *__restrict__ part_count, const uint32_t *__restrict__ part_off,
-                                                         uint32_t *__restrict__ part_cursor, uint32_t *__restrict__ queue) {
-    extern __shared__ uint32_t sm[];
-    uint32_t *s_mask = sm;                          // [pw][6]
-    uint32_t *s_cnt = sm + size_t(pw) * kWords;     // [pw]
-    uint32_t *s_base = s_cnt + pw;                  // [pw] (FILL)
-    for (uint32_t i = threadIdx.x; i < pw; i += blockDim.x) {
-#pragma unroll
-        for (int k = 0; k < kWords; ++k) s_mask[i * kWords + k] = part_mask[size_t(p0 + i) * 8 + k];
-        s_cnt[i] = 0;
-    }
-    __syncthreads();
-    const uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = qi < nq;
+                                                         const uint32_t *__restrict__ part_mask, uint32_t p0, uint32_t p1,
+                                                         uint32_t *__restrict__ rows, uint32_t *__restrict__ part_count,
+                                                         uint32_t *__restrict__ group_count) {
+    __shared__ uint4 s_mask[kRouteParts * 2];
+    __shared__ uint32_t s_row[32][kRouteThreads / 32 + 1];
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t pb = p0 + blockIdx.y * kRouteParts;
+    const uint32_t np = min(kRouteParts, p1 - pb);
+    const uint4 *masks = reinterpret_cast<const uint4 *>(part_mask);
+    for (uint32_t i = tid; i < 2 * np; i += kRouteThreads) s_mask[i] = masks[size_t(pb) * 2 + i];
+    const uint32_t qi = blockIdx.x * kRouteThreads + tid;
     uint32_t q[kWords];
 #pragma unroll
-    for (int k = 0; k < kWords; ++k) q[k] = valid ? queries[size_t(qi) * kWords + k] : 0u;
-    if (valid) {
-        for (uint32_t i = 0; i < pw; ++i)
-            if (subset6(s_mask + i * kWords, q)) atomicAdd(&s_cnt[i], 1u);
-    }
+    for (int k = 0; k < kWords; ++k) q[k] = qi < nq ? queries[size_t(qi) * kWords + k] : 0u;
+    const uint32_t live = __ballot_sync(kFull, qi < nq);
+    const uint32_t row_words = route_row_words(nq), groups = route_groups(nq);
     __syncthreads();
-    if constexpr (!FILL) {
-        for (uint32_t i = threadIdx.x; i < pw; i += blockDim.x)
-            if (s_cnt[i]) atomicAdd(&part_count[p0 + i], s_cnt[i]);
-    } else {
-    for (uint32_t i = threadIdx.x; i < pw; i += blockDim.x) {
-        const uint32_t c = s_cnt[i];
-        s_base[i] = c ? part_off[p0 + i] + atomicAdd(&part_cursor[p0 + i], c) : 0u;
-        s_cnt[i] = 0;
-    }
-    __syncthreads();
-    if (valid) {
-        for (uint32_t i = 0; i < pw; ++i) {
-            if (subset6(s_mask + i * kWords, q)) {
-                const uint32_t pos = s_base[i] + atomicAdd(&s_cnt[i], 1u);
-                uint4 *dst = reinterpret_cast<uint4 *>(queue + size_t(pos) * kQueueWords);
-                dst[0] = make_uint4(q[0], q[1], q[2], q[3]);
-                dst[1] = make_uint4(q[4], q[5], qi, 0u);
+    for (uint32_t b = 0; b < np; b += 32) {
+        uint32_t mine = 0;  // partition pb + b + lane: the warp's queries
+        const uint32_t nb = min(32u, np - b);
+        for (uint32_t i = 0; i < nb; ++i) {
+            const uint4 m0 = s_mask[2 * (b + i)], m1 = s_mask[2 * (b + i) + 1];
+            uint32_t x = m0.x & ~q[0];
+            x = andnot_or(m0.y, q[1], x);
+            x = andnot_or(m0.z, q[2], x);
+            x = andnot_or(m0.w, q[3], x);
+            x = andnot_or(m1.x, q[4], x);
+            x = andnot_or(m1.y, q[5], x);
+            const uint32_t hit = __ballot_sync(kFull, x == 0);
+            if (lane == i) mine = hit;
+        }
+        s_row[lane][warp] = mine & live;
+        __syncthreads();
+        // eight threads per partition write its 256 queries' words
+        const uint32_t r = tid >> 3, w = tid & 7, p = pb + b + r;
+        const uint32_t word = s_row[r][w];
+        if (r < nb) rows[size_t(p - p0) * row_words + blockIdx.x * 8 + w] = word;
+        if (COUNT) {
+            uint32_t c = __popc(word);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) c += __shfl_xor_sync(kFull, c, o);
+            if (w == 0 && r < nb && c) {
+                atomicAdd(&part_count[p], c);
+                if (groups) atomicAdd(&group_count[size_t(p) * groups + blockIdx.x * kRouteThreads / kGroupQueries], c);
             }
         }
-    }
+        __syncthreads();
     }
 }
 
-constexpr int kSliceRows = kBits + 1;  // 192 bit rows + the all-zero padding row
-
-// Bit-sliced query masks of one 256-query chunk: z[b * 8 + w] bit l is set
-// when query 32 w + l of the chunk lacks filter bit b, or does not exist
-// (so an absent query is never a candidate).
-__global__ void __launch_bounds__(kChunk) k_slices(const uint32_t *__restrict__ queue, const uint32_t *__restrict__ part_off,
-                                                   const uint32_t *__restrict__ part_count,
-                                                   const uint32_t *__restrict__ chunk_off, uint32_t n_parts,
-                                                   uint32_t *__restrict__ slices) {
-    const uint32_t c = blockIdx.x;
-    uint32_t lo = 0, hi = n_parts;  // partition of this chunk: chunk_off[lo] <= c < chunk_off[lo + 1]
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (chunk_off[mid] <= c) lo = mid;
-        else hi = mid;
-    }
-    const uint32_t p = lo;
-    const uint32_t chunk = c - chunk_off[p];
-    const uint32_t nq = min((uint32_t)kChunk, part_count[p] - chunk * kChunk);
-    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t j = w * 32 + lane;
-    uint32_t q[kWords];
-    const bool valid = j < nq;
-#pragma unroll
-    for (int k = 0; k < kWords; ++k)
-        q[k] = valid ? queue[size_t(part_off[p] + chunk * kChunk + j) * kQueueWords + k] : 0u;
-    uint32_t mine[kWords];
-#pragma unroll
-    for (int k = 0; k < kWords; ++k) {
-#pragma unroll
-        for (int b = 0; b < 32; ++b) {
-            const uint32_t z = __ballot_sync(kFull, !valid || !((q[k] >> b) & 1u));
-            if (lane == (unsigned)b) mine[k] = z;
+// Offsets of the work plan from the partitions' counts, one CTA: queue
+// positions, 256-query chunks, and work items (groups of kItemChunks chunks
+// x tile segments), the items over queue positions (order: the partition at
+// each position; null: id order).
+__global__ void __launch_bounds__(kPlanThreads) k_plan(const uint32_t *__restrict__ part_count,
+                                                       const uint32_t *__restrict__ part_tile_begin,
+                                                       const uint32_t *__restrict__ order, uint32_t n_parts,
+                                                       uint32_t seg_tiles, uint32_t *__restrict__ part_off,
+                                                       uint32_t *__restrict__ chunk_off, uint32_t *__restrict__ item_off) {
+    __shared__ uint32_t s_sum[3][kPlanThreads / 32];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t base[3] = {0, 0, 0};
+    for (uint32_t t0 = 0; t0 < n_parts; t0 += kPlanThreads) {
+        const uint32_t pos = t0 + threadIdx.x;
+        uint32_t v[3] = {0, 0, 0};
+        if (pos < n_parts) {
+            v[0] = part_count[pos];
+            v[1] = (v[0] + kChunk - 1) / kChunk;
+            const uint32_t p = order ? order[pos] : pos;
+            const uint32_t nt = part_tile_begin[p + 1] - part_tile_begin[p];
+            v[2] = ((part_count[p] + kItemQueries - 1) / kItemQueries) * ((nt + seg_tiles - 1) / seg_tiles);
         }
-    }
-    uint32_t *zc = slices + size_t(c) * kSliceRows * 8;
+        uint32_t incl[3];
 #pragma unroll
-    for (int k = 0; k < kWords; ++k) zc[(k * 32 + lane) * 8 + w] = mine[k];
-    if (lane == 0) zc[kNoBit * 8 + w] = 0u;  // the padding row: no query lacks it
+        for (int k = 0; k < 3; ++k) {
+            incl[k] = warp_incl_scan(v[k]);
+            if (lane == 31) s_sum[k][warp] = incl[k];
+        }
+        __syncthreads();
+        if (warp < 3) s_sum[warp][lane] = warp_incl_scan(s_sum[warp][lane]);
+        __syncthreads();
+        uint32_t *out[3] = {part_off, chunk_off, item_off};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if (pos < n_parts) out[k][pos] = base[k] + (warp ? s_sum[k][warp - 1] : 0u) + incl[k] - v[k];
+            base[k] += s_sum[k][kPlanThreads / 32 - 1];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        part_off[n_parts] = base[0];
+        chunk_off[n_parts] = base[1];
+        item_off[n_parts] = base[2];
+    }
+}
+
+// 32 x 32 bit transpose over a warp: bit j of lane i <- bit i of lane j.
+// Five rounds exchange the off-diagonal blocks of 16, 8, .. 1 bits.
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t x, unsigned lane) {
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        constexpr uint32_t kLow[5] = {0x55555555u, 0x33333333u, 0x0F0F0F0Fu, 0x00FF00FFu, 0x0000FFFFu};
+        const uint32_t low = kLow[s == 1 ? 0 : s == 2 ? 1 : s == 4 ? 2 : s == 8 ? 3 : 4];
+        const uint32_t y = __shfl_xor_sync(kFull, x, s);
+        const bool up = (lane & s) != 0;
+        const uint32_t keep = up ? ~low : low;
+        x = (x & keep) | (__funnelshift_l(y, y, up ? 32 - s : s) & ~keep);
+    }
+    return x;
+}
+
+// Fills the partitions' queues from their routing rows (partitions
+// [p0, p0 + gridDim.x)): CTA (p, y) takes the queries of positions
+// [2048 y, 2048 y + 2048), finds them in the row (counts per group, then a
+// prefix sum over a group's words), and per 256-query chunk writes the queue
+// records (32 bytes: 6 query words, query id, pad) and the chunk's
+// bit-sliced masks: z[b * 8 + w] bit l is set when query 32 w + l of the chunk
+// lacks filter bit b, or does not exist (so an absent query is never a
+// candidate).  The slices are bit transposes of the query words, 15
+// instructions per 32 x 32 bits where a vote per bit took 128; they leave
+// through shared memory (words swizzled over the banks) in whole lines.
+__global__ void __launch_bounds__(kChunk) k_fill_queues(const uint32_t *__restrict__ queries, uint32_t nq,
+                                                        const uint32_t *__restrict__ rows, uint32_t p0,
+                                                        const uint32_t *__restrict__ part_count,
+                                                        const uint32_t *__restrict__ group_count,
+                                                        const uint32_t *__restrict__ part_off,
+                                                        const uint32_t *__restrict__ chunk_off, uint32_t *__restrict__ queue,
+                                                        uint32_t *__restrict__ slices) {
+    static_assert(kScanThreads == kChunk && kGroupQueries == 32 * kChunk, "one routing word per thread and group");
+    __shared__ uint32_t s_list[kFillRanks];
+    __shared__ uint32_t s_z[kSliceWords];
+    const uint32_t p = p0 + blockIdx.x, r0 = blockIdx.y * kFillRanks, count = part_count[p];
+    if (r0 >= count) return;
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t r1 = min(count, r0 + kFillRanks);
+    const uint32_t row_words = route_row_words(nq), groups = route_groups(nq);
+    const uint32_t *row = rows + size_t(blockIdx.x) * row_words;
+    uint32_t at = 0;  // position of the group's first query
+    for (uint32_t w0 = 0, g = 0; w0 < row_words && at < r1; w0 += kChunk, ++g) {
+        const uint32_t in_group = groups ? group_count[size_t(p) * groups + g] : count;
+        if (at + in_group > r0) {
+            uint32_t x = w0 + tid < row_words ? row[w0 + tid] : 0u;
+            uint32_t total;
+            uint32_t r = at + block_excl_scan<uint32_t>(__popc(x), total);
+            for (; x && r < r1; ++r) {
+                if (r >= r0) s_list[r - r0] = (w0 + tid) * 32 + __ffs(x) - 1;
+                x &= x - 1;
+            }
+        }
+        at += in_group;
+    }
+    __syncthreads();
+    const uint32_t qbase = part_off[p] + r0, c0 = chunk_off[p] + r0 / kChunk;
+    for (uint32_t j0 = 0; r0 + j0 < r1; j0 += kChunk) {
+        const uint32_t j = j0 + tid;
+        uint32_t q[kWords] = {0, 0, 0, 0, 0, 0};
+        if (r0 + j < r1) {
+            const uint32_t qi = s_list[j];
+#pragma unroll
+            for (int k = 0; k < kWords; ++k) q[k] = queries[size_t(qi) * kWords + k];
+            uint4 *dst = reinterpret_cast<uint4 *>(queue + size_t(qbase + j) * kQueueWords);
+            dst[0] = make_uint4(q[0], q[1], q[2], q[3]);
+            dst[1] = make_uint4(q[4], q[5], qi, 0u);
+        }
+#pragma unroll
+        for (int k = 0; k < kWords; ++k) {
+            const uint32_t row_z = k * 32 + lane;
+            s_z[row_z * 8 + (warp ^ ((row_z >> 2) & 7))] = ~warp_transpose(q[k], lane);
+        }
+        if (tid < 8) s_z[kNoBit * 8 + tid] = 0u;  // the padding row: no query lacks it
+        __syncthreads();
+        uint32_t *zc = slices + size_t(c0 + j0 / kChunk) * kSliceWords;
+        for (uint32_t i = tid; i < uint32_t(kSliceWords); i += kChunk)
+            zc[i] = s_z[i < kNoBit * 8 ? (i & ~7u) + ((i ^ (i >> 5)) & 7u) : i];
+        __syncthreads();
+    }
+}
+
+// Partitions per routing window, and windows: a window's rows take at most
+// `words` words.
+inline uint32_t route_window(uint32_t n_parts, uint32_t nq, size_t words) {
+    const size_t fit = words / route_row_words(nq) / 32 * 32;
+    return uint32_t(std::min<size_t>(n_parts, std::max<size_t>(fit, 32)));
+}
+
+// Routing rows of partitions [p0, p1), counted or not.
+inline void launch_route(bool count, const uint32_t *d_queries, uint32_t nq, const DevTable &t, uint32_t p0, uint32_t p1,
+                         uint32_t *rows, uint32_t *part_count, uint32_t *group_count, cudaStream_t st) {
+    const dim3 grid(blocks_for(nq, kRouteThreads), blocks_for(p1 - p0, kRouteParts));
+    if (count) k_route<true><<<grid, kRouteThreads, 0, st>>>(d_queries, nq, t.part_mask.p, p0, p1, rows, part_count, group_count);
+    else k_route<false><<<grid, kRouteThreads, 0, st>>>(d_queries, nq, t.part_mask.p, p0, p1, rows, part_count, group_count);
+    TM_CHECK_LAUNCH();
+}
+
+// Queues and slices of every partition, a window of routing rows at a time.
+// rows holds the only window's rows already, or each window's are made again.
+inline void launch_fill_queues(const uint32_t *d_queries, uint32_t nq, const DevTable &t, uint32_t window, uint32_t *rows,
+                               uint32_t *part_count, uint32_t *group_count, const uint32_t *part_off,
+                               const uint32_t *chunk_off, uint32_t *queue, uint32_t *slices, cudaStream_t st) {
+    for (uint32_t p0 = 0; p0 < t.n_parts; p0 += window) {
+        const uint32_t p1 = std::min(t.n_parts, p0 + window);
+        if (window < t.n_parts) launch_route(false, d_queries, nq, t, p0, p1, rows, part_count, group_count, st);
+        k_fill_queues<<<dim3(p1 - p0, blocks_for(nq, kFillRanks)), kChunk, 0, st>>>(
+            d_queries, nq, rows, p0, part_count, group_count, part_off, chunk_off, queue, slices);
+        TM_CHECK_LAUNCH();
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -217,8 +361,6 @@ struct MatchArgs {
     // its tile visits with at most 16 candidates; null when off
     unsigned long long *work;
 };
-
-constexpr int kSliceWords = kSliceRows * 8;  // 193 x 256 bits
 
 // A chunk's staged query records (8 KB).  kPadQuery marks the gather's
 // padding records (no query).
@@ -1130,14 +1272,14 @@ inline void launch_unique_sort(uint32_t *keys, const uint64_t *qoff, uint32_t nq
     TM_CHECK_LAUNCH();
 }
 
-// Copies na words at a, then nb words at b, into mapped pinned host memory
+// Copies na words at a, nb at b, then nc at c, into mapped pinned host memory
 // (dst is its device view).  Used for the few numbers the host needs in the
 // middle of a batch (queue sizes, pair and key totals).
 __global__ void k_readback(const uint32_t *__restrict__ a, uint32_t na, const uint32_t *__restrict__ b, uint32_t nb,
-                           uint32_t *__restrict__ dst) {
-    const uint32_t n = na + nb;
+                           const uint32_t *__restrict__ c, uint32_t nc, uint32_t *__restrict__ dst) {
+    const uint32_t n = na + nb + nc;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        dst[i] = i < na ? a[i] : b[i - na];
+        dst[i] = i < na ? a[i] : i < na + nb ? b[i - na] : c[i - na - nb];
 }
 
 // Keys narrowed to 16 bits for the trip to the host (tables whose largest

@@ -80,19 +80,6 @@ struct Arena {
     }
 };
 
-// Work-plan counts per partition: 256-query chunks, and work items (groups
-// of kItemChunks chunks x tile segments).
-__global__ void k_plan_counts(const uint32_t *__restrict__ part_count, const uint32_t *__restrict__ part_tile_begin,
-                              uint32_t n_parts, uint32_t seg_tiles, uint32_t *__restrict__ nchunks,
-                              uint32_t *__restrict__ nitems) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n_parts) return;
-    const uint32_t c = (part_count[p] + kChunk - 1) / kChunk;
-    const uint32_t nt = part_tile_begin[p + 1] - part_tile_begin[p];
-    nchunks[p] = c;
-    nitems[p] = ((c + kItemChunks - 1) / kItemChunks) * ((nt + seg_tiles - 1) / seg_tiles);
-}
-
 // Exclusive scan with block sums held in the arena (up to 2048 x 2048 elements).
 template <class Tin, class Tout>
 void scan_fixed(const Tin *in, Tout *out, size_t n, uint64_t *sums, uint64_t *offs, cudaStream_t st) {
@@ -138,38 +125,36 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     }
     unsigned long long *counters = ar.take<unsigned long long>(4, "counters");
     uint32_t *part_count = ar.take<uint32_t>(P, "partition counts");
-    uint32_t *part_cursor = ar.take<uint32_t>(P, "partition cursors");
     uint32_t *part_off = ar.take<uint32_t>(size_t(P) + 1, "partition offsets");
-    uint32_t *nchunks = ar.take<uint32_t>(P, "plan");
-    uint32_t *nitems = ar.take<uint32_t>(P, "plan");
     uint32_t *chunk_off = ar.take<uint32_t>(size_t(P) + 1, "plan");
     uint32_t *item_off = ar.take<uint32_t>(size_t(P) + 1, "plan");
-    uint64_t *sums = ar.take<uint64_t>(kScanTile, "scan");
-    uint64_t *offs = ar.take<uint64_t>(kScanTile + 1, "scan");
+    // block sums of a scan over at most kNoAllocMaxQueries
+    constexpr size_t kScanBlocks = (kNoAllocMaxQueries + kScanTile - 1) / kScanTile;
+    uint64_t *sums = ar.take<uint64_t>(kScanBlocks, "scan");
+    uint64_t *offs = ar.take<uint64_t>(kScanBlocks + 1, "scan");
     uint32_t *qkeys = ar.take<uint32_t>(nq, "query key counts");
     uint32_t *qcursor = ar.take<uint32_t>(nq, "query cursors");
     uint64_t *qoff = ar.take<uint64_t>(size_t(nq) + 1, "query offsets");
     uint32_t *ucount = ar.take<uint32_t>(nq, "unique counts");
     TM_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), st));
     TM_CUDA(cudaMemsetAsync(part_count, 0, P * sizeof(uint32_t), st));
-    TM_CUDA(cudaMemsetAsync(part_cursor, 0, P * sizeof(uint32_t), st));
     TM_CUDA(cudaMemsetAsync(qkeys, 0, nq * sizeof(uint32_t), st));
     TM_CUDA(cudaMemsetAsync(qcursor, 0, nq * sizeof(uint32_t), st));
 
-    // routing counts and the work plan
-    const unsigned rblocks = blocks_for(nq, kRouteThreads);
-    for (uint32_t p0 = 0; p0 < P; p0 += kMaxRouteParts) {
-        const uint32_t pw = std::min(kMaxRouteParts, P - p0);
-        const size_t smem = size_t(pw) * (kWords + 2) * sizeof(uint32_t);
-        k_route<false><<<rblocks, kRouteThreads, smem, st>>>(d_queries, nq, t.part_mask.p, p0, pw, part_count, nullptr,
-                                                            nullptr, nullptr);
-        TM_CHECK_LAUNCH();
-    }
-    scan_fixed<uint32_t, uint32_t>(part_count, part_off, P, sums, offs, st);
-    k_plan_counts<<<blocks_for(P, 256), 256, 0, st>>>(part_count, t.part_tile_begin.p, P, seg_tiles, nchunks, nitems);
+    // routing counts and the work plan; the routing rows lie in what the
+    // queues leave free, as many partitions at a time as fit (the first
+    // pass's rows stay where the whole matrix fits with the queues)
+    static_assert(kNoAllocMaxQueries <= kGroupQueries, "no counts per group");
+    const size_t row_words = route_row_words(nq);
+    uint32_t window = route_window(P, nq, ar.left() / sizeof(uint32_t));
+    auto rows_at_end = [&](uint32_t parts) {
+        return reinterpret_cast<uint32_t *>(ar.base + kNoAllocScratchBytes) - size_t(parts) * row_words;
+    };
+    uint32_t *rows = rows_at_end(window);
+    for (uint32_t p0 = 0; p0 < P; p0 += window)
+        launch_route(true, d_queries, nq, t, p0, std::min(P, p0 + window), rows, part_count, nullptr, st);
+    k_plan<<<1, kPlanThreads, 0, st>>>(part_count, t.part_tile_begin.p, nullptr, P, seg_tiles, part_off, chunk_off, item_off);
     TM_CHECK_LAUNCH();
-    scan_fixed<uint32_t, uint32_t>(nchunks, chunk_off, P, sums, offs, st);
-    scan_fixed<uint32_t, uint32_t>(nitems, item_off, P, sums, offs, st);
     uint32_t routed = 0, chunks = 0;
     TM_CUDA(cudaMemcpyAsync(&routed, part_off + P, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     TM_CUDA(cudaMemcpyAsync(&chunks, chunk_off + P, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -177,17 +162,14 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
 
     uint32_t *queue = ar.take<uint32_t>(size_t(std::max<uint32_t>(routed, 1)) * kQueueWords, "partition queues");
     uint32_t *slices = ar.take<uint32_t>(size_t(std::max<uint32_t>(chunks, 1)) * kSliceWords, "query slices");
-    for (uint32_t p0 = 0; p0 < P; p0 += kMaxRouteParts) {
-        const uint32_t pw = std::min(kMaxRouteParts, P - p0);
-        const size_t smem = size_t(pw) * (kWords + 2) * sizeof(uint32_t);
-        k_route<true><<<rblocks, kRouteThreads, smem, st>>>(d_queries, nq, t.part_mask.p, p0, pw, nullptr, part_off,
-                                                           part_cursor, queue);
-        TM_CHECK_LAUNCH();
+    const uint32_t fits = route_window(P, nq, ar.left() / sizeof(uint32_t));
+    if (fits < window) {
+        window = fits;
+        rows = rows_at_end(window);
+        if (ar.left() < size_t(window) * row_words * sizeof(uint32_t))
+            throw Error(TM_ERR_CAPACITY, "no-allocation scratch exhausted at the routing rows; split the batch");
     }
-    if (chunks) {
-        k_slices<<<chunks, kChunk, 0, st>>>(queue, part_off, part_count, chunk_off, P, slices);
-        TM_CHECK_LAUNCH();
-    }
+    launch_fill_queues(d_queries, nq, t, window, rows, part_count, nullptr, part_off, chunk_off, queue, slices, st);
     // hit records fill what is left of the array; after the match the part
     // they did not use goes to the keys
     const size_t rec_room = ar.left() / sizeof(HitRec);
