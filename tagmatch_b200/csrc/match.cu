@@ -221,10 +221,11 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
         queue_len = bs.routed;
         slice_len = chunks;
     }
-    s.queue.reserve((queue_len + kChunk) * kQueueWords);
+    s.queue.reserve(std::max<size_t>(queue_len, 1) * 2);
+    uint4 *queue_lo = s.queue.p, *queue_hi = s.queue.p + queue_len;
     s.slices.reserve(std::max<size_t>(slice_len, 1) * kSliceWords);
-    launch_fill_queues(d_queries, nq, t, window, s.rows.p, part_count, group_count, s.part_off.p, s.chunk_off.p, s.queue.p,
-                       s.slices.p, st);
+    launch_fill_queues(d_queries, nq, t, window, s.rows.p, part_count, group_count, s.part_off.p, s.chunk_off.p, queue_lo,
+                       queue_hi, s.slices.p, st);
     // route, queues (both again per window), plan, match, scan, readback
     bs.launches += windows * (windows > 1 ? 3 : 2) + 3 + scan_launches(nq) + (ahead ? 0u : 1u);
     // ---- match (regrow and re-run on pair overflow) ----
@@ -246,7 +247,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
             TM_CUDA(cudaMemsetAsync(s.item_stats.p, 0, 2 * size_t(items) * sizeof(unsigned long long), st));
         }
         MatchArgs a{t.tile_words.p, t.tile_info.p, t.tile_keys.p, t.slot_key_off.p, t.part_tile_begin.p, part_count,
-                    s.part_off.p, s.item_off.p, s.chunk_off.p, s.queue.p, s.slices.p, P, s.seg_tiles, counters,
+                    s.part_off.p, s.item_off.p, s.chunk_off.p, queue_lo, queue_hi, s.slices.p, P, s.seg_tiles, counters,
                     s.recs.p, (unsigned long long)s.recs.cap, qkeys, fpl_trip_cost(), order, s.record_items ? s.item_stats.p : nullptr,
                     work_counters ? s.work.p : nullptr};
         if (match_begin && attempt == 0) TM_CUDA(cudaEventRecord(match_begin, st));

@@ -17,7 +17,7 @@ struct MatchScratch {
     DevBuf<uint32_t> zeroed;
     DevBuf<uint32_t> rows;        // routing matrix: [P][nq / 32] bits
     DevBuf<uint32_t> part_off;    // [P + 1]
-    DevBuf<uint32_t> queue;       // [routed][8]
+    DevBuf<uint4> queue;          // two planes of [routed]
     DevBuf<uint32_t> item_off;    // [P + 1] work items per partition (prefix)
     DevBuf<uint32_t> chunk_off;   // [P + 1] 256-query chunks per partition (prefix)
     DevBuf<uint32_t> slices;      // [chunks][192][8] bit-sliced "lacks bit" masks

@@ -12,9 +12,7 @@ namespace {
 constexpr int kMatchThreads = 256;
 constexpr int kMatchWarps = kMatchThreads / 32;
 constexpr int kWarpRecs = 64;  // staged hit records per warp (1 KB)
-constexpr int kQuad = 1;       // tiles a warp selects candidates for at once (for all chunks of its item)
-constexpr int kTileLanes = 32 / kQuad;  // lanes per tile in the selection: 8 words x kItemChunks chunks
-static_assert(kTileLanes == 8 * kItemChunks, "selection lanes");
+static_assert(kItemQueries == 1024, "an item's queries are 32 words of 32, one per lane");
 constexpr unsigned long long kSpinLimit = 1ull << 26;
 
 inline unsigned blocks_for(size_t n, unsigned t) { return unsigned((n + t - 1) / t); }
@@ -164,8 +162,8 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, unsigned lane) {
 // [p0, p0 + gridDim.x)): CTA (p, y) takes the queries of positions
 // [2048 y, 2048 y + 2048), finds them in the row (counts per group, then a
 // prefix sum over a group's words), and per 256-query chunk writes the queue
-// records (32 bytes: 6 query words, query id, pad) and the chunk's
-// bit-sliced masks: z[b * 8 + w] bit l is set when query 32 w + l of the chunk
+// records (words 0 .. 3 in one plane; words 4 and 5, the query id and a pad
+// in the other) and the chunk's bit-sliced masks: z[b * 8 + w] bit l is set when query 32 w + l of the chunk
 // lacks filter bit b, or does not exist (so an absent query is never a
 // candidate).  The slices are bit transposes of the query words, 15
 // instructions per 32 x 32 bits where a vote per bit took 128; they leave
@@ -175,7 +173,8 @@ __global__ void __launch_bounds__(kChunk) k_fill_queues(const uint32_t *__restri
                                                         const uint32_t *__restrict__ part_count,
                                                         const uint32_t *__restrict__ group_count,
                                                         const uint32_t *__restrict__ part_off,
-                                                        const uint32_t *__restrict__ chunk_off, uint32_t *__restrict__ queue,
+                                                        const uint32_t *__restrict__ chunk_off,
+                                                        uint4 *__restrict__ queue_lo, uint4 *__restrict__ queue_hi,
                                                         uint32_t *__restrict__ slices) {
     static_assert(kScanThreads == kChunk && kGroupQueries == 32 * kChunk, "one routing word per thread and group");
     __shared__ uint32_t s_list[kFillRanks];
@@ -209,9 +208,8 @@ __global__ void __launch_bounds__(kChunk) k_fill_queues(const uint32_t *__restri
             const uint32_t qi = s_list[j];
 #pragma unroll
             for (int k = 0; k < kWords; ++k) q[k] = queries[size_t(qi) * kWords + k];
-            uint4 *dst = reinterpret_cast<uint4 *>(queue + size_t(qbase + j) * kQueueWords);
-            dst[0] = make_uint4(q[0], q[1], q[2], q[3]);
-            dst[1] = make_uint4(q[4], q[5], qi, 0u);
+            queue_lo[size_t(qbase) + j] = make_uint4(q[0], q[1], q[2], q[3]);
+            queue_hi[size_t(qbase) + j] = make_uint4(q[4], q[5], qi, 0u);
         }
 #pragma unroll
         for (int k = 0; k < kWords; ++k) {
@@ -247,12 +245,12 @@ inline void launch_route(bool count, const uint32_t *d_queries, uint32_t nq, con
 // rows holds the only window's rows already, or each window's are made again.
 inline void launch_fill_queues(const uint32_t *d_queries, uint32_t nq, const DevTable &t, uint32_t window, uint32_t *rows,
                                uint32_t *part_count, uint32_t *group_count, const uint32_t *part_off,
-                               const uint32_t *chunk_off, uint32_t *queue, uint32_t *slices, cudaStream_t st) {
+                               const uint32_t *chunk_off, uint4 *queue_lo, uint4 *queue_hi, uint32_t *slices, cudaStream_t st) {
     for (uint32_t p0 = 0; p0 < t.n_parts; p0 += window) {
         const uint32_t p1 = std::min(t.n_parts, p0 + window);
         if (window < t.n_parts) launch_route(false, d_queries, nq, t, p0, p1, rows, part_count, group_count, st);
         k_fill_queues<<<dim3(p1 - p0, blocks_for(nq, kFillRanks)), kChunk, 0, st>>>(
-            d_queries, nq, rows, p0, part_count, group_count, part_off, chunk_off, queue, slices);
+            d_queries, nq, rows, p0, part_count, group_count, part_off, chunk_off, queue_lo, queue_hi, slices);
         TM_CHECK_LAUNCH();
     }
 }
@@ -337,7 +335,7 @@ struct MatchArgs {
     const uint32_t *part_off;
     const uint32_t *item_off;
     const uint32_t *chunk_off;
-    const uint32_t *queue;
+    const uint4 *queue_lo, *queue_hi;
     const uint32_t *slices;
     uint32_t n_parts;
     uint32_t seg_tiles;            // tiles per work item
@@ -362,19 +360,20 @@ struct MatchArgs {
     unsigned long long *work;
 };
 
-// A chunk's staged query records (8 KB).  kPadQuery marks the gather's
-// padding records (no query).
+// Marks the gather's padding records (no query).
 constexpr uint32_t kPadQuery = 0xFFFFFFFFu;
-constexpr int kStageWords = kChunk * kQueueWords;
 
 // Shared memory of one matcher CTA (dynamic; ~54 KB, 4 CTAs per SM).
 struct MatchSmem {
-    uint32_t q[kItemChunks][kStageWords];                // the item's chunks' query records
+    // the item's query records; in two planes, so that the 16-byte reads of
+    // scattered records spread over all banks (in 32-byte records each half
+    // had every other 16 bytes to itself)
+    uint4 q_lo[kItemQueries], q_hi[kItemQueries];
     HitRec rec[kMatchWarps][kWarpRecs];                  // staged hit records per warp
-    // candidate lists per warp and tile: the chunks' candidates in chunk
-    // order (query index in its chunk), padded to a multiple of 4
-    uint8_t list[kMatchWarps][kQuad][kItemQueries + 8];
-    TileKeys tk[kMatchWarps][kQuad];                     // key-count planes of the warp's tiles
+    // candidate lists per warp: 1024 / T bytes for each of the T tiles it
+    // selects for at once, the chunks' candidates in chunk order (query index
+    // in its chunk), padded to a multiple of 4
+    uint8_t list[kMatchWarps][kItemQueries];
     uint4 tf[kMatchWarps][kWords][kTile / 4];            // a warp's tile: word k of filters 4 g .. 4 g + 3
     uint64_t full, empty;
     uint32_t item;
@@ -389,23 +388,32 @@ static_assert(4 * (sizeof(MatchSmem) + 1024) <= 228 * 1024, "the matcher's share
 
 // Moves a warp's n staged records to the global record buffer (one atomic
 // reserves their place; past the capacity they are only counted, and the
-// host re-runs the batch with a larger buffer).
-__device__ __forceinline__ void flush_recs(HitRec *buf, uint32_t n, const MatchArgs &a, unsigned lane) {
+// host re-runs the batch with a larger buffer).  The records' key counts,
+// the per-query key totals and the pair count are made here, with every lane
+// at work, instead of at the few lanes that hit when a record is staged.
+// Returns the lane's matching pairs.
+__device__ __forceinline__ uint32_t flush_recs(HitRec *buf, uint32_t n, const MatchArgs &a, unsigned lane) {
     __syncwarp();
     unsigned long long base = 0;
     if (lane == 0) base = atomicAdd(&a.counters[1], (unsigned long long)n);
     base = __shfl_sync(kFull, base, 0);
-    if (base + n <= a.rec_cap) {
-        for (uint32_t i = lane; i < n; i += 32) a.recs[base + i] = buf[i];
+    const bool fits = base + n <= a.rec_cap;
+    uint32_t pairs = 0;
+    for (uint32_t i = lane; i < n; i += 32) {
+        HitRec r = buf[i];
+        r.nkeys = mask_keys(a.tile_keys[r.tile], r.mask, a.slot_key_off, r.tile);
+        atomicAdd(&a.qkeys[r.query], r.nkeys);
+        pairs += __popc(r.mask);
+        if (fits) a.recs[base + i] = r;
     }
     __syncwarp();
+    return pairs;
 }
 
-// A work item: kItemChunks consecutive 256-query chunks of one partition
-// (nq[c] queries in chunk c, 0 past the partition's last chunk) against one
-// segment of its tiles.
+// A work item: up to kItemQueries consecutive queries of one partition's
+// queue (its chunks' slices from zchunk on) against one segment of its tiles.
 struct ItemRef {
-    uint32_t p, qbase, nq[kItemChunks], tb, te, zchunk;
+    uint32_t qbase, nq, tb, te, zchunk;
 };
 
 __device__ __forceinline__ ItemRef locate(const MatchArgs &a, uint32_t item) {
@@ -418,70 +426,111 @@ __device__ __forceinline__ ItemRef locate(const MatchArgs &a, uint32_t item) {
     const uint32_t local = item - a.item_off[lo];
     if (a.part_order) lo = a.part_order[lo];
     ItemRef r;
-    r.p = lo;
     const uint32_t pq = a.part_count[lo];
-    const uint32_t nchunks = (pq + kChunk - 1) / kChunk;
-    const uint32_t ngroups = (nchunks + kItemChunks - 1) / kItemChunks;
+    const uint32_t ngroups = (pq + kItemQueries - 1) / kItemQueries;
     const uint32_t group = local % ngroups, seg = local / ngroups;
-    const uint32_t c0 = group * kItemChunks;
-    r.qbase = a.part_off[lo] + c0 * kChunk;
-#pragma unroll
-    for (int c = 0; c < kItemChunks; ++c)
-        r.nq[c] = c0 + c < nchunks ? min((uint32_t)kChunk, pq - (c0 + c) * kChunk) : 0u;
+    r.qbase = a.part_off[lo] + group * kItemQueries;
+    r.nq = min((uint32_t)kItemQueries, pq - group * kItemQueries);
     r.tb = a.part_tile_begin[lo] + seg * a.seg_tiles;
     r.te = min(r.tb + a.seg_tiles, a.part_tile_begin[lo + 1]);
-    r.zchunk = a.chunk_off[lo] + c0;
+    r.zchunk = a.chunk_off[lo] + group * kItemChunks;
     return r;
 }
 
-// Thread 0: claim the next item and start the copies of its chunks' query
-// records; the item id is published through the full barrier's phase
-// completion.  Returns whether copies are in flight.
+// Thread 0: claim the next item and start the copies of its query records;
+// the item id is published through the full barrier's phase completion.
+// Returns whether copies are in flight.
 __device__ __forceinline__ bool produce(const MatchArgs &a, uint32_t total, MatchSmem &S) {
     const uint32_t item = uint32_t(atomicAdd(&a.counters[0], 1ull));
     S.item = item;
     if (item < total) {
         const ItemRef r = locate(a, item);
-        uint32_t bytes = 0;
-#pragma unroll
-        for (int c = 0; c < kItemChunks; ++c) bytes += r.nq[c] * kQueueWords * sizeof(uint32_t);
+        const uint32_t bytes = r.nq * sizeof(uint4);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(&S.full, bytes);
-#pragma unroll
-        for (int c = 0; c < kItemChunks; ++c) {
-            if (!r.nq[c]) continue;
-            tma_bulk_g2s(S.q[c], a.queue + (size_t(r.qbase) + size_t(c) * kChunk) * kQueueWords,
-                         r.nq[c] * kQueueWords * sizeof(uint32_t), &S.full);
-        }
+        mbar_expect_tx(&S.full, 2 * bytes);
+        tma_bulk_g2s(S.q_lo, a.queue_lo + r.qbase, bytes, &S.full);
+        tma_bulk_g2s(S.q_hi, a.queue_hi + r.qbase, bytes, &S.full);
         return true;
     }
     mbar_arrive(&S.full);  // nothing to copy: complete the phase so consumers see the end
     return false;
 }
 
-// The subset test.  Persistent CTAs take work items (partition, two
+// Lane per query: tests W candidates per lane (their words in q) against the
+// tile's filters, 4 per step, and sets bit l of m[c] when candidate c holds
+// filter l.  One broadcast 128-bit load gives word k of four filters; such a
+// load takes two of the shared-memory pipe's cycles, so that with one
+// candidate per lane the loads took as long as the LOP3s (48 against 56
+// cycles per 128 tests and quarter SM).  A hit is added with a predicated
+// add, which has a pipe of its own to go to; an or shares the LOP3s' (64
+// against 53 cycles measured).
+template <int W>
+__device__ __forceinline__ void test_queries(const uint4 (*tf)[kTile / 4], uint32_t groups, const uint4 (&lo)[W],
+                                             const uint4 (&hi)[W], uint32_t (&m)[W]) {
+#pragma unroll
+    for (int c = 0; c < W; ++c) m[c] = 0;
+#pragma unroll
+    for (int g = 0; g < kTile / 4; ++g) {
+        if (g >= (int)groups) break;
+        const uint4 w0 = tf[0][g], w1 = tf[1][g], w2 = tf[2][g], w3 = tf[3][g], w4 = tf[4][g], w5 = tf[5][g];
+#pragma unroll
+        for (int c = 0; c < W; ++c) {
+            uint32_t x0 = w0.x & ~lo[c].x, x1 = w0.y & ~lo[c].x, x2 = w0.z & ~lo[c].x, x3 = w0.w & ~lo[c].x;
+            x0 = andnot_or(w1.x, lo[c].y, x0);
+            x1 = andnot_or(w1.y, lo[c].y, x1);
+            x2 = andnot_or(w1.z, lo[c].y, x2);
+            x3 = andnot_or(w1.w, lo[c].y, x3);
+            x0 = andnot_or(w2.x, lo[c].z, x0);
+            x1 = andnot_or(w2.y, lo[c].z, x1);
+            x2 = andnot_or(w2.z, lo[c].z, x2);
+            x3 = andnot_or(w2.w, lo[c].z, x3);
+            x0 = andnot_or(w3.x, lo[c].w, x0);
+            x1 = andnot_or(w3.y, lo[c].w, x1);
+            x2 = andnot_or(w3.z, lo[c].w, x2);
+            x3 = andnot_or(w3.w, lo[c].w, x3);
+            x0 = andnot_or(w4.x, hi[c].x, x0);
+            x1 = andnot_or(w4.y, hi[c].x, x1);
+            x2 = andnot_or(w4.z, hi[c].x, x2);
+            x3 = andnot_or(w4.w, hi[c].x, x3);
+            x0 = andnot_or(w5.x, hi[c].y, x0);
+            x1 = andnot_or(w5.y, hi[c].y, x1);
+            x2 = andnot_or(w5.z, hi[c].y, x2);
+            x3 = andnot_or(w5.w, hi[c].y, x3);
+            add_if_zero(m[c], x0, 1u << (4 * g));
+            add_if_zero(m[c], x1, 2u << (4 * g));
+            add_if_zero(m[c], x2, 4u << (4 * g));
+            add_if_zero(m[c], x3, 8u << (4 * g));
+        }
+    }
+}
+
+// The subset test.  Persistent CTAs take work items (partition, up to four
 // consecutive 256-query chunks of its queue, segment of its tiles) from an
-// atomic counter; thread 0 stages the item's query records and slices with
-// bulk TMA copies into the CTA's two chunk buffers.  Each warp takes two
-// tiles (<= 32 filters each) at a time:
-//  * selection, for both tiles and both chunks at once: the tile's 8
-//    selector bits (bits every member holds); lane l ORs the "lacks bit"
-//    slices of 32-query word l & 7 of chunk (l >> 3) & 1 for tile l >> 4,
-//    so a query that lacks any of them is dropped; the remaining candidates
-//    go to the tile's list (one byte per query: the first chunk's, then the
-//    second's, placed by a prefix sum over the tile's 16 words);
-// then, tile by tile, over the candidates of both chunks together (one pass
-// over the tile's filters for 512 queries: fuller passes and trips):
-//  * many candidates: one candidate query per lane, the tile's filters read
-//    from shared memory (one broadcast 128-bit load gives word k of four
-//    filters): 6 LOP3 per (query, filter), the lane's hit mask over the tile
-//    built bit by bit; one pass per 32 candidates;
+// atomic counter; thread 0 stages the item's query records with bulk TMA
+// copies.  Each warp takes T tiles (<= 32 filters each) at a time, T x (the
+// item's 32-query words, rounded up to a power of two) = 32 lanes: one tile
+// for a full item, 32 tiles for an item of at most 32 queries, so that an
+// item's selection is shared by as many tiles as its queries leave room for
+// (one tile at a time took 32 visits where one is enough; one query against
+// a million filters spent 33 us in the subset test):
+//  * selection: the tile's 8 selector bits (bits every member holds); each
+//    lane ORs the "lacks bit" slices of its tile and 32-query word, so a query
+//    that lacks any of them is dropped; the remaining candidates go to the
+//    tile's list (one byte per query, placed by a prefix sum over the tile's
+//    words);
+// then, tile by tile, over the candidates of all chunks together (one pass
+// over the tile's filters for up to 1,024 queries: fuller passes and trips):
+//  * many candidates: candidate queries over the lanes (two per lane while
+//    more than 32 are left, then one), the tile's filters read from shared
+//    memory (test_queries), the lane's hit mask over the tile built bit by
+//    bit;
 //  * few candidates: one filter per lane (the tile in registers), four
 //    candidates per trip, one ballot per candidate for its hit mask;
 //  * each (query, tile) with a hit becomes a 16-byte record (query, tile,
-//    hit mask, key count from the tile's key-count bit planes), staged in a
-//    per-warp buffer and flushed with one atomic; the query's key total is
-//    added to qkeys[query] (for the prefix sum that places its keys).
+//    hit mask, key count), staged in a per-warp buffer and flushed with one
+//    atomic; the flush counts the records' keys from the tiles' key-count bit
+//    planes and adds them to qkeys[query] (for the prefix sum that places a
+//    query's keys).
 // The path per tile is chosen from the candidate count and the tile size
 // (estimated instruction costs; the choice does not change results).
 // COUNT: diagnostics instantiation that also tallies its work (a.work);
@@ -504,9 +553,24 @@ __global__ void __launch_bounds__(kMatchThreads, 4) k_match(MatchArgs a) {  // 4
     uint32_t w_tiles = 0, w_passes = 0, w_cand = 0, w_trips = 0, w_items = 0, w_groups = 0, w_lanes = 0, w_small = 0;
     uint32_t wn = 0;      // records staged by this warp (warp-uniform)
     uint32_t w_recs = 0;  // records this warp has produced (warp-uniform)
-    uint32_t pairs = 0;  // matching (query, filter) pairs found by this lane
+    uint32_t pairs = 0;   // matching (query, filter) pairs counted by this lane
     const uint32_t lane_lt = (1u << lane) - 1u;
     uint32_t *tfw = reinterpret_cast<uint32_t *>(S.tf[warp]);
+    uint8_t *list = S.list[warp];
+    HitRec *rec = S.rec[warp];
+    // stages one record for every lane with a hit mask m
+    auto stage = [&](uint32_t m, uint32_t query, uint32_t t) {
+        const uint32_t wm = __ballot_sync(kFull, m != 0);
+        if (wm == 0) return;
+        const uint32_t k = __popc(wm);
+        if (wn + k > (uint32_t)kWarpRecs) {
+            pairs += flush_recs(rec, wn, a, lane);
+            wn = 0;
+        }
+        if (m) rec[wn + __popc(wm & lane_lt)] = HitRec{query, t, m, 0u};
+        wn += k;
+        if (TIMED) w_recs += k;
+    };
     for (uint32_t it = 0;; ++it) {
         // stage the next item once every warp has released the buffers
         // (they held item it - 1); thread 0 keeps track of the copies in
@@ -540,74 +604,67 @@ __global__ void __launch_bounds__(kMatchThreads, 4) k_match(MatchArgs a) {  // 4
             item_c0 = clock64();
             item_recs0 = w_recs;
         }
-        for (uint32_t t0 = r.tb + warp * kQuad; t0 < r.te; t0 += kMatchWarps * kQuad) {
-            // selection for the warp's tiles and all chunks of the item at
-            // once: lane l serves word l & 7 of chunk (l >> 3) % kItemChunks
-            // for tile t0 + l / kTileLanes; the tile's 8 selector bits OR the
-            // "lacks" slices of the lane's 32 queries (read through L1: the
-            // item's slices are shared by all its tiles)
-            const uint32_t gi = lane / kTileLanes, tl = lane % kTileLanes, ch = tl >> 3, w = lane & 7;
+        // lanes per tile: the item's 32-query words, as a power of two
+        const uint32_t words = (r.nq + 31) >> 5;
+        const uint32_t lg = words > 1 ? 32 - __clz(words - 1) : 0u, tiles = 32u >> lg;
+        const uint32_t wi = lane & ((1u << lg) - 1u), gi = lane >> lg;  // the lane's word, its tile of the step
+        const uint32_t last = lane | ((1u << lg) - 1u);                   // the last lane of its tile
+        // queries of the lane's word, and its slices
+        const uint32_t live = wi * 32 + 32 <= r.nq ? kFull : wi * 32 >= r.nq ? 0u : (1u << (r.nq - wi * 32)) - 1u;
+        const uint32_t *zl = a.slices + (size_t(r.zchunk) + (wi >> 3)) * kSliceWords + (wi & 7);
+        for (uint32_t t0 = r.tb + warp * tiles; t0 < r.te; t0 += kMatchWarps * tiles) {
             const uint32_t tq = t0 + gi;
-            uint32_t nqc = r.nq[0];  // queries in the lane's chunk (no dynamic index into r)
-#pragma unroll
-            for (int c = 1; c < kItemChunks; ++c)
-                if (ch == (uint32_t)c) nqc = r.nq[c];
             uint32_t cand = 0, tcount = 0;
-            if (tq < r.te) {
+            if (tq < r.te && live) {  // words past the item's queries have no slices
                 const TileInfo ti = a.tile_info[tq];
                 tcount = ti.count;
-                if (nqc) {  // chunks past the partition's last have no slices
-                    const uint32_t *zl = a.slices + (size_t(r.zchunk) + ch) * kSliceWords + w;
-                    const uint32_t lack =
-                        __ldg(&zl[(ti.sel[0] & 0xFFu) * 8]) | __ldg(&zl[((ti.sel[0] >> 8) & 0xFFu) * 8]) |
-                        __ldg(&zl[((ti.sel[0] >> 16) & 0xFFu) * 8]) | __ldg(&zl[(ti.sel[0] >> 24) * 8]) |
-                        __ldg(&zl[(ti.sel[1] & 0xFFu) * 8]) | __ldg(&zl[((ti.sel[1] >> 8) & 0xFFu) * 8]) |
-                        __ldg(&zl[((ti.sel[1] >> 16) & 0xFFu) * 8]) | __ldg(&zl[(ti.sel[1] >> 24) * 8]);
-                    cand = ~lack;
-                    if (w * 32 + 32 > nqc) cand &= w * 32 >= nqc ? 0u : ((1u << (nqc - w * 32)) - 1u);
-                }
-                if (tl == 0) S.tk[warp][gi] = a.tile_keys[tq];
+                const uint32_t lack =
+                    __ldg(&zl[(ti.sel[0] & 0xFFu) * 8]) | __ldg(&zl[((ti.sel[0] >> 8) & 0xFFu) * 8]) |
+                    __ldg(&zl[((ti.sel[0] >> 16) & 0xFFu) * 8]) | __ldg(&zl[(ti.sel[0] >> 24) * 8]) |
+                    __ldg(&zl[(ti.sel[1] & 0xFFu) * 8]) | __ldg(&zl[((ti.sel[1] >> 8) & 0xFFu) * 8]) |
+                    __ldg(&zl[((ti.sel[1] >> 16) & 0xFFu) * 8]) | __ldg(&zl[(ti.sel[1] >> 24) * 8]);
+                cand = ~lack & live;
             }
-            if (COUNT) w_tiles += __popc(__ballot_sync(kFull, tq < r.te && tl == 0));  // lane 0 reports
+            if (COUNT) w_tiles += __popc(__ballot_sync(kFull, tq < r.te && wi == 0));  // lane 0 reports
             // candidate lists (query index in its chunk, one byte each): a
-            // prefix sum over each tile's words (chunk by chunk) places every
-            // lane's queries
+            // prefix sum over each tile's words places every lane's queries,
+            // from the word's highest down
             const uint32_t cnt = __popc(cand);
             uint32_t incl = cnt;
-#pragma unroll
-            for (int o = 1; o < kTileLanes; o <<= 1) {
+            for (uint32_t o = 1; o < (1u << lg); o <<= 1) {
                 const uint32_t v = __shfl_up_sync(kFull, incl, o);
-                if (tl >= (unsigned)o) incl += v;
+                if (wi >= o) incl += v;
             }
             {
-                uint8_t *lst = S.list[warp][gi];
-                uint32_t pos = incl - cnt;
-                while (cand) {
-                    lst[pos++] = uint8_t(w * 32 + __ffs(cand) - 1);
-                    cand &= cand - 1;
+                uint8_t *at = list + ((gi << lg) << 5) + incl;
+                if (lane == last) {
+                    // pad to a multiple of 4 (its hits are dropped)
+                    for (uint32_t x = incl; x & 3u; ++x) at[x - incl] = 0;
                 }
-                const uint32_t nt = __shfl_sync(kFull, incl, lane | (kTileLanes - 1));
-                if (tl < 4) lst[nt + tl] = 0;  // pad to a multiple of 4 (its hits are dropped)
+                while (cand) {
+                    const uint32_t bit = 31u - __clz(cand);
+                    cand ^= 1u << bit;
+                    *--at = uint8_t(wi * 32 + bit);
+                }
             }
             __syncwarp();
-            for (int i = 0; i < kQuad; ++i) {
-                const uint32_t n = __shfl_sync(kFull, incl, kTileLanes * i + kTileLanes - 1);
+            for (uint32_t todo = __ballot_sync(kFull, lane == last && incl != 0); todo; todo &= todo - 1) {
+                const uint32_t end = __ffs(todo) - 1, first = end & ~((1u << lg) - 1u);  // the tile's lanes
+                const uint32_t n = __shfl_sync(kFull, incl, end), count = __shfl_sync(kFull, tcount, first);
+                const uint32_t t = t0 + (end >> lg);
                 // list positions where chunks 1 .. kItemChunks - 1 begin: the
                 // candidate at position x is in chunk sum_c (x >= cb[c])
                 uint32_t cb[kItemChunks - 1];
 #pragma unroll
-                for (int c = 0; c + 1 < kItemChunks; ++c) cb[c] = __shfl_sync(kFull, incl, kTileLanes * i + 8 * c + 7);
-                auto chunk_of = [&](uint32_t x) {
+                for (int c = 0; c + 1 < kItemChunks; ++c) cb[c] = __shfl_sync(kFull, incl, min(first + 8 * c + 7, end));
+                auto query_at = [&](uint32_t x, uint32_t in_chunk) {
                     uint32_t c = 0;
 #pragma unroll
-                    for (int k = 0; k + 1 < kItemChunks; ++k) c += x >= cb[k] ? 1u : 0u;
-                    return c;
+                    for (int k = 0; k + 1 < kItemChunks; ++k) c += x >= cb[k] ? (uint32_t)kChunk : 0u;
+                    return c + in_chunk;
                 };
                 if (COUNT) w_cand += n;  // the warp's candidates (lane 0 reports)
-                if (n == 0) continue;
-                const uint32_t t = t0 + i;
-                const uint32_t count = __shfl_sync(kFull, tcount, kTileLanes * i);
-                const uint8_t *lst = S.list[warp][i];
+                const uint8_t *lst = list + (first << 5);
                 uint32_t f[kWords];
 #pragma unroll
                 for (int k = 0; k < kWords; ++k) f[k] = __ldg(&a.tile_words[(size_t(t) * kWords + k) * kTile + lane]);
@@ -618,81 +675,45 @@ __global__ void __launch_bounds__(kMatchThreads, 4) k_match(MatchArgs a) {  // 4
 #pragma unroll
                     for (int k = 0; k < kWords; ++k) tfw[k * kTile + lane] = f[k];
                     __syncwarp();
-                    for (uint32_t p0 = 0; p0 < n; p0 += 32) {
+                    uint32_t p0 = 0;
+                    for (; p0 + 32 < n; p0 += 64) {
+                        const uint32_t j0 = p0 + lane, j1 = j0 + 32;
+                        const uint32_t i0 = query_at(j0, lst[j0]), i1 = j1 < n ? query_at(j1, lst[j1]) : 0u;
+                        const uint4 lo[2] = {S.q_lo[i0], S.q_lo[i1]}, hi[2] = {S.q_hi[i0], S.q_hi[i1]};
+                        uint32_t m[2];
+                        test_queries<2>(S.tf[warp], groups, lo, hi, m);
+                        if (COUNT) {
+                            w_passes += 2;
+                            w_groups += 2 * groups;
+                            w_lanes += min(64u, n - p0);
+                        }
+                        stage(m[0] & vm, hi[0].z, t);
+                        stage(j1 < n ? m[1] & vm : 0u, hi[1].z, t);
+                    }
+                    if (p0 < n) {
+                        const uint32_t j0 = p0 + lane, i0 = j0 < n ? query_at(j0, lst[j0]) : 0u;
+                        const uint4 lo[1] = {S.q_lo[i0]}, hi[1] = {S.q_hi[i0]};
+                        uint32_t m[1];
+                        test_queries<1>(S.tf[warp], groups, lo, hi, m);
                         if (COUNT) {
                             ++w_passes;
                             w_groups += groups;
-                            w_lanes += min(32u, n - p0);
+                            w_lanes += n - p0;
                             if (p0 == 0 && n <= 16) ++w_small;
                         }
-                        const uint32_t j = p0 + lane;
-                        const uint4 *sq = reinterpret_cast<const uint4 *>(S.q[chunk_of(j)]);
-                        const uint32_t c2 = j < n ? 2u * lst[j] : 0u;
-                        const uint4 qa = sq[c2], qb = sq[c2 + 1];
-                        uint32_t m = 0;
-#pragma unroll
-                        for (int g = 0; g < kTile / 4; ++g) {
-                            if (g >= (int)groups) break;
-                            const uint4 w0 = S.tf[warp][0][g], w1 = S.tf[warp][1][g], w2 = S.tf[warp][2][g];
-                            const uint4 w3 = S.tf[warp][3][g], w4 = S.tf[warp][4][g], w5 = S.tf[warp][5][g];
-                            uint32_t x0 = w0.x & ~qa.x, x1 = w0.y & ~qa.x, x2 = w0.z & ~qa.x, x3 = w0.w & ~qa.x;
-                            x0 = andnot_or(w1.x, qa.y, x0);
-                            x1 = andnot_or(w1.y, qa.y, x1);
-                            x2 = andnot_or(w1.z, qa.y, x2);
-                            x3 = andnot_or(w1.w, qa.y, x3);
-                            x0 = andnot_or(w2.x, qa.z, x0);
-                            x1 = andnot_or(w2.y, qa.z, x1);
-                            x2 = andnot_or(w2.z, qa.z, x2);
-                            x3 = andnot_or(w2.w, qa.z, x3);
-                            x0 = andnot_or(w3.x, qa.w, x0);
-                            x1 = andnot_or(w3.y, qa.w, x1);
-                            x2 = andnot_or(w3.z, qa.w, x2);
-                            x3 = andnot_or(w3.w, qa.w, x3);
-                            x0 = andnot_or(w4.x, qb.x, x0);
-                            x1 = andnot_or(w4.y, qb.x, x1);
-                            x2 = andnot_or(w4.z, qb.x, x2);
-                            x3 = andnot_or(w4.w, qb.x, x3);
-                            x0 = andnot_or(w5.x, qb.y, x0);
-                            x1 = andnot_or(w5.y, qb.y, x1);
-                            x2 = andnot_or(w5.z, qb.y, x2);
-                            x3 = andnot_or(w5.w, qb.y, x3);
-                            if (x0 == 0) m |= 1u << (4 * g);
-                            if (x1 == 0) m |= 2u << (4 * g);
-                            if (x2 == 0) m |= 4u << (4 * g);
-                            if (x3 == 0) m |= 8u << (4 * g);
-                        }
-                        m &= vm;
-                        if (j >= n) m = 0;
-                        const uint32_t wm = __ballot_sync(kFull, m != 0);
-                        if (wm == 0) continue;
-                        if (wn + 32 > (uint32_t)kWarpRecs) {
-                            flush_recs(S.rec[warp], wn, a, lane);
-                            wn = 0;
-                        }
-                        if (m) {
-                            const uint32_t nk = mask_keys(S.tk[warp][i], m, a.slot_key_off, t);
-                            S.rec[warp][wn + __popc(wm & lane_lt)] = HitRec{qb.z, t, m, nk};
-                            atomicAdd(&a.qkeys[qb.z], nk);
-                            pairs += __popc(m);
-                        }
-                        wn += __popc(wm);
-                        if (TIMED) w_recs += __popc(wm);
+                        stage(j0 < n ? m[0] & vm : 0u, hi[0].z, t);
                     }
                 } else {
                     const bool lane_valid = lane < count;
                     for (uint32_t j = 0; j < n; j += 4) {
                         if (COUNT) ++w_trips;
                         const uint32_t idx4 = *reinterpret_cast<const uint32_t *>(lst + j);
-                        const uint32_t ia = (idx4 & 0xFFu) * 2, ib = ((idx4 >> 8) & 0xFFu) * 2;
-                        const uint32_t ic = ((idx4 >> 16) & 0xFFu) * 2, id = (idx4 >> 24) * 2;
-                        const uint4 *sa = reinterpret_cast<const uint4 *>(S.q[chunk_of(j)]);
-                        const uint4 *sb = reinterpret_cast<const uint4 *>(S.q[chunk_of(j + 1)]);
-                        const uint4 *sc = reinterpret_cast<const uint4 *>(S.q[chunk_of(j + 2)]);
-                        const uint4 *sd = reinterpret_cast<const uint4 *>(S.q[chunk_of(j + 3)]);
-                        const uint4 p0 = sa[ia], p1 = sa[ia + 1];
-                        const uint4 q0 = sb[ib], q1 = sb[ib + 1];
-                        const uint4 r0 = sc[ic], r1 = sc[ic + 1];
-                        const uint4 u0 = sd[id], u1 = sd[id + 1];
+                        const uint32_t ia = query_at(j, idx4 & 0xFFu), ib = query_at(j + 1, (idx4 >> 8) & 0xFFu);
+                        const uint32_t ic = query_at(j + 2, (idx4 >> 16) & 0xFFu), id = query_at(j + 3, idx4 >> 24);
+                        const uint4 p0 = S.q_lo[ia], p1 = S.q_hi[ia];
+                        const uint4 q0 = S.q_lo[ib], q1 = S.q_hi[ib];
+                        const uint4 r0 = S.q_lo[ic], r1 = S.q_hi[ic];
+                        const uint4 u0 = S.q_lo[id], u1 = S.q_hi[id];
                         uint32_t x0 = f[0] & ~p0.x, x1 = f[0] & ~q0.x, x2 = f[0] & ~r0.x, x3 = f[0] & ~u0.x;
                         x0 = andnot_or(f[1], p0.y, x0);
                         x1 = andnot_or(f[1], q0.y, x1);
@@ -718,28 +739,14 @@ __global__ void __launch_bounds__(kMatchThreads, 4) k_match(MatchArgs a) {  // 4
                         if (!__any_sync(kFull, lane_valid && min(min(x0, x1), min(x2, x3)) == 0)) continue;
                         // warp-uniform from here: one ballot per candidate gives the
                         // tile's hit mask for that query; lane k < 4 stages record k
-                        // (list padding repeats query 0 and is dropped)
+                        // (list padding repeats a query and is dropped)
                         const uint32_t b0 = __ballot_sync(kFull, x0 == 0) & vm;
                         const uint32_t b1 = __ballot_sync(kFull, x1 == 0) & vm;
                         const uint32_t b2 = __ballot_sync(kFull, x2 == 0) & vm;
                         const uint32_t b3 = __ballot_sync(kFull, x3 == 0) & vm;
                         const uint32_t mine = lane == 0 ? b0 : lane == 1 ? b1 : lane == 2 ? b2 : b3;
                         const uint32_t qid = lane == 0 ? p1.z : lane == 1 ? q1.z : lane == 2 ? r1.z : u1.z;
-                        const bool wr = lane < 4 && mine != 0 && j + lane < n;
-                        const uint32_t wm = __ballot_sync(kFull, wr);
-                        if (wm == 0) continue;
-                        if (wn + 4 > (uint32_t)kWarpRecs) {
-                            flush_recs(S.rec[warp], wn, a, lane);
-                            wn = 0;
-                        }
-                        if (wr) {
-                            const uint32_t nk = mask_keys(S.tk[warp][i], mine, a.slot_key_off, t);
-                            S.rec[warp][wn + __popc(wm & lane_lt)] = HitRec{qid, t, mine, nk};
-                            atomicAdd(&a.qkeys[qid], nk);
-                            pairs += __popc(mine);
-                        }
-                        wn += __popc(wm);
-                        if (TIMED) w_recs += __popc(wm);
+                        stage(lane < 4 && j + lane < n ? mine : 0u, qid, t);
                     }
                 }
                 __syncwarp();  // the tile buffer is rebuilt for the next tile
@@ -753,7 +760,7 @@ __global__ void __launch_bounds__(kMatchThreads, 4) k_match(MatchArgs a) {  // 4
         }
         if (lane == 0) mbar_arrive(&S.empty);
     }
-    if (wn) flush_recs(S.rec[warp], wn, a, lane);
+    if (wn) pairs += flush_recs(rec, wn, a, lane);
     pairs = __reduce_add_sync(kFull, pairs);
     if (lane == 0 && pairs) atomicAdd(&a.counters[3], (unsigned long long)pairs);
     if (COUNT && lane == 0) {

@@ -160,7 +160,7 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     TM_CUDA(cudaMemcpyAsync(&chunks, chunk_off + P, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     TM_CUDA(cudaStreamSynchronize(st));
 
-    uint32_t *queue = ar.take<uint32_t>(size_t(std::max<uint32_t>(routed, 1)) * kQueueWords, "partition queues");
+    uint4 *queue = ar.take<uint4>(size_t(std::max<uint32_t>(routed, 1)) * 2, "partition queues");
     uint32_t *slices = ar.take<uint32_t>(size_t(std::max<uint32_t>(chunks, 1)) * kSliceWords, "query slices");
     const uint32_t fits = route_window(P, nq, ar.left() / sizeof(uint32_t));
     if (fits < window) {
@@ -169,14 +169,15 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
         if (ar.left() < size_t(window) * row_words * sizeof(uint32_t))
             throw Error(TM_ERR_CAPACITY, "no-allocation scratch exhausted at the routing rows; split the batch");
     }
-    launch_fill_queues(d_queries, nq, t, window, rows, part_count, nullptr, part_off, chunk_off, queue, slices, st);
+    launch_fill_queues(d_queries, nq, t, window, rows, part_count, nullptr, part_off, chunk_off, queue, queue + routed, slices,
+                       st);
     // hit records fill what is left of the array; after the match the part
     // they did not use goes to the keys
     const size_t rec_room = ar.left() / sizeof(HitRec);
     if (rec_room < 256) throw Error(TM_ERR_CAPACITY, "no-allocation scratch exhausted before the hit records; split the batch");
     HitRec *recs = ar.take<HitRec>(rec_room - 32, "hit records");
     MatchArgs a{t.tile_words.p, t.tile_info.p, t.tile_keys.p, t.slot_key_off.p, t.part_tile_begin.p, part_count, part_off,
-                item_off, chunk_off, queue, slices, P, seg_tiles, counters, recs, (unsigned long long)(rec_room - 32), qkeys,
+                item_off, chunk_off, queue, queue + routed, slices, P, seg_tiles, counters, recs, (unsigned long long)(rec_room - 32), qkeys,
                 fpl_trip_cost(), nullptr, nullptr, nullptr};
     launch_match<false>(a, unsigned(sms) * 4, st);
     TM_CHECK_LAUNCH();

@@ -16,7 +16,7 @@ constexpr int kTile = 32;          // filters per tile (one per lane of a warp)
 constexpr int kChunk = 256;        // queries per partition batch (QUERIES_BATCH_SIZE, parameters.hh:13)
 constexpr int kItemChunks = 4;     // 256-query chunks of one partition that a subset-test work item covers
 constexpr int kItemQueries = kItemChunks * kChunk;
-constexpr int kQueueWords = 8;     // queued query record: 6 filter words, query id, pad (32 bytes)
+constexpr int kQueueWords = 8;     // queued query record, in two planes of 16 bytes: 6 filter words, query id, pad
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
 // Tile descriptor (16 bytes): the positions of up to 8 bits that every
@@ -57,6 +57,11 @@ __device__ __forceinline__ uint32_t keys_of_mask(const TileKeys &tk, uint32_t m)
 
 __device__ __forceinline__ uint32_t andnot_or(uint32_t f, uint32_t q, uint32_t acc) {
     return (f & ~q) | acc;  // one LOP3
+}
+
+// acc += v when x is 0, as a compare and a predicated add.
+__device__ __forceinline__ void add_if_zero(uint32_t &acc, uint32_t x, uint32_t v) {
+    asm("{\n .reg .pred p;\n setp.eq.u32 p, %1, 0;\n @p add.u32 %0, %0, %2;\n}\n" : "+r"(acc) : "r"(x), "r"(v));
 }
 
 __device__ __forceinline__ bool subset6(const uint32_t *f, const uint32_t *q) {
