@@ -296,13 +296,11 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
                                     cudaMemcpyDeviceToHost, st));
     }
     // ---- keys ----
-    const unsigned gblocks = std::max(1u, std::min(blocks_for(hc[1], kFillThreads * kFillPerLane), unsigned(s.sm_count) * 16));
     // fill; each retry: match, scan, readback
     bs.launches += 1 + (2 + scan_launches(nq)) * uint32_t(bs.retries);
     bs.pairs = hc[3];
     s.keys.reserve(std::max<uint64_t>(total, 1));
-    k_key_fill<<<gblocks, kFillThreads, 0, st>>>(s.recs.p, counters, t.slot_key_off.p, t.tile_keys.p, t.keys.p, s.qoff.p, qcursor, s.keys.p);
-    TM_CHECK_LAUNCH();
+    launch_key_fill(t, s.recs.p, counters, hc[1], s.qoff.p, qcursor, nq, s.keys.p, s.sm_count, st);
     if (!unique) {
         TM_CUDA(cudaStreamSynchronize(st));
         *d_offsets = s.qoff.p;

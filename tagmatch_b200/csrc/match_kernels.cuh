@@ -798,100 +798,89 @@ inline void launch_match(const MatchArgs &a, unsigned grid, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 // Key gather
 // ---------------------------------------------------------------------------
-// records per lane per warp step (loads in flight) and the gather's
-// minimum resident CTAs per SM (register budget); build-time tunables
-#ifndef TM_FILL_PER_LANE
-#define TM_FILL_PER_LANE 2
-#endif
-#ifndef TM_FILL_MIN_CTAS
-#define TM_FILL_MIN_CTAS 6
-#endif
-constexpr int kFillPerLane = TM_FILL_PER_LANE;
+constexpr int kFillPerLane = 2;  // records per lane and warp step (loads in flight)
+constexpr int kFillCtas = 6;     // resident per SM, at least (register budget)
 
 constexpr int kFillThreads = 256;
 constexpr int kFillWarps = kFillThreads / 32;
 constexpr int kFillStep = 32 * kFillPerLane;  // records per warp step
+// The block variant of the gather: records per block, and the most queries
+// of a batch that takes it (4 bytes of shared memory each).
+constexpr uint32_t kFillBlockRecs = 2048;
+constexpr uint32_t kFillBlockQueries = 2048;
 
-// Position of the k-th set bit (k from 0) of x, which has more than k set
-// bits: halving popcounts.
-__device__ __forceinline__ uint32_t nth_set_bit(uint32_t x, uint32_t k) {
-    uint32_t pos = 0;
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
-        const uint32_t lowc = __popc(x & ((1u << s) - 1u));
-        if (k >= lowc) {
-            k -= lowc;
-            x >>= s;
-            pos += s;
-        }
-    }
-    return pos;
+// Owners of 32 consecutive positions p0 + lane, when lane i owns a non-empty
+// stretch that begins at `start` (increasing with i; live: the lane has one):
+// the begins inside the window as a bit mask, and the lanes that began before
+// it.  Eight instructions, where a binary search by shuffles takes five
+// rounds of three on the shared-memory pipe.
+__device__ __forceinline__ uint32_t owner_of(uint32_t start, bool live, uint32_t p0, uint32_t lane_le) {
+    const uint32_t begins = __reduce_or_sync(kFull, live && start >= p0 && start - p0 < 32u ? 1u << (start - p0) : 0u);
+    const uint32_t before = __popc(__ballot_sync(kFull, live && start < p0));
+    return before + __popc(begins & lane_le) - 1u;
 }
 
 // Copies every record's keys into its query's range (qoff).  Each record's
-// keys are reserved with one atomic on the query's cursor (qcursor, zeroed
-// by the caller).  The table keeps keys in slot order, so each run of
-// adjacent hit bits [lo, hi) of a record's mask is the key range
-// [o[lo], o[hi]) of the tile's slot offsets o.  A warp takes 32 x
-// kFillPerLane records per step and numbers all their runs (a prefix sum
-// over the lanes' run counts); lane i of a batch then takes run 32 b + i:
-// a 5-step shuffle search for the lane whose records hold it, the record
-// from shared memory, the run's first bit by halving popcounts, its key
-// range from the slot offsets, and its place in the record's output from
-// the keys of the hit bits below it (the tile's key-count planes).  The
-// warp copies the batch's runs together, 32 keys per step (a prefix sum
-// over the run lengths and, for key j, a 5-step search for the run that
-// owns it), so the stores coalesce and a record with several runs costs no
-// extra pass over the warp.
-__global__ void __launch_bounds__(kFillThreads, TM_FILL_MIN_CTAS) k_key_fill(
+// keys are reserved on the query's cursor (qcursor, zeroed by the caller).
+// The table keeps keys in slot order, so each run of adjacent hit bits
+// [lo, hi) of a record's mask is the key range [o[lo], o[hi]) of the tile's
+// slot offsets o.  A warp takes 32 x kFillPerLane records per step and
+// numbers all their runs (a prefix sum over the lanes' run counts); lane i of
+// a batch then takes run 32 b + i: the lane whose records hold it (owner_of),
+// the record from shared memory, the run's first bit, its key range from the
+// slot offsets, and its place in the record's output from the keys of the hit
+// bits below it (the tile's key-count planes).  The warp copies the batch's
+// runs together, 32 keys per step (a prefix sum over the run lengths and, for
+// key j, the run that owns it), so the stores coalesce and a record with
+// several runs costs no extra pass over the warp.
+//
+// BLOCK: a CTA takes kFillBlockRecs consecutive records, sums their keys per
+// query in shared memory and reserves each query's keys with one global
+// atomic.  Atomics on one address follow one another, and in a batch of few
+// queries the heaviest holds a good part of all records: 500 queries of the
+// ten-million table (1.8 M records) took 272 us, six times the time per
+// record of a batch of 20,011.
+template <bool BLOCK>
+__global__ void __launch_bounds__(kFillThreads, kFillCtas) k_key_fill(
     const HitRec *__restrict__ recs, const unsigned long long *__restrict__ counters,
     const uint32_t *__restrict__ slot_key_off, const TileKeys *__restrict__ tile_keys, const uint32_t *__restrict__ tkeys,
-    const uint64_t *__restrict__ qoff, uint32_t *__restrict__ qcursor, uint32_t *__restrict__ out) {
+    const uint64_t *__restrict__ qoff, uint32_t *__restrict__ qcursor, uint32_t nq, uint32_t *__restrict__ out) {
+    extern __shared__ uint32_t s_cur[];  // BLOCK: [nq] the block's cursor per query
     // per warp and record of the step: tile, hit mask, keys, runs of the
     // lane's earlier records; and the record's first output position
     __shared__ uint4 s_rec[kFillWarps][kFillStep];
     __shared__ unsigned long long s_dst[kFillWarps][kFillStep];
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lane_le = (2u << lane) - 1u;
     const unsigned long long n = counters[1];
-    const unsigned long long warps = (unsigned long long)gridDim.x * kFillWarps;
-    const unsigned long long wid = (unsigned long long)blockIdx.x * kFillWarps + warp;
-    for (unsigned long long base = wid * kFillStep; base < n; base += warps * kFillStep) {
+    // records [base, end) by the calling warp, kFillStep at most
+    auto step = [&](unsigned long long base, unsigned long long end) {
         HitRec r[kFillPerLane];
 #pragma unroll
         for (int j = 0; j < kFillPerLane; ++j) {
             const unsigned long long i = base + j * 32 + lane;
-            r[j] = i < n ? recs[i] : HitRec{kPadQuery, 0u, 0u, 0u};
+            r[j] = i < end ? recs[i] : HitRec{kPadQuery, 0u, 0u, 0u};
         }
         uint32_t nruns = 0;
         unsigned long long dst[kFillPerLane];
 #pragma unroll
         for (int j = 0; j < kFillPerLane; ++j) {
-            const bool live = r[j].query != kPadQuery && r[j].nkeys != 0;
+            const bool live = r[j].query != kPadQuery;
             const uint32_t m = live ? r[j].mask : 0u;
-            dst[j] = live ? qoff[r[j].query] + atomicAdd(&qcursor[r[j].query], r[j].nkeys) : 0ull;
-            s_rec[warp][j * 32 + lane] = make_uint4(r[j].tile, m, live ? r[j].nkeys : 0u, nruns);
+            dst[j] = live ? qoff[r[j].query] + atomicAdd(BLOCK ? &s_cur[r[j].query] : &qcursor[r[j].query], r[j].nkeys) : 0ull;
+            s_rec[warp][j * 32 + lane] = make_uint4(r[j].tile, m, r[j].nkeys, nruns);
             nruns += __popc(m & ~(m << 1));  // run starts
         }
-        uint32_t incl = nruns;
-#pragma unroll
-        for (int s = 1; s < 32; s <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFull, incl, s);
-            if (lane >= (unsigned)s) incl += v;
-        }
+        const uint32_t incl = warp_incl_scan(nruns);
         const uint32_t total = __shfl_sync(kFull, incl, 31);
         const uint32_t excl = incl - nruns;
         __syncwarp();
         for (uint32_t rb = 0; rb < total; rb += 32) {
             const uint32_t ri = rb + lane;
-            uint32_t owner = 0;  // first lane whose inclusive run count exceeds ri
-#pragma unroll
-            for (int s = 16; s >= 1; s >>= 1) {
-                const uint32_t v = __shfl_sync(kFull, incl, owner + s - 1);
-                if (v <= ri) owner += s;
-            }
+            const uint32_t owner = owner_of(excl, nruns != 0, rb, lane_le);
             const uint32_t oexcl = __shfl_sync(kFull, excl, owner);
             const bool have = ri < total;
-            uint32_t slot = owner, src = 0, end = 0, below = 0, t = 0, nk = 0;
+            uint32_t slot = owner, src = 0, end_key = 0, below = 0, t = 0, nk = 0;
             bool last = true;
             TileKeys tk{{0u, 0u, 0u}, 0u};
             if (have) {
@@ -904,13 +893,16 @@ __global__ void __launch_bounds__(kFillThreads, TM_FILL_MIN_CTAS) k_key_fill(
                 const uint32_t m = rc.y;
                 t = rc.x;
                 nk = rc.z;
-                const uint32_t lo = nth_set_bit(m & ~(m << 1), k - rc.w);
-                const uint32_t hi = lo + uint32_t(__ffsll(~((unsigned long long)m >> lo))) - 1u;
+                uint32_t starts = m & ~(m << 1);
+                for (uint32_t i = k - rc.w; i; --i) starts &= starts - 1;  // few: most records have one run
+                const uint32_t lo = __ffs(starts) - 1u;
+                const uint32_t above = ~(m >> lo);  // first clear bit from lo on (none: the run ends the tile)
+                const uint32_t hi = above ? lo + __ffs(above) - 1u : 32u;
                 const uint32_t *o = slot_key_off + size_t(t) * kTile;
                 below = m & ((1u << lo) - 1u);  // hit bits of the earlier runs
                 last = hi >= 32u || (m >> hi) == 0u;
                 src = o[lo];
-                if (!last) end = o[hi];
+                if (!last) end_key = o[hi];
                 if (below) tk = tile_keys[t];
             }
             if (rb == 0) {
@@ -924,34 +916,68 @@ __global__ void __launch_bounds__(kFillThreads, TM_FILL_MIN_CTAS) k_key_fill(
             unsigned long long d = 0;
             if (have) {
                 const uint32_t bk = below ? mask_keys(tk, below, slot_key_off, t) : 0u;
-                len = last ? nk - bk : end - src;
+                len = last ? nk - bk : end_key - src;
                 d = s_dst[warp][slot] + bk;
             }
-            // the batch's runs, copied together
-            uint32_t kin = len;
-#pragma unroll
-            for (int s = 1; s < 32; s <<= 1) {
-                const uint32_t v = __shfl_up_sync(kFull, kin, s);
-                if (lane >= (unsigned)s) kin += v;
-            }
+            // the batch's runs, copied together: key j of the batch comes from
+            // src - start + j and goes to d - start + j of its run
+            const uint32_t kin = warp_incl_scan(len);
             const uint32_t keys = __shfl_sync(kFull, kin, 31);
             const uint32_t start = kin - len;
+            src -= start;
+            d -= start;
             for (uint32_t j0 = 0; j0 < keys; j0 += 32) {
                 const uint32_t kk = j0 + lane;
-                uint32_t ro = 0;  // first lane whose inclusive key count exceeds kk
-#pragma unroll
-                for (int s = 16; s >= 1; s >>= 1) {
-                    const uint32_t v = __shfl_sync(kFull, kin, ro + s - 1);
-                    if (v <= kk) ro += s;
-                }
-                const uint32_t ostart = __shfl_sync(kFull, start, ro);
+                const uint32_t ro = owner_of(start, len != 0, j0, lane_le);
                 const uint32_t osrc = __shfl_sync(kFull, src, ro);
                 const unsigned long long odst = __shfl_sync(kFull, d, ro);
-                if (kk < keys) out[odst + (kk - ostart)] = tkeys[osrc + (kk - ostart)];
+                if (kk < keys) out[odst + kk] = tkeys[osrc + kk];
             }
         }
         __syncwarp();  // the shared entries are rewritten by the next step
+    };
+    if constexpr (BLOCK) {
+        for (unsigned long long b0 = (unsigned long long)blockIdx.x * kFillBlockRecs; b0 < n;
+             b0 += (unsigned long long)gridDim.x * kFillBlockRecs) {
+            const unsigned long long b1 = min(n, b0 + kFillBlockRecs);
+            for (uint32_t q = threadIdx.x; q < nq; q += kFillThreads) s_cur[q] = 0;
+            __syncthreads();
+            for (unsigned long long i = b0 + threadIdx.x; i < b1; i += kFillThreads) {
+                const HitRec r = recs[i];
+                atomicAdd(&s_cur[r.query], r.nkeys);
+            }
+            __syncthreads();
+            for (uint32_t q = threadIdx.x; q < nq; q += kFillThreads) {
+                const uint32_t c = s_cur[q];
+                if (c) s_cur[q] = atomicAdd(&qcursor[q], c);
+            }
+            __syncthreads();
+            for (unsigned long long base = b0 + warp * kFillStep; base < b1; base += kFillWarps * kFillStep) step(base, b1);
+            __syncthreads();  // the cursors are rewritten for the next block
+        }
+    } else {
+        const unsigned long long warps = (unsigned long long)gridDim.x * kFillWarps;
+        for (unsigned long long base = ((unsigned long long)blockIdx.x * kFillWarps + warp) * kFillStep; base < n;
+             base += warps * kFillStep)
+            step(base, n);
     }
+}
+
+// Gathers the keys of n_recs records of nq queries (qcursor zeroed).
+inline void launch_key_fill(const DevTable &t, const HitRec *recs, const unsigned long long *counters,
+                            unsigned long long n_recs, const uint64_t *qoff, uint32_t *qcursor, uint32_t nq, uint32_t *out,
+                            int sm_count, cudaStream_t st) {
+    const unsigned most = unsigned(sm_count) * 16;
+    if (nq <= kFillBlockQueries) {
+        const unsigned grid = std::max(1u, std::min(blocks_for(n_recs, kFillBlockRecs), most));
+        k_key_fill<true><<<grid, kFillThreads, nq * sizeof(uint32_t), st>>>(recs, counters, t.slot_key_off.p, t.tile_keys.p,
+                                                                           t.keys.p, qoff, qcursor, nq, out);
+    } else {
+        const unsigned grid = std::max(1u, std::min(blocks_for(n_recs, kFillThreads * kFillPerLane), most));
+        k_key_fill<false><<<grid, kFillThreads, 0, st>>>(recs, counters, t.slot_key_off.p, t.tile_keys.p, t.keys.p, qoff,
+                                                         qcursor, nq, out);
+    }
+    TM_CHECK_LAUNCH();
 }
 
 // ---------------------------------------------------------------------------

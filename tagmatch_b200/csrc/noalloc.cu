@@ -191,7 +191,6 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
 
     // keys
     ar.trim(recs + hc[1]);
-    const unsigned gblocks = std::max(1u, std::min(blocks_for(hc[1], kFillThreads * kFillPerLane), unsigned(sms) * 16));
     uint64_t *key_off = unique ? qoff : d_out_offsets;
     scan_fixed<uint32_t, uint64_t>(qkeys, key_off, nq, sums, offs, st);
     uint64_t total = 0;
@@ -201,8 +200,7 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
         *n_keys = total;
         if (total > capacity)
             throw Error(TM_ERR_CAPACITY, "output key buffer too small: " + std::to_string(total) + " keys needed");
-        k_key_fill<<<gblocks, kFillThreads, 0, st>>>(recs, counters, t.slot_key_off.p, t.tile_keys.p, t.keys.p, d_out_offsets, qcursor, d_out_keys);
-        TM_CHECK_LAUNCH();
+        launch_key_fill(t, recs, counters, hc[1], d_out_offsets, qcursor, nq, d_out_keys, sms, st);
         TM_CUDA(cudaStreamSynchronize(st));
         return;
     }
@@ -219,8 +217,7 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     const size_t second_bytes = bitmap ? bitmap_bytes : key_bytes;
     uint32_t *second = second_bytes <= rec_bytes ? reinterpret_cast<uint32_t *>(recs)
                                                  : ar.take<uint32_t>(second_bytes / sizeof(uint32_t), "match_unique keys");
-    k_key_fill<<<gblocks, kFillThreads, 0, st>>>(recs, counters, t.slot_key_off.p, t.tile_keys.p, t.keys.p, qoff, qcursor, keys);
-    TM_CHECK_LAUNCH();
+    launch_key_fill(t, recs, counters, hc[1], qoff, qcursor, nq, keys, sms, st);
     if (bitmap) {
         launch_unique_mark(keys, qoff, nq, words, second, ucount, sms, st);
     } else {
