@@ -194,24 +194,13 @@ int tm_balanced_partitioning(const uint32_t *filters, uint64_t n, uint32_t max_p
         tmb::gpu_partition(f.p, uint32_t(n), max_p, false, pr, st);
         const uint64_t np = pr.parts.size();
         *n_partitions = np;
-        std::vector<uint32_t> order(n), words(size_t(n) * TM_FILTER_WORDS);
-        if (n) {
-            TM_CUDA(cudaMemcpy(order.data(), pr.order.p, size_t(n) * 4, cudaMemcpyDeviceToHost));
-            TM_CUDA(cudaMemcpy(words.data(), pr.words.p, size_t(n) * 24, cudaMemcpyDeviceToHost));
-        }
-        for (uint64_t p = 0; p < np; ++p) {
-            const tmb::Range r = pr.parts[p];
-            uint32_t m[TM_FILTER_WORDS];
-            for (int k = 0; k < TM_FILTER_WORDS; ++k) m[k] = 0xFFFFFFFFu;
-            for (uint32_t i = r.begin; i < r.end; ++i) {
-                partition_of[order[i]] = uint32_t(p);
-                for (int k = 0; k < TM_FILTER_WORDS; ++k) m[k] &= words[size_t(i) * TM_FILTER_WORDS + k];
-            }
-            if (p < capacity) {
-                if (masks) std::memcpy(masks + p * TM_FILTER_WORDS, m, sizeof(m));
-                if (sizes) sizes[p] = r.end - r.begin;
-            }
-        }
+        tmb::DevBuf<uint32_t> of, ands;
+        tmb::assign_partitions(pr, of, ands, st);
+        const uint64_t fit = std::min<uint64_t>(np, capacity);
+        if (n) TM_CUDA(cudaMemcpy(partition_of, of.p, size_t(n) * 4, cudaMemcpyDeviceToHost));
+        if (masks && fit) TM_CUDA(cudaMemcpy(masks, ands.p, size_t(fit) * 24, cudaMemcpyDeviceToHost));
+        if (sizes)
+            for (uint64_t p = 0; p < fit; ++p) sizes[p] = pr.parts[p].end - pr.parts[p].begin;
         return np > capacity ? TM_ERR_CAPACITY : TM_OK;
     } catch (const tmb::Error &x) {
         return x.status;

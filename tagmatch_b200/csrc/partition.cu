@@ -37,6 +37,8 @@ namespace {
 
 constexpr int kPChunk = 1024;  // filters per partitioner chunk
 constexpr int kPThreads = 256;
+constexpr int kPeelThreads = 1024;
+constexpr uint32_t kPeelMax = 65536;  // filters of a range that one CTA peels: 64 per thread
 constexpr uint32_t kActFinal = 0x100;
 constexpr uint32_t kActChop = 0x200;
 // Exponent of the tile-split weight (1 - table frequency of the bit)^k.  A
@@ -50,6 +52,7 @@ struct Counters {
     uint32_t next_chunks;
     uint32_t finals;
     uint32_t leaves;
+    uint32_t peels;
 };
 
 __device__ __forceinline__ uint32_t find_seg(const uint32_t *chunk_off, uint32_t n_act, uint32_t chunk) {
@@ -267,6 +270,7 @@ struct ChildCtx {
     Seg *next;
     Range *finals;
     Range *leaves;
+    Seg *peel;
     Counters *cnt;
     uint32_t max_p;
     uint32_t finals_cap, leaves_cap;
@@ -300,11 +304,31 @@ __device__ void push_final(const ChildCtx &c, uint32_t b, uint32_t e) {
     }
 }
 
+// A range whose pivot mask is empty: peeled by one CTA when it is short
+// enough, level by level until it is.  There is one at most: such ranges
+// are the zero sides of zero sides of the whole table, or the zero side that
+// a peel leaves.
+__device__ void push_peel(const ChildCtx &c, uint32_t b, uint32_t e) {
+    if (e - b > kPeelMax) {
+        push_active(c, b, e, nullptr, kPhasePeel);
+        return;
+    }
+    c.cnt->peels = 1;
+    Seg s;
+    s.begin = b;
+    s.end = e;
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) s.used[i] = 0u;
+    s.flags = kPhasePeel;
+    s.pad = 0;
+    *c.peel = s;
+}
+
 // A side of a balancing split (the partition rules of do_balanced_partitioning).
 __device__ void balance_child(const ChildCtx &c, uint32_t b, uint32_t e, const uint32_t *used, bool mask_empty) {
     const uint32_t size = e - b;
     if (size > c.max_p) push_active(c, b, e, used, kPhaseBalance | (mask_empty ? kMaskEmpty : 0u));
-    else if (mask_empty && size > 0) push_active(c, b, e, nullptr, kPhasePeel);
+    else if (mask_empty && size > 0) push_peel(c, b, e);
     else push_final(c, b, e);
 }
 
@@ -332,7 +356,7 @@ __global__ void k_children(const Seg *__restrict__ segs, uint32_t n_act, const u
             balance_child(c, m, seg.end, used, false);
         } else if (phase == kPhasePeel) {
             push_final(c, m, seg.end);
-            push_active(c, seg.begin, m, nullptr, kPhasePeel);
+            push_peel(c, seg.begin, m);
         } else {
             tile_child(c, seg.begin, m, used);
             tile_child(c, m, seg.end, used);
@@ -342,6 +366,147 @@ __global__ void k_children(const Seg *__restrict__ segs, uint32_t n_act, const u
     } else {
         push_leaf(c, seg.begin, seg.end);  // cannot split further: chopped into tiles of 32
     }
+}
+
+// 32 x 32 bit transpose over a warp: bit j of lane i <- bit i of lane j.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, unsigned lane) {
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        const uint32_t low = s == 16 ? 0x0000FFFFu : s == 8 ? 0x00FF00FFu : s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
+        const uint32_t y = __shfl_xor_sync(kFull, x, s);
+        const bool up = (lane & s) != 0;
+        const uint32_t keep = up ? ~low : low;
+        x = (x & keep) | (__funnelshift_l(y, y, up ? 32 - s : s) & ~keep);
+    }
+    return x;
+}
+
+// Peels one range to its end (nonzero_mask_partitioning, partitioning.cc:
+// 230-250) in one CTA: while some bit is held by a part of the filters left,
+// those that hold the most frequent one (the first on ties) split off, behind
+// the rest and in order.  A filter's place follows from the peel that takes
+// it, so nothing moves until the end: each thread keeps a column of the
+// filters left (16-bit positions in shared memory) and drops what a peel
+// takes; the peeled filters' bits are subtracted from the bit counts; then
+// one stable scatter by peel number, last peel first.  Level by level, each of
+// up to 192 peels took eleven launches and a wait: 100 of the 110 levels of a
+// million filters, 10 of the call's 23 ms; this kernel takes 0.4 ms for them.
+// list: scratch as long as the filters (words_alt and order_alt are free too).
+__global__ void __launch_bounds__(kPeelThreads) k_peel(const Seg *__restrict__ seg_p, const uint32_t *__restrict__ freq,
+                                                       uint32_t *words, uint32_t *order, uint32_t *words_alt,
+                                                       uint32_t *order_alt, uint8_t *peel_of, ChildCtx c) {
+    constexpr int kWarps = kPeelThreads / 32;
+    constexpr int kMaxPeels = kBits + 1;
+    extern __shared__ uint16_t s_left[];  // [64][kPeelThreads] the threads' columns
+    __shared__ uint32_t s_cnt[kBits];     // filters left that hold the bit
+    __shared__ uint32_t s_size[kMaxPeels + 1], s_pos[kWarps][kMaxPeels], s_bit, s_listed;
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Seg seg = *seg_p;
+    const uint32_t n = seg.end - seg.begin;
+    const uint32_t *w0 = words + size_t(seg.begin) * kWords;
+    uint8_t *cls = peel_of + seg.begin;
+    uint32_t *list = order_alt + seg.begin;  // peeled filters, free until the scatter
+    if (tid < kBits) s_cnt[tid] = freq[tid];
+    if (tid == 0) s_listed = 0;
+    uint32_t left = 0;
+    for (uint32_t i = tid; i < n; i += kPeelThreads) s_left[left++ * kPeelThreads + tid] = uint16_t(i);
+    uint32_t total = n, peel = 0;
+    __syncthreads();
+    for (;; ++peel) {
+        if (warp == 0) {
+            unsigned long long best = ~0ull;
+#pragma unroll
+            for (int k = 0; k < kWords; ++k) {
+                const uint32_t b = k * 32 + lane;
+                const unsigned long long key = ((unsigned long long)(0xFFFFFFFFu - s_cnt[b]) << 8) | b;  // first maximum
+                best = key < best ? key : best;
+            }
+            best = warp_min_u64(best);
+            const uint32_t maxf = 0xFFFFFFFFu - uint32_t(best >> 8);
+            // all filters left share the bit, or are all-zero: the last part
+            if (lane == 0) s_bit = maxf == total || maxf == 0 ? kActFinal : uint32_t(best & 0xFF);
+        }
+        __syncthreads();
+        const uint32_t bit = s_bit, listed = s_listed;
+        __syncthreads();  // both are rewritten
+        if (bit == kActFinal) break;
+        // drop the column's filters that hold the bit, four loads in flight
+        uint32_t kept = 0;
+        for (uint32_t j = 0; j < left; j += 4) {
+            uint32_t e[4], x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                e[u] = j + u < left ? s_left[(j + u) * kPeelThreads + tid] : 0u;
+                x[u] = j + u < left ? w0[size_t(e[u]) * kWords + (bit >> 5)] : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (j + u >= left) break;
+                if ((x[u] >> (bit & 31)) & 1u) {
+                    cls[e[u]] = uint8_t(peel);
+                    list[atomicAdd(&s_listed, 1u)] = e[u];
+                } else {
+                    s_left[kept++ * kPeelThreads + tid] = uint16_t(e[u]);
+                }
+            }
+        }
+        left = kept;
+        __syncthreads();
+        // subtract the peeled filters' bits, 32 filters per warp at a time
+        const uint32_t end = s_listed;
+        for (uint32_t g = listed + warp * 32; g < end; g += kPeelThreads) {
+            const bool have = g + lane < end;
+            const uint32_t e = have ? list[g + lane] : 0u;
+#pragma unroll
+            for (int k = 0; k < kWords; ++k) {
+                const uint32_t held = __popc(transpose32(have ? w0[size_t(e) * kWords + k] : 0u, lane));
+                if (held) atomicSub(&s_cnt[k * 32 + lane], held);
+            }
+        }
+        if (tid == 0) s_size[peel] = end - listed;
+        total -= end - listed;
+        __syncthreads();
+    }
+    for (uint32_t j = 0; j < left; ++j) cls[s_left[j * kPeelThreads + tid]] = uint8_t(peel);
+    if (tid == 0) s_size[peel] = total;
+    // stable scatter: part p lies before the parts of the earlier peels
+    for (uint32_t i = tid; i < uint32_t(kWarps * kMaxPeels); i += kPeelThreads) (&s_pos[0][0])[i] = 0;
+    __syncthreads();
+    const uint32_t per = ((n + kWarps - 1) / kWarps + 31) & ~31u;
+    const uint32_t r0 = min(n, warp * per), r1 = min(n, r0 + per);
+    for (uint32_t i = r0 + lane; i < r1; i += 32) atomicAdd(&s_pos[warp][cls[i]], 1u);
+    __syncthreads();
+    if (tid <= peel) {
+        uint32_t at = n;
+        for (uint32_t p = 0; p <= tid; ++p) at -= s_size[p];
+        push_final(c, seg.begin + at, seg.begin + at + s_size[tid]);
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t k = s_pos[w][tid];
+            s_pos[w][tid] = at;
+            at += k;
+        }
+    }
+    __syncthreads();
+    for (uint32_t g = r0; g < r1; g += 32) {
+        const bool have = g + lane < r1;
+        const uint32_t i = have ? g + lane : 0u;
+        const uint32_t p = have ? cls[i] : 256u + lane;  // absent lanes match no one
+        const uint32_t same = __match_any_sync(kFull, p);
+        const uint32_t rank = __popc(same & ((1u << lane) - 1u));
+        uint32_t at = have ? s_pos[warp][p] : 0u;
+        __syncwarp();
+        if (have && rank == 0) s_pos[warp][p] = at + __popc(same);
+        __syncwarp();
+        if (have) {
+            at += rank;
+#pragma unroll
+            for (int k = 0; k < kWords; ++k) words_alt[size_t(seg.begin + at) * kWords + k] = w0[size_t(i) * kWords + k];
+            order_alt[seg.begin + at] = order[seg.begin + i];
+        }
+    }
+    __syncthreads();
+    for (size_t i = size_t(seg.begin) * kWords + tid; i < size_t(seg.end) * kWords; i += kPeelThreads) words[i] = words_alt[i];
+    for (uint32_t i = seg.begin + tid; i < seg.end; i += kPeelThreads) order[i] = order_alt[i];
 }
 
 __global__ void k_mark_tiles(const Range *__restrict__ leaves, uint32_t n_leaves, uint32_t *__restrict__ mark) {
@@ -381,10 +546,13 @@ void gpu_partition(const uint32_t *d_filters, uint32_t n, uint32_t max_p, bool w
     DevBuf<uint32_t> nch, chunk_off, freq, action, zc;
     DevBuf<uint64_t> zoff;
     DevBuf<Range> finals, leaves;
+    DevBuf<Seg> peel;
+    DevBuf<uint8_t> peel_of;
     DevBuf<Counters> cnt;
     DevBuf<float> weights;
     ScanScratch scr;
     cnt.reserve(1);
+    peel.reserve(1);
     weights.reserve(kBits);
     uint32_t finals_cap = n + 1024;
     uint32_t leaves_cap = with_tiles ? n + 1 : 1;
@@ -444,9 +612,9 @@ void gpu_partition(const uint32_t *d_filters, uint32_t n, uint32_t max_p, bool w
         k_copy_back<<<total_chunks, kPThreads, 0, st>>>(segs[cur].p, chunk_off.p, n_act, alt_words.p, alt_order.p, out.words.p,
                                                        out.order.p);
         TM_CHECK_LAUNCH();
-        segs[cur ^ 1].reserve(size_t(n_act) * 2 + 2);
+        segs[cur ^ 1].reserve(size_t(n_act) * 2 + kBits + 3);  // and the parts of a peeled range
         TM_CUDA(cudaMemsetAsync(&cnt.p->next, 0, 2 * sizeof(uint32_t), st));
-        ChildCtx c{segs[cur ^ 1].p, finals.p, leaves.p, cnt.p, max_p, finals_cap, leaves_cap, with_tiles};
+        ChildCtx c{segs[cur ^ 1].p, finals.p, leaves.p, peel.p, cnt.p, max_p, finals_cap, leaves_cap, with_tiles};
         k_children<<<blocks_for(n_act, 128), 128, 0, st>>>(segs[cur].p, n_act, action.p, chunk_off.p, zoff.p, c);
         TM_CHECK_LAUNCH();
         TM_CUDA(cudaMemcpyAsync(&hc, cnt.p, sizeof(Counters), cudaMemcpyDeviceToHost, st));
@@ -455,6 +623,31 @@ void gpu_partition(const uint32_t *d_filters, uint32_t n, uint32_t max_p, bool w
         n_act = hc.next;
         total_chunks = hc.next_chunks;
         cur ^= 1;
+        // the range to peel, with its bit counts; its parts may become tile
+        // ranges, which join the next level
+        if (hc.peels) {
+            Seg ps;
+            TM_CUDA(cudaMemcpyAsync(&ps, peel.p, sizeof(Seg), cudaMemcpyDeviceToHost, st));
+            TM_CUDA(cudaStreamSynchronize(st));
+            const uint32_t zero_off[2] = {0, (ps.end - ps.begin + kPChunk - 1) / kPChunk};
+            peel_of.reserve(n);
+            TM_CUDA(cudaMemcpyAsync(chunk_off.p, zero_off, sizeof(zero_off), cudaMemcpyHostToDevice, st));
+            TM_CUDA(cudaMemsetAsync(freq.p, 0, kBits * sizeof(uint32_t), st));
+            k_freq<<<zero_off[1], kPThreads, 0, st>>>(peel.p, chunk_off.p, 1, out.words.p, freq.p);
+            TM_CHECK_LAUNCH();
+            TM_CUDA(cudaMemsetAsync(&cnt.p->peels, 0, sizeof(uint32_t), st));
+            ChildCtx pc{segs[cur].p, finals.p, leaves.p, peel.p, cnt.p, max_p, finals_cap, leaves_cap, with_tiles};
+            constexpr int columns = int(sizeof(uint16_t)) * int(kPeelMax);
+            TM_CUDA(cudaFuncSetAttribute(k_peel, cudaFuncAttributeMaxDynamicSharedMemorySize, columns));
+            k_peel<<<1, kPeelThreads, columns, st>>>(peel.p, freq.p, out.words.p, out.order.p, alt_words.p, alt_order.p,
+                                                     peel_of.p, pc);
+            TM_CHECK_LAUNCH();
+            TM_CUDA(cudaMemcpyAsync(&hc, cnt.p, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+            TM_CUDA(cudaStreamSynchronize(st));
+            if (hc.finals > finals_cap || hc.leaves > leaves_cap) throw Error(TM_ERR_INTERNAL, "partitioner list overflow");
+            n_act = hc.next;
+            total_chunks = hc.next_chunks;
+        }
     }
 
     // partitions in position order
@@ -472,6 +665,56 @@ void gpu_partition(const uint32_t *d_filters, uint32_t n, uint32_t max_p, bool w
             TM_CHECK_LAUNCH();
         }
     }
+    TM_CUDA(cudaStreamSynchronize(st));
+}
+
+namespace {
+
+// Position i of the partitioner's order -> its partition (ranges sorted by
+// position), stored at the filter's original index, and the partition's AND.
+__global__ void k_assign(const uint32_t *__restrict__ words, const uint32_t *__restrict__ order, uint32_t n,
+                         const Range *__restrict__ parts, uint32_t n_parts, uint32_t *__restrict__ partition_of,
+                         uint32_t *__restrict__ masks) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t p = 0xFFFFFFFFu;
+    if (i < n) {
+        uint32_t lo = 0, hi = n_parts;  // last partition that begins at or before i
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (parts[mid].begin <= i) lo = mid;
+            else hi = mid;
+        }
+        p = lo;
+        partition_of[order[i]] = p;
+    }
+    // a warp inside one partition adds its AND once
+    const uint32_t p0 = __shfl_sync(kFull, p, 0);
+    const bool one = __all_sync(kFull, p == p0 || i >= n);
+#pragma unroll
+    for (int k = 0; k < kWords; ++k) {
+        const uint32_t w = i < n ? words[size_t(i) * kWords + k] : 0xFFFFFFFFu;
+        const uint32_t all = __reduce_and_sync(kFull, w);
+        if (one) {
+            if ((threadIdx.x & 31) == 0 && i < n) atomicAnd(&masks[size_t(p) * kWords + k], all);
+        } else if (i < n) {
+            atomicAnd(&masks[size_t(p) * kWords + k], w);
+        }
+    }
+}
+
+}  // namespace
+
+void assign_partitions(const PartitionResult &pr, DevBuf<uint32_t> &partition_of, DevBuf<uint32_t> &masks, cudaStream_t st) {
+    const uint32_t P = uint32_t(pr.parts.size());
+    partition_of.reserve(std::max<uint32_t>(pr.n, 1));
+    masks.reserve(size_t(std::max<uint32_t>(P, 1)) * kWords);
+    if (!pr.n || !P) return;
+    DevBuf<Range> parts;
+    parts.reserve(P);
+    TM_CUDA(cudaMemcpyAsync(parts.p, pr.parts.data(), sizeof(Range) * P, cudaMemcpyHostToDevice, st));
+    TM_CUDA(cudaMemsetAsync(masks.p, 0xFF, size_t(P) * kWords * sizeof(uint32_t), st));
+    k_assign<<<blocks_for(pr.n, 256), 256, 0, st>>>(pr.words.p, pr.order.p, pr.n, parts.p, P, partition_of.p, masks.p);
+    TM_CHECK_LAUNCH();
     TM_CUDA(cudaStreamSynchronize(st));
 }
 

@@ -60,6 +60,10 @@ struct DevTable {
 void gpu_partition(const uint32_t *d_filters, uint32_t n, uint32_t max_p, bool with_tiles, PartitionResult &out,
                    cudaStream_t st);
 
+// Each filter's partition (by original index) and each partition's AND of its
+// members (all ones when it has none), on the device.
+void assign_partitions(const PartitionResult &pr, DevBuf<uint32_t> &partition_of, DevBuf<uint32_t> &masks, cudaStream_t st);
+
 // Builds the matcher table from a partitioning run (with_tiles) and the
 // per-filter keys (CSR over the original filter order, on the device).
 void build_table(const PartitionResult &pr, const uint32_t *d_key_off, const uint32_t *d_keys, uint64_t n_keys,
