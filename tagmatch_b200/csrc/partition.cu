@@ -39,6 +39,7 @@ constexpr int kPChunk = 1024;  // filters per partitioner chunk
 constexpr int kPThreads = 256;
 constexpr int kPeelThreads = 1024;
 constexpr uint32_t kPeelMax = 65536;  // filters of a range that one CTA peels: 64 per thread
+constexpr uint32_t kSmallRange = 1024;  // filters of a tile range that one warp splits to its end
 constexpr uint32_t kActFinal = 0x100;
 constexpr uint32_t kActChop = 0x200;
 // Exponent of the tile-split weight (1 - table frequency of the bit)^k.  A
@@ -53,6 +54,7 @@ struct Counters {
     uint32_t finals;
     uint32_t leaves;
     uint32_t peels;
+    uint32_t small;
 };
 
 __device__ __forceinline__ uint32_t find_seg(const uint32_t *chunk_off, uint32_t n_act, uint32_t chunk) {
@@ -271,6 +273,7 @@ struct ChildCtx {
     Range *finals;
     Range *leaves;
     Seg *peel;
+    Seg *small;  // short tile ranges, split to their end by k_split_small
     Counters *cnt;
     uint32_t max_p;
     uint32_t finals_cap, leaves_cap;
@@ -290,6 +293,22 @@ __device__ void push_active(const ChildCtx &c, uint32_t b, uint32_t e, const uin
     atomicAdd(&c.cnt->next_chunks, (e - b + kPChunk - 1) / kPChunk);
 }
 
+// A tile range: short ones are put aside for k_split_small.
+__device__ void push_tile_range(const ChildCtx &c, uint32_t b, uint32_t e, const uint32_t *used) {
+    if (e - b > kSmallRange) {
+        push_active(c, b, e, used, kPhaseTile);
+        return;
+    }
+    Seg s;
+    s.begin = b;
+    s.end = e;
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) s.used[i] = used ? used[i] : 0u;
+    s.flags = kPhaseTile;
+    s.pad = 0;
+    c.small[atomicAdd(&c.cnt->small, 1u)] = s;
+}
+
 __device__ void push_leaf(const ChildCtx &c, uint32_t b, uint32_t e) {
     uint32_t k = atomicAdd(&c.cnt->leaves, 1u);
     if (k < c.leaves_cap) c.leaves[k] = Range{b, e};
@@ -299,7 +318,7 @@ __device__ void push_final(const ChildCtx &c, uint32_t b, uint32_t e) {
     uint32_t k = atomicAdd(&c.cnt->finals, 1u);
     if (k < c.finals_cap) c.finals[k] = Range{b, e};
     if (c.with_tiles) {
-        if (e - b > (uint32_t)kTile) push_active(c, b, e, nullptr, kPhaseTile);
+        if (e - b > (uint32_t)kTile) push_tile_range(c, b, e, nullptr);
         else if (e > b) push_leaf(c, b, e);
     }
 }
@@ -333,7 +352,7 @@ __device__ void balance_child(const ChildCtx &c, uint32_t b, uint32_t e, const u
 }
 
 __device__ void tile_child(const ChildCtx &c, uint32_t b, uint32_t e, const uint32_t *used) {
-    if (e - b > (uint32_t)kTile) push_active(c, b, e, used, kPhaseTile);
+    if (e - b > (uint32_t)kTile) push_tile_range(c, b, e, used);
     else if (e > b) push_leaf(c, b, e);
 }
 
@@ -390,11 +409,12 @@ __device__ __forceinline__ uint32_t transpose32(uint32_t x, unsigned lane) {
 // takes; the peeled filters' bits are subtracted from the bit counts; then
 // one stable scatter by peel number, last peel first.  Level by level, each of
 // up to 192 peels took eleven launches and a wait: 100 of the 110 levels of a
-// million filters, 10 of the call's 23 ms; this kernel takes 0.4 ms for them.
-// list: scratch as long as the filters (words_alt and order_alt are free too).
+// a million filters, 10 of the call's 23 ms.
+// pos: the filters' places, first the list of peeled filters; as long as the
+// range, as peel_of is.
 __global__ void __launch_bounds__(kPeelThreads) k_peel(const Seg *__restrict__ seg_p, const uint32_t *__restrict__ freq,
-                                                       uint32_t *words, uint32_t *order, uint32_t *words_alt,
-                                                       uint32_t *order_alt, uint8_t *peel_of, ChildCtx c) {
+                                                       const uint32_t *__restrict__ words, uint32_t *pos, uint8_t *peel_of,
+                                                       ChildCtx c) {
     constexpr int kWarps = kPeelThreads / 32;
     constexpr int kMaxPeels = kBits + 1;
     extern __shared__ uint16_t s_left[];  // [64][kPeelThreads] the threads' columns
@@ -404,8 +424,8 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel(const Seg *__restrict__ s
     const Seg seg = *seg_p;
     const uint32_t n = seg.end - seg.begin;
     const uint32_t *w0 = words + size_t(seg.begin) * kWords;
-    uint8_t *cls = peel_of + seg.begin;
-    uint32_t *list = order_alt + seg.begin;  // peeled filters, free until the scatter
+    uint8_t *cls = peel_of;
+    uint32_t *list = pos;
     if (tid < kBits) s_cnt[tid] = freq[tid];
     if (tid == 0) s_listed = 0;
     uint32_t left = 0;
@@ -497,16 +517,120 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel(const Seg *__restrict__ s
         __syncwarp();
         if (have && rank == 0) s_pos[warp][p] = at + __popc(same);
         __syncwarp();
-        if (have) {
-            at += rank;
-#pragma unroll
-            for (int k = 0; k < kWords; ++k) words_alt[size_t(seg.begin + at) * kWords + k] = w0[size_t(i) * kWords + k];
-            order_alt[seg.begin + at] = order[seg.begin + i];
-        }
+        if (have) pos[i] = at + rank;
     }
-    __syncthreads();
-    for (size_t i = size_t(seg.begin) * kWords + tid; i < size_t(seg.end) * kWords; i += kPeelThreads) words[i] = words_alt[i];
-    for (uint32_t i = seg.begin + tid; i < seg.end; i += kPeelThreads) order[i] = order_alt[i];
+}
+
+// Moves the peeled range's filters to their places.
+__global__ void k_peel_move(const Seg *__restrict__ seg_p, const uint32_t *__restrict__ pos, const uint32_t *__restrict__ words,
+                            const uint32_t *__restrict__ order, uint32_t *__restrict__ words_out,
+                            uint32_t *__restrict__ order_out) {
+    const Seg seg = *seg_p;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= seg.end - seg.begin) return;
+    const size_t from = size_t(seg.begin) + i, to = size_t(seg.begin) + pos[i];
+#pragma unroll
+    for (int k = 0; k < kWords; ++k) words_out[to * kWords + k] = words[from * kWords + k];
+    order_out[to] = order[from];
+}
+
+// Splits a short tile range to its end, one warp per range: the rules of
+// k_decide and tile_child, over a stack of sub-ranges instead of a level of
+// launches per depth (the tile splits are uneven: 250,000 filters took 81
+// levels, 7 of the 54 ms of a consolidation).  The filters lie in shared
+// memory and only their 16-bit positions move; bit counts of a sub-range are
+// bit transposes of 32 filters and popcounts, lane l counting bit l of each
+// word.  34 KB per warp, so six warps share an SM.
+struct SmallRange {
+    uint32_t b, e, used[kWords];
+};
+struct SplitSmem {
+    uint32_t w[kWords][kSmallRange];
+    uint32_t order[kSmallRange];
+    uint16_t at[kSmallRange], ones[kSmallRange];
+    SmallRange stack[kSmallRange / kTile];  // pending sub-ranges are disjoint and longer than a tile
+};
+
+__global__ void __launch_bounds__(32) k_split_small(uint32_t *__restrict__ words, uint32_t *__restrict__ order,
+                                                    const float *__restrict__ tile_weight, ChildCtx c) {
+    extern __shared__ __align__(16) unsigned char split_raw[];
+    SplitSmem &S = *reinterpret_cast<SplitSmem *>(split_raw);
+    const unsigned lane = threadIdx.x;
+    const Seg seg = c.small[blockIdx.x];
+    const uint32_t n = seg.end - seg.begin;
+    for (uint32_t i = lane; i < n * kWords; i += 32) S.w[i % kWords][i / kWords] = words[size_t(seg.begin) * kWords + i];
+    for (uint32_t i = lane; i < n; i += 32) {
+        S.order[i] = order[seg.begin + i];
+        S.at[i] = uint16_t(i);
+    }
+    float weight[kWords];
+#pragma unroll
+    for (int k = 0; k < kWords; ++k) weight[k] = tile_weight[k * 32 + lane];
+    if (lane == 0) {
+        S.stack[0].b = 0;
+        S.stack[0].e = n;
+        for (int k = 0; k < kWords; ++k) S.stack[0].used[k] = seg.used[k];
+    }
+    __syncwarp();
+    for (uint32_t depth = 1; depth;) {
+        const SmallRange r = S.stack[--depth];
+        const uint32_t size = r.e - r.b;
+        uint32_t f[kWords] = {0, 0, 0, 0, 0, 0};
+        for (uint32_t g = r.b; g < r.e; g += 32) {
+            const bool have = g + lane < r.e;
+            const uint32_t i = have ? S.at[g + lane] : 0u;
+#pragma unroll
+            for (int k = 0; k < kWords; ++k) f[k] += __popc(transpose32(have ? S.w[k][i] : 0u, lane));
+        }
+        unsigned long long best = ~0ull;
+#pragma unroll
+        for (int k = 0; k < kWords; ++k) {
+            if (f[k] > 0 && f[k] < size && !((r.used[k] >> lane) & 1u)) {
+                const float score = float(f[k]) * weight[k];
+                const unsigned long long key = ((unsigned long long)(~__float_as_uint(score)) << 8) | (k * 32 + lane);
+                best = key < best ? key : best;
+            }
+        }
+        best = warp_min_u64(best);
+        if (best == ~0ull) {  // cannot split further: chopped into tiles of 32
+            if (lane == 0) push_leaf(c, seg.begin + r.b, seg.begin + r.e);
+            continue;
+        }
+        const uint32_t bit = uint32_t(best & 0xFF);
+        // stable split: the zero side moves up, the one side waits in `ones`
+        uint32_t zeros = 0, ones = 0;
+        for (uint32_t g = r.b; g < r.e; g += 32) {
+            const bool have = g + lane < r.e;
+            const uint32_t i = have ? S.at[g + lane] : 0u;
+            const bool one = have && ((S.w[bit >> 5][i] >> (bit & 31)) & 1u);
+            const uint32_t m1 = __ballot_sync(kFull, one), m0 = __ballot_sync(kFull, have && !one);
+            const uint32_t below = (1u << lane) - 1u;
+            if (one) S.ones[ones + __popc(m1 & below)] = uint16_t(i);
+            else if (have) S.at[r.b + zeros + __popc(m0 & below)] = uint16_t(i);
+            ones += __popc(m1);
+            zeros += __popc(m0);
+            __syncwarp();
+        }
+        const uint32_t mid = r.b + zeros;
+        for (uint32_t j = lane; j < ones; j += 32) S.at[mid + j] = S.ones[j];
+        if (lane == 0) {
+            SmallRange child = r;
+            child.used[bit >> 5] |= 1u << (bit & 31);
+            const uint32_t edge[3] = {r.b, mid, r.e};
+            uint32_t d = depth;
+            for (int s = 0; s < 2; ++s) {
+                child.b = edge[s];
+                child.e = edge[s + 1];
+                if (child.e - child.b > (uint32_t)kTile) S.stack[d++] = child;
+                else if (child.e > child.b) push_leaf(c, seg.begin + child.b, seg.begin + child.e);
+            }
+        }
+        depth += (zeros > (uint32_t)kTile ? 1u : 0u) + (ones > (uint32_t)kTile ? 1u : 0u);
+        __syncwarp();
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < n * kWords; i += 32) words[size_t(seg.begin) * kWords + i] = S.w[i % kWords][S.at[i / kWords]];
+    for (uint32_t i = lane; i < n; i += 32) order[seg.begin + i] = S.order[S.at[i]];
 }
 
 __global__ void k_mark_tiles(const Range *__restrict__ leaves, uint32_t n_leaves, uint32_t *__restrict__ mark) {
@@ -543,16 +667,17 @@ void gpu_partition(const uint32_t *d_filters, uint32_t n, uint32_t max_p, bool w
     alt_words.reserve(size_t(n) * kWords);
     alt_order.reserve(n);
     DevBuf<Seg> segs[2];
-    DevBuf<uint32_t> nch, chunk_off, freq, action, zc;
+    DevBuf<uint32_t> nch, chunk_off, freq, action, zc, peel_pos;
     DevBuf<uint64_t> zoff;
     DevBuf<Range> finals, leaves;
-    DevBuf<Seg> peel;
+    DevBuf<Seg> peel, small;
     DevBuf<uint8_t> peel_of;
     DevBuf<Counters> cnt;
     DevBuf<float> weights;
     ScanScratch scr;
     cnt.reserve(1);
     peel.reserve(1);
+    if (with_tiles) small.reserve(n / (kTile + 1) + 1);  // disjoint ranges, each longer than a tile
     weights.reserve(kBits);
     uint32_t finals_cap = n + 1024;
     uint32_t leaves_cap = with_tiles ? n + 1 : 1;
@@ -614,7 +739,7 @@ void gpu_partition(const uint32_t *d_filters, uint32_t n, uint32_t max_p, bool w
         TM_CHECK_LAUNCH();
         segs[cur ^ 1].reserve(size_t(n_act) * 2 + kBits + 3);  // and the parts of a peeled range
         TM_CUDA(cudaMemsetAsync(&cnt.p->next, 0, 2 * sizeof(uint32_t), st));
-        ChildCtx c{segs[cur ^ 1].p, finals.p, leaves.p, peel.p, cnt.p, max_p, finals_cap, leaves_cap, with_tiles};
+        ChildCtx c{segs[cur ^ 1].p, finals.p, leaves.p, peel.p, small.p, cnt.p, max_p, finals_cap, leaves_cap, with_tiles};
         k_children<<<blocks_for(n_act, 128), 128, 0, st>>>(segs[cur].p, n_act, action.p, chunk_off.p, zoff.p, c);
         TM_CHECK_LAUNCH();
         TM_CUDA(cudaMemcpyAsync(&hc, cnt.p, sizeof(Counters), cudaMemcpyDeviceToHost, st));
@@ -629,25 +754,41 @@ void gpu_partition(const uint32_t *d_filters, uint32_t n, uint32_t max_p, bool w
             Seg ps;
             TM_CUDA(cudaMemcpyAsync(&ps, peel.p, sizeof(Seg), cudaMemcpyDeviceToHost, st));
             TM_CUDA(cudaStreamSynchronize(st));
-            const uint32_t zero_off[2] = {0, (ps.end - ps.begin + kPChunk - 1) / kPChunk};
-            peel_of.reserve(n);
+            const uint32_t np = ps.end - ps.begin, zero_off[2] = {0, (np + kPChunk - 1) / kPChunk};
+            peel_of.reserve(np);
+            peel_pos.reserve(np);
             TM_CUDA(cudaMemcpyAsync(chunk_off.p, zero_off, sizeof(zero_off), cudaMemcpyHostToDevice, st));
             TM_CUDA(cudaMemsetAsync(freq.p, 0, kBits * sizeof(uint32_t), st));
             k_freq<<<zero_off[1], kPThreads, 0, st>>>(peel.p, chunk_off.p, 1, out.words.p, freq.p);
             TM_CHECK_LAUNCH();
             TM_CUDA(cudaMemsetAsync(&cnt.p->peels, 0, sizeof(uint32_t), st));
-            ChildCtx pc{segs[cur].p, finals.p, leaves.p, peel.p, cnt.p, max_p, finals_cap, leaves_cap, with_tiles};
+            ChildCtx pc{segs[cur].p, finals.p, leaves.p, peel.p, small.p, cnt.p, max_p, finals_cap, leaves_cap, with_tiles};
             constexpr int columns = int(sizeof(uint16_t)) * int(kPeelMax);
             TM_CUDA(cudaFuncSetAttribute(k_peel, cudaFuncAttributeMaxDynamicSharedMemorySize, columns));
-            k_peel<<<1, kPeelThreads, columns, st>>>(peel.p, freq.p, out.words.p, out.order.p, alt_words.p, alt_order.p,
-                                                     peel_of.p, pc);
+            k_peel<<<1, kPeelThreads, columns, st>>>(peel.p, freq.p, out.words.p, peel_pos.p, peel_of.p, pc);
             TM_CHECK_LAUNCH();
+            k_peel_move<<<blocks_for(np, 256), 256, 0, st>>>(peel.p, peel_pos.p, out.words.p, out.order.p, alt_words.p,
+                                                             alt_order.p);
+            TM_CHECK_LAUNCH();
+            TM_CUDA(cudaMemcpyAsync(out.words.p + size_t(ps.begin) * kWords, alt_words.p + size_t(ps.begin) * kWords,
+                                    size_t(np) * kWords * 4, cudaMemcpyDeviceToDevice, st));
+            TM_CUDA(cudaMemcpyAsync(out.order.p + ps.begin, alt_order.p + ps.begin, size_t(np) * 4, cudaMemcpyDeviceToDevice, st));
             TM_CUDA(cudaMemcpyAsync(&hc, cnt.p, sizeof(Counters), cudaMemcpyDeviceToHost, st));
             TM_CUDA(cudaStreamSynchronize(st));
             if (hc.finals > finals_cap || hc.leaves > leaves_cap) throw Error(TM_ERR_INTERNAL, "partitioner list overflow");
             n_act = hc.next;
             total_chunks = hc.next_chunks;
         }
+    }
+
+    if (hc.small) {
+        ChildCtx sc{nullptr, finals.p, leaves.p, peel.p, small.p, cnt.p, max_p, finals_cap, leaves_cap, with_tiles};
+        TM_CUDA(cudaFuncSetAttribute(k_split_small, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SplitSmem))));
+        k_split_small<<<hc.small, 32, sizeof(SplitSmem), st>>>(out.words.p, out.order.p, weights.p, sc);
+        TM_CHECK_LAUNCH();
+        TM_CUDA(cudaMemcpyAsync(&hc, cnt.p, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+        TM_CUDA(cudaStreamSynchronize(st));
+        if (hc.leaves > leaves_cap) throw Error(TM_ERR_INTERNAL, "partitioner list overflow");
     }
 
     // partitions in position order

@@ -59,3 +59,22 @@ def test_table_with_peeled_tiles(n, max_p):
         off, keys = tm.match_batch(q)
     eoff, ekeys = oracle.match(f, ko, k, q)
     assert_same_multisets(off, keys, eoff, ekeys)
+
+
+@pytest.mark.parametrize("n", [32, 33, 64, 1023, 1024, 1025, 2049, 5000])
+@pytest.mark.parametrize("shared_bit", [False, True])
+def test_table_around_one_warp_ranges(n, shared_bit):
+    """Tile ranges around what one warp splits to its end (1,024 filters); a bit
+    that all filters share keeps them in one partition."""
+    f, ko, k = workload.generate_filters(n, 73)
+    if shared_bit:
+        f = np.unique(f | np.array([1, 0, 0, 0, 0, 0], dtype=np.uint32), axis=0)
+        ko, k = ko[: f.shape[0] + 1], k[: ko[f.shape[0]]]
+    q = workload.generate_queries(200, f, 73)
+    with TagMatch() as tm:
+        tm.set_persistence(False)
+        tm.add_many(f, ko, k)
+        tm.consolidate(65536, 1)
+        off, keys = tm.match_batch(q)
+    eoff, ekeys = oracle.match(f, ko, k, q)
+    assert_same_multisets(off, keys, eoff, ekeys)
