@@ -104,12 +104,37 @@ bool read_db(const std::string &fn, std::vector<Entry> &out, std::map<FilterKey,
     return true;
 }
 
+unsigned worker_threads() { return std::max(1u, std::min(32u, std::thread::hardware_concurrency())); }
+
+// Runs f(0) .. f(n - 1), each on a thread of its own (one alone on the
+// caller's).  An exception of f (memory) is thrown again here.
+template <class F>
+void on_threads(unsigned n, F f) {
+    if (n == 1) {
+        f(0u);
+        return;
+    }
+    std::vector<std::exception_ptr> failed(n);
+    std::vector<std::thread> ts;
+    for (unsigned t = 0; t < n; ++t)
+        ts.emplace_back([&, t] {
+            try {
+                f(t);
+            } catch (...) {
+                failed[t] = std::current_exception();
+            }
+        });
+    for (auto &x : ts) x.join();
+    for (auto &e : failed)
+        if (e) std::rethrow_exception(e);
+}
+
 // Sorts v with cmp on all hardware threads: sorted chunks, then pairwise
 // merges.
 template <class T, class Cmp>
 void parallel_sort(std::vector<T> &v, Cmp cmp) {
     const size_t n = v.size();
-    const unsigned th = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
+    const unsigned th = worker_threads();
     if (n < (size_t(1) << 16) || th == 1) {
         std::sort(v.begin(), v.end(), cmp);
         return;
@@ -219,10 +244,9 @@ void Engine::add_many(const uint32_t *filters, uint64_t n, const uint32_t *key_o
     std::lock_guard<std::mutex> lk(api_mtx_);
     if (bulk_koff_.empty()) bulk_koff_.push_back(0);
     bulk_words_.insert(bulk_words_.end(), filters, filters + n * kWords);
-    for (uint64_t i = 0; i < n; ++i) {
-        bulk_keys_.insert(bulk_keys_.end(), keys + key_off[i], keys + key_off[i + 1]);
-        bulk_koff_.push_back(bulk_keys_.size());
-    }
+    const uint64_t base = bulk_keys_.size();
+    if (n) bulk_keys_.insert(bulk_keys_.end(), keys + key_off[0], keys + key_off[n]);
+    for (uint64_t i = 0; i < n; ++i) bulk_koff_.push_back(base + (key_off[i + 1] - key_off[0]));
 }
 
 void Engine::clear_bulk() {
@@ -265,48 +289,99 @@ void Engine::consolidate_bulk() {
     filters_.clear();
     key_off_.assign(1, 0);
     keys_.clear();
-    filters_.reserve(m * kWords);
-    key_off_.reserve(m + 1);
-    keys_.reserve(bulk_keys_.size());
-    std::vector<uint32_t> ks;
-    auto emit = [&](const uint32_t *w, std::vector<uint32_t> &kv) {
-        if (kv.empty()) return;
-        filters_.insert(filters_.end(), w, w + kWords);
-        keys_.insert(keys_.end(), kv.begin(), kv.end());
-        if (keys_.size() >= 0xFFFFFFFFull) throw Error(TM_ERR_INVALID, "table too large (2^32 keys)");
-        key_off_.push_back(uint32_t(keys_.size()));
-    };
-    auto it = updates_.begin();
-    size_t i = 0;
-    while (i < m || it != updates_.end()) {
-        const bool take_map = i == m || (it != updates_.end() && less_words(it->first.w.data(), v[i].w));
-        if (take_map) {
+    auto same = [](const SortEntry &a, const SortEntry &b) { return std::memcmp(a.w, b.w, 24) == 0; };
+    if (updates_.empty()) {
+        // nothing staged beside the bulk adds: stretches of whole groups of
+        // equal filters on all threads, then put together
+        struct Stretch {
+            std::vector<uint32_t> filters, counts, keys;
+        };
+        const unsigned th = unsigned(std::max<size_t>(1, std::min<size_t>(worker_threads(), m / 4096)));
+        std::vector<size_t> edge(th + 1);
+        for (unsigned t = 0; t <= th; ++t) {
+            size_t at = m * t / th;
+            while (at > 0 && at < m && same(v[at - 1], v[at])) ++at;
+            edge[t] = at;
+        }
+        std::vector<Stretch> part(th);
+        on_threads(th, [&](unsigned t) {
+            Stretch &x = part[t];
+            x.filters.reserve((edge[t + 1] - edge[t]) * kWords);
+            x.counts.reserve(edge[t + 1] - edge[t]);
+            x.keys.reserve(size_t(double(bulk_keys_.size()) * double(edge[t + 1] - edge[t]) / double(m) * 1.1) + 64);
+            for (size_t i = edge[t], j; i < edge[t + 1]; i = j) {
+                const size_t k0 = x.keys.size();
+                for (j = i; j < edge[t + 1] && same(v[i], v[j]); ++j) {
+                    const uint32_t e = v[j].idx;
+                    x.keys.insert(x.keys.end(), bulk_keys_.begin() + bulk_koff_[e], bulk_keys_.begin() + bulk_koff_[e + 1]);
+                }
+                if (x.keys.size() == k0) continue;  // no keys: dropped
+                std::sort(x.keys.begin() + k0, x.keys.end());
+                x.keys.erase(std::unique(x.keys.begin() + k0, x.keys.end()), x.keys.end());
+                x.filters.insert(x.filters.end(), v[i].w, v[i].w + kWords);
+                x.counts.push_back(uint32_t(x.keys.size() - k0));
+            }
+        });
+        std::vector<size_t> f0(th + 1, 0), k0(th + 1, 0);
+        for (unsigned t = 0; t < th; ++t) {
+            f0[t + 1] = f0[t] + part[t].counts.size();
+            k0[t + 1] = k0[t] + part[t].keys.size();
+        }
+        if (k0[th] >= 0xFFFFFFFFull) throw Error(TM_ERR_INVALID, "table too large (2^32 keys)");
+        filters_.resize(f0[th] * kWords);
+        key_off_.resize(f0[th] + 1);
+        keys_.resize(k0[th]);
+        on_threads(th, [&](unsigned t) {
+            const Stretch &x = part[t];
+            std::copy(x.filters.begin(), x.filters.end(), filters_.begin() + f0[t] * kWords);
+            std::copy(x.keys.begin(), x.keys.end(), keys_.begin() + k0[t]);
+            uint32_t at = uint32_t(k0[t]);
+            for (size_t i = 0; i < x.counts.size(); ++i) key_off_[f0[t] + i + 1] = at += x.counts[i];
+        });
+    } else {
+        filters_.reserve(m * kWords);
+        key_off_.reserve(m + 1);
+        keys_.reserve(bulk_keys_.size());
+        std::vector<uint32_t> ks;
+        auto emit = [&](const uint32_t *w, std::vector<uint32_t> &kv) {
+            if (kv.empty()) return;
+            filters_.insert(filters_.end(), w, w + kWords);
+            keys_.insert(keys_.end(), kv.begin(), kv.end());
+            if (keys_.size() >= 0xFFFFFFFFull) throw Error(TM_ERR_INVALID, "table too large (2^32 keys)");
+            key_off_.push_back(uint32_t(keys_.size()));
+        };
+        auto it = updates_.begin();
+        size_t i = 0;
+        while (i < m || it != updates_.end()) {
+            const bool take_map = i == m || (it != updates_.end() && less_words(it->first.w.data(), v[i].w));
+            if (take_map) {
+                ks.clear();
+                it->second.apply(ks);
+                emit(it->first.w.data(), ks);
+                ++it;
+                continue;
+            }
+            // one group of equal filters from the bulk adds
+            size_t j = i;
             ks.clear();
-            it->second.apply(ks);
-            emit(it->first.w.data(), ks);
-            ++it;
-            continue;
+            while (j < m && std::memcmp(v[j].w, v[i].w, 24) == 0) {
+                const uint32_t e = v[j].idx;
+                ks.insert(ks.end(), bulk_keys_.begin() + bulk_koff_[e], bulk_keys_.begin() + bulk_koff_[e + 1]);
+                ++j;
+            }
+            if (it != updates_.end() && std::memcmp(it->first.w.data(), v[i].w, 24) == 0) {
+                KeysetChange c = it->second;
+                c.to_add.insert(ks.begin(), ks.end());
+                ks.clear();
+                c.apply(ks);
+                ++it;
+            } else {
+                std::sort(ks.begin(), ks.end());
+                ks.erase(std::unique(ks.begin(), ks.end()), ks.end());
+            }
+            emit(v[i].w, ks);
+            i = j;
         }
-        // one group of equal filters from the bulk adds
-        size_t j = i;
-        ks.clear();
-        while (j < m && std::memcmp(v[j].w, v[i].w, 24) == 0) {
-            const uint32_t e = v[j].idx;
-            ks.insert(ks.end(), bulk_keys_.begin() + bulk_koff_[e], bulk_keys_.begin() + bulk_koff_[e + 1]);
-            ++j;
-        }
-        if (it != updates_.end() && std::memcmp(it->first.w.data(), v[i].w, 24) == 0) {
-            KeysetChange c = it->second;
-            c.to_add.insert(ks.begin(), ks.end());
-            ks.clear();
-            c.apply(ks);
-            ++it;
-        } else {
-            std::sort(ks.begin(), ks.end());
-            ks.erase(std::unique(ks.begin(), ks.end()), ks.end());
-        }
-        emit(v[i].w, ks);
-        i = j;
     }
     updates_.clear();
     clear_bulk();

@@ -655,34 +655,56 @@ void gpu_partition(const uint32_t *d_filters, uint32_t n, uint32_t max_p, bool w
     out.n = n;
     out.parts.clear();
     out.bit_freq.assign(kBits, 0);
-    out.words.reserve(size_t(n) * kWords);
-    out.order.reserve(n);
-    if (with_tiles) out.tile_mark.reserve(n);
-    if (n == 0) return;
+    if (n == 0) {
+        out.words.reserve(1);
+        out.order.reserve(1);
+        if (with_tiles) out.tile_mark.reserve(1);
+        return;
+    }
+    DevPieces kept;
+    kept.want(out.words, size_t(n) * kWords);
+    kept.want(out.order, n);
+    if (with_tiles) kept.want(out.tile_mark, n);
+    kept.allocate(out.block);
     TM_CUDA(cudaMemcpyAsync(out.words.p, d_filters, size_t(n) * kWords * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
     k_init_order<<<blocks_for(n, 256), 256, 0, st>>>(out.order.p, n);
     TM_CHECK_LAUNCH();
 
-    DevBuf<uint32_t> alt_words, alt_order;
-    alt_words.reserve(size_t(n) * kWords);
-    alt_order.reserve(n);
-    DevBuf<Seg> segs[2];
-    DevBuf<uint32_t> nch, chunk_off, freq, action, zc, peel_pos;
+    // the working buffers; those sized by the ranges of a level grow past
+    // what they start with when a level has more
+    DevBuf<unsigned char> block;
+    DevBuf<uint32_t> alt_words, alt_order, nch, chunk_off, freq, action, zc, peel_pos;
     DevBuf<uint64_t> zoff;
+    DevBuf<Seg> segs[2], peel, small;
     DevBuf<Range> finals, leaves;
-    DevBuf<Seg> peel, small;
     DevBuf<uint8_t> peel_of;
     DevBuf<Counters> cnt;
     DevBuf<float> weights;
     ScanScratch scr;
-    cnt.reserve(1);
-    peel.reserve(1);
-    if (with_tiles) small.reserve(n / (kTile + 1) + 1);  // disjoint ranges, each longer than a tile
-    weights.reserve(kBits);
-    uint32_t finals_cap = n + 1024;
-    uint32_t leaves_cap = with_tiles ? n + 1 : 1;
-    finals.reserve(finals_cap);
-    leaves.reserve(leaves_cap);
+    const uint32_t finals_cap = n + 1024, leaves_cap = with_tiles ? n + 1 : 1;
+    const size_t level = 1024, chunks = (size_t(n) + kPChunk - 1) / kPChunk + level, peeled = std::min(n, kPeelMax);
+    DevPieces work;
+    work.want(alt_words, size_t(n) * kWords);
+    work.want(alt_order, n);
+    work.want(finals, finals_cap);
+    work.want(leaves, leaves_cap);
+    work.want(cnt, 1);
+    work.want(peel, 1);
+    work.want(small, with_tiles ? n / (kTile + 1) + 1 : 1);  // disjoint ranges, each longer than a tile
+    work.want(weights, kBits);
+    work.want(segs[0], 2 * level);
+    work.want(segs[1], 2 * level);
+    work.want(nch, level);
+    work.want(chunk_off, level + 1);
+    work.want(freq, level * kBits);
+    work.want(action, level);
+    work.want(zc, chunks);
+    work.want(zoff, chunks + 1);
+    work.want(peel_pos, peeled);
+    work.want(peel_of, peeled);
+    work.want(scr.levels[0], chunks / kScanTile + 1);
+    work.want(scr.levels[1], chunks / kScanTile + 2);
+    work.allocate(block);
 
     // root
     Seg root;
@@ -1011,9 +1033,18 @@ void build_table(const PartitionResult &pr, const uint32_t *d_key_off, const uin
     t.n_parts = uint32_t(pr.parts.size());
     t.n_keys = n_keys;
     ScanScratch scr;
-    DevBuf<uint32_t> mark_off, tile_begin, nkeys;
+    DevBuf<unsigned char> block;
+    DevBuf<uint32_t> mark_off, tile_begin, nkeys, mk;
+    DevBuf<uint8_t> bit_order;
     DevBuf<Range> parts;
-    mark_off.reserve(size_t(n) + 1);
+    DevPieces work;
+    work.want(mark_off, size_t(n) + 1);
+    work.want(parts, t.n_parts);
+    work.want(bit_order, kBits);
+    work.want(mk, 1);
+    work.want(scr.levels[0], size_t(n) / kScanTile + 2);
+    work.want(scr.levels[1], size_t(n) / kScanTile + 3);
+    work.allocate(block);
     if (n) {
         exclusive_scan<uint32_t, uint32_t>(pr.tile_mark.p, mark_off.p, n, scr, st);
         TM_CUDA(cudaMemcpyAsync(&t.n_tiles, mark_off.p + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -1046,8 +1077,6 @@ void build_table(const PartitionResult &pr, const uint32_t *d_key_off, const uin
     for (int b = 0; b < kBits; ++b) order_h[b] = uint8_t(b);
     std::stable_sort(order_h.begin(), order_h.end(),
                      [&](uint8_t x, uint8_t y) { return pr.bit_freq[x] < pr.bit_freq[y]; });
-    DevBuf<uint8_t> bit_order;
-    bit_order.reserve(kBits);
     TM_CUDA(cudaMemcpyAsync(bit_order.p, order_h.data(), kBits, cudaMemcpyHostToDevice, st));
     if (nt) {
         k_build_tiles<<<blocks_for(size_t(nt) * 32, 256), 256, 0, st>>>(pr.words.p, pr.order.p, tile_begin.p, nt,
@@ -1081,8 +1110,6 @@ void build_table(const PartitionResult &pr, const uint32_t *d_key_off, const uin
         k_tile_keys<<<blocks_for(size_t(nt) * 32, 256), 256, 0, st>>>(t.slot_key_off.p, nt, t.tile_keys.p);
         TM_CHECK_LAUNCH();
     }
-    DevBuf<uint32_t> mk;
-    mk.reserve(1);
     TM_CUDA(cudaMemsetAsync(mk.p, 0, sizeof(uint32_t), st));
     if (n_keys) {
         k_max_key<<<256, 256, 0, st>>>(t.keys.p, n_keys, mk.p);

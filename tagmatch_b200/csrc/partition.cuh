@@ -29,6 +29,7 @@ struct Range {
 struct PartitionResult {
     uint32_t n = 0;                  // filters
     std::vector<Range> parts;        // partitions in id order (sorted by position)
+    DevBuf<unsigned char> block;     // holds the buffers below
     DevBuf<uint32_t> words;          // [n][6] filters in partition order
     DevBuf<uint32_t> order;          // [n] original index of each position
     DevBuf<uint32_t> tile_mark;      // [n] 1 where a tile starts (with_tiles only)

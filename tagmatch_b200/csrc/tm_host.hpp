@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 namespace tmb {
 
@@ -36,21 +37,35 @@ template <class T>
 struct DevBuf {
     T *p = nullptr;
     size_t cap = 0;
+    bool owned = true;  // false: part of another allocation (borrow)
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), cap(o.cap) { o.p = nullptr; o.cap = 0; }
+    DevBuf(DevBuf &&o) noexcept : p(o.p), cap(o.cap), owned(o.owned) { o.forget(); }
     DevBuf &operator=(DevBuf &&o) noexcept {
         if (this != &o) {
             release();
             p = o.p;
             cap = o.cap;
-            o.p = nullptr;
-            o.cap = 0;
+            owned = o.owned;
+            o.forget();
         }
         return *this;
     }
     ~DevBuf() { release(); }
+    // Starts on n elements at q, which the caller keeps alive; growing past
+    // them takes an allocation of its own.
+    void borrow(T *q, size_t n) {
+        release();
+        p = q;
+        cap = n;
+        owned = false;
+    }
+    void forget() {
+        p = nullptr;
+        cap = 0;
+        owned = true;
+    }
     // Grows by at least half the current capacity, so a slowly growing
     // demand reallocates (and frees, which synchronises the device) rarely.
     void reserve(size_t n) {
@@ -68,11 +83,41 @@ struct DevBuf {
         cap = n ? n : 1;
     }
     void release() {
-        if (p) cudaFree(p);
-        p = nullptr;
-        cap = 0;
+        if (p && owned) cudaFree(p);
+        forget();
     }
     T *get() const { return p; }
+};
+
+// One device allocation cut into 256-byte aligned pieces, for calls that need
+// many buffers at once (an allocation and its release take 0.1-0.3 ms each).
+// want() states the pieces, then allocate() hands them out.
+class DevPieces {
+public:
+    template <class T>
+    void want(DevBuf<T> &b, size_t n) {
+        const size_t count = n ? n : 1;
+        pieces_.push_back(Piece{&b, total_, count, [](void *buf, unsigned char *at, size_t elements) {
+                                    static_cast<DevBuf<T> *>(buf)->borrow(reinterpret_cast<T *>(at), elements);
+                                }});
+        total_ = (total_ + count * sizeof(T) + 255) & ~size_t(255);
+    }
+    // block must outlive the buffers
+    void allocate(DevBuf<unsigned char> &block) {
+        block.reserve(total_);
+        for (const Piece &x : pieces_) x.hand(x.buf, block.p + x.at, x.count);
+        pieces_.clear();
+        total_ = 0;
+    }
+
+private:
+    struct Piece {
+        void *buf;
+        size_t at, count;
+        void (*hand)(void *, unsigned char *, size_t);
+    };
+    size_t total_ = 0;
+    std::vector<Piece> pieces_;
 };
 
 // Pinned host buffer (grow-only).
