@@ -189,15 +189,27 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     const uint32_t *order = ordered ? s.d_part_order.p : nullptr;
     s.part_off.reserve(size_t(P) + 1);
     s.chunk_off.reserve(size_t(P) + 1);
-    s.item_off.reserve(size_t(P) + 1);
-    k_plan<<<1, kPlanThreads, 0, st>>>(part_count, t.part_tile_begin.p, order, P, s.seg_tiles, s.part_off.p, s.chunk_off.p,
-                                       s.item_off.p);
+    s.item_off.reserve(size_t(P) + 2);
+    // batches whose items are timed for the cost model take the tiles per item
+    // as they are set: the model learns their effect
+    const uint32_t least = least_seg(nq);
+    const uint32_t want_items = s.record_items ? 0 : uint32_t(s.sm_count) * 4 * kItemsPerCta;
+    k_plan<<<1, kPlanThreads, 0, st>>>(part_count, t.part_tile_begin.p, order, P, s.seg_tiles, least, want_items, s.part_off.p,
+                                       s.chunk_off.p, s.item_off.p, s.item_off.p + P + 1);
     TM_CHECK_LAUNCH();
     // the host's copy of the plan, once the counts are back
     uint32_t items = 0, chunks = 0;
     auto host_plan = [&](const uint32_t *counts) {
         s.h_part_count.assign(counts, counts + P);
         s.h_item_off.resize(size_t(P) + 1);
+        uint32_t seg = s.seg_tiles;  // as k_plan chooses it
+        for (int h = 0; want_items && h < kSegHalvings; ++h) {
+            uint64_t total = 0;
+            for (uint32_t p = 0; p < P; ++p)
+                total += part_items(counts[p], t.h_part_tiles[p + 1] - t.h_part_tiles[p], halved_seg(s.seg_tiles, h, least));
+            if (total >= want_items) break;
+            seg = halved_seg(s.seg_tiles, h + 1, least);
+        }
         for (uint32_t pos = 0; pos < P; ++pos) {
             bs.routed += counts[pos];
             bs.dense += uint64_t(counts[pos]) * t.h_part_size[pos];
@@ -207,9 +219,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
             const uint32_t p = ordered ? s.part_order[pos] : pos;
             s.h_item_off[pos] = items;
             // an item: kItemChunks chunks of the partition x one tile segment
-            const uint32_t ng = (counts[p] + kItemQueries - 1) / kItemQueries;
-            const uint32_t nt = t.h_part_tiles[p + 1] - t.h_part_tiles[p];
-            items += ng * ((nt + s.seg_tiles - 1) / s.seg_tiles);
+            items += part_items(counts[p], t.h_part_tiles[p + 1] - t.h_part_tiles[p], seg);
         }
         s.h_item_off[P] = items;
         bs.items = items;
@@ -247,7 +257,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
             TM_CUDA(cudaMemsetAsync(s.item_stats.p, 0, 2 * size_t(items) * sizeof(unsigned long long), st));
         }
         MatchArgs a{t.tile_words.p, t.tile_info.p, t.tile_keys.p, t.slot_key_off.p, t.part_tile_begin.p, part_count,
-                    s.part_off.p, s.item_off.p, s.chunk_off.p, queue_lo, queue_hi, s.slices.p, P, s.seg_tiles, counters,
+                    s.part_off.p, s.item_off.p, s.chunk_off.p, queue_lo, queue_hi, s.slices.p, P, s.item_off.p + P + 1, counters,
                     s.recs.p, (unsigned long long)s.recs.cap, qkeys, fpl_trip_cost(), order, s.record_items ? s.item_stats.p : nullptr,
                     work_counters ? s.work.p : nullptr};
         if (match_begin && attempt == 0) TM_CUDA(cudaEventRecord(match_begin, st));

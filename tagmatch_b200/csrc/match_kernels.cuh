@@ -97,17 +97,62 @@ __global__ void __launch_bounds__(kRouteThreads) k_route(const uint32_t *__restr
     }
 }
 
+// Tiles per work item of a batch: the configured number, halved until the
+// batch has kItemsPerCta items for each of the subset test's CTAs, or an item
+// would no longer give its eight warps a step of tiles each.  With fewer items
+// than that a batch takes as long as its largest item: 1,000 queries on a
+// million filters make 312 items of 128 tiles for 592 CTAs.  Measured
+// there and with 2,000 queries on 300,000 (us): as configured 374 and 512,
+// with 2 items per CTA 322 and 428, with 4 309 and 430; with 8 the claims cost
+// what they even out.
+constexpr uint32_t kItemsPerCta = 4;
+constexpr int kSegHalvings = 5;
+__host__ __device__ inline uint32_t least_seg(uint32_t nq) {
+    uint32_t tiles = 32;  // a warp's tiles per step, for items of nq queries
+    for (uint32_t words = (nq + 31) / 32; tiles > 1 && words > 1; words = (words + 1) / 2) tiles /= 2;
+    return kMatchWarps * tiles;
+}
+__host__ __device__ inline uint32_t halved_seg(uint32_t seg, int halvings, uint32_t least) {
+    const uint32_t s = seg >> halvings;
+    return s > least ? s : seg < least ? seg : least;
+}
+// Work items of a partition with `count` queries and nt tiles.
+__host__ __device__ inline uint32_t part_items(uint32_t count, uint32_t nt, uint32_t seg) {
+    return (count + kItemQueries - 1) / kItemQueries * ((nt + seg - 1) / seg);
+}
+
 // Offsets of the work plan from the partitions' counts, one CTA: queue
 // positions, 256-query chunks, and work items (groups of kItemChunks chunks
 // x tile segments), the items over queue positions (order: the partition at
-// each position; null: id order).
+// each position; null: id order).  *seg_out: tiles per item, from seg_tiles
+// and the items wanted (0: seg_tiles as it is).
 __global__ void __launch_bounds__(kPlanThreads) k_plan(const uint32_t *__restrict__ part_count,
                                                        const uint32_t *__restrict__ part_tile_begin,
                                                        const uint32_t *__restrict__ order, uint32_t n_parts,
-                                                       uint32_t seg_tiles, uint32_t *__restrict__ part_off,
-                                                       uint32_t *__restrict__ chunk_off, uint32_t *__restrict__ item_off) {
+                                                       uint32_t seg_tiles, uint32_t least, uint32_t want_items,
+                                                       uint32_t *__restrict__ part_off, uint32_t *__restrict__ chunk_off,
+                                                       uint32_t *__restrict__ item_off, uint32_t *__restrict__ seg_out) {
     __shared__ uint32_t s_sum[3][kPlanThreads / 32];
+    __shared__ uint32_t s_items[kSegHalvings];  // items are counted in 32 bits
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t seg = seg_tiles;
+    if (want_items) {
+        if (threadIdx.x < kSegHalvings) s_items[threadIdx.x] = 0;
+        __syncthreads();
+        uint32_t items[kSegHalvings] = {};
+        for (uint32_t p = threadIdx.x; p < n_parts; p += kPlanThreads) {
+            const uint32_t count = part_count[p], nt = part_tile_begin[p + 1] - part_tile_begin[p];
+#pragma unroll
+            for (int h = 0; h < kSegHalvings; ++h) items[h] += part_items(count, nt, halved_seg(seg_tiles, h, least));
+        }
+#pragma unroll
+        for (int h = 0; h < kSegHalvings; ++h) {
+            const uint32_t sum = __reduce_add_sync(kFull, items[h]);
+            if (lane == 0 && sum) atomicAdd(&s_items[h], sum);
+        }
+        __syncthreads();
+        for (int h = 0; h < kSegHalvings && s_items[h] < want_items; ++h) seg = halved_seg(seg_tiles, h + 1, least);
+    }
     uint32_t base[3] = {0, 0, 0};
     for (uint32_t t0 = 0; t0 < n_parts; t0 += kPlanThreads) {
         const uint32_t pos = t0 + threadIdx.x;
@@ -116,8 +161,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(const uint32_t *__restric
             v[0] = part_count[pos];
             v[1] = (v[0] + kChunk - 1) / kChunk;
             const uint32_t p = order ? order[pos] : pos;
-            const uint32_t nt = part_tile_begin[p + 1] - part_tile_begin[p];
-            v[2] = ((part_count[p] + kItemQueries - 1) / kItemQueries) * ((nt + seg_tiles - 1) / seg_tiles);
+            v[2] = part_items(part_count[p], part_tile_begin[p + 1] - part_tile_begin[p], seg);
         }
         uint32_t incl[3];
 #pragma unroll
@@ -140,6 +184,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(const uint32_t *__restric
         part_off[n_parts] = base[0];
         chunk_off[n_parts] = base[1];
         item_off[n_parts] = base[2];
+        *seg_out = seg;
     }
 }
 
@@ -338,7 +383,7 @@ struct MatchArgs {
     const uint4 *queue_lo, *queue_hi;
     const uint32_t *slices;
     uint32_t n_parts;
-    uint32_t seg_tiles;            // tiles per work item
+    const uint32_t *seg;           // tiles per work item (k_plan)
     // [0] next item, [1] hit records, [2] error flags, [3] matching
     // (query, filter) pairs
     unsigned long long *counters;
@@ -416,7 +461,7 @@ struct ItemRef {
     uint32_t qbase, nq, tb, te, zchunk;
 };
 
-__device__ __forceinline__ ItemRef locate(const MatchArgs &a, uint32_t item) {
+__device__ __forceinline__ ItemRef locate(const MatchArgs &a, uint32_t item, uint32_t seg_tiles) {
     uint32_t lo = 0, hi = a.n_parts;
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
@@ -431,8 +476,8 @@ __device__ __forceinline__ ItemRef locate(const MatchArgs &a, uint32_t item) {
     const uint32_t group = local % ngroups, seg = local / ngroups;
     r.qbase = a.part_off[lo] + group * kItemQueries;
     r.nq = min((uint32_t)kItemQueries, pq - group * kItemQueries);
-    r.tb = a.part_tile_begin[lo] + seg * a.seg_tiles;
-    r.te = min(r.tb + a.seg_tiles, a.part_tile_begin[lo + 1]);
+    r.tb = a.part_tile_begin[lo] + seg * seg_tiles;
+    r.te = min(r.tb + seg_tiles, a.part_tile_begin[lo + 1]);
     r.zchunk = a.chunk_off[lo] + group * kItemChunks;
     return r;
 }
@@ -444,7 +489,7 @@ __device__ __forceinline__ bool produce(const MatchArgs &a, uint32_t total, Matc
     const uint32_t item = uint32_t(atomicAdd(&a.counters[0], 1ull));
     S.item = item;
     if (item < total) {
-        const ItemRef r = locate(a, item);
+        const ItemRef r = locate(a, item, *a.seg);
         const uint32_t bytes = r.nq * sizeof(uint4);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(&S.full, 2 * bytes);
@@ -596,7 +641,7 @@ __global__ void __launch_bounds__(kMatchThreads, 4) k_match(MatchArgs a) {  // 4
         }
         const uint32_t item = S.item;
         if (__any_sync(kFull, item >= total || S.fail)) break;
-        const ItemRef r = locate(a, item);
+        const ItemRef r = locate(a, item, *a.seg);
         if (COUNT) ++w_items;
         long long item_c0 = 0;
         uint32_t item_recs0 = 0;

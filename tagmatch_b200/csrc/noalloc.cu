@@ -127,7 +127,7 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     uint32_t *part_count = ar.take<uint32_t>(P, "partition counts");
     uint32_t *part_off = ar.take<uint32_t>(size_t(P) + 1, "partition offsets");
     uint32_t *chunk_off = ar.take<uint32_t>(size_t(P) + 1, "plan");
-    uint32_t *item_off = ar.take<uint32_t>(size_t(P) + 1, "plan");
+    uint32_t *item_off = ar.take<uint32_t>(size_t(P) + 2, "plan");
     // block sums of a scan over at most kNoAllocMaxQueries
     constexpr size_t kScanBlocks = (kNoAllocMaxQueries + kScanTile - 1) / kScanTile;
     uint64_t *sums = ar.take<uint64_t>(kScanBlocks, "scan");
@@ -153,7 +153,8 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     uint32_t *rows = rows_at_end(window);
     for (uint32_t p0 = 0; p0 < P; p0 += window)
         launch_route(true, d_queries, nq, t, p0, std::min(P, p0 + window), rows, part_count, nullptr, st);
-    k_plan<<<1, kPlanThreads, 0, st>>>(part_count, t.part_tile_begin.p, nullptr, P, seg_tiles, part_off, chunk_off, item_off);
+    k_plan<<<1, kPlanThreads, 0, st>>>(part_count, t.part_tile_begin.p, nullptr, P, seg_tiles, least_seg(nq),
+                                       uint32_t(sms) * 4 * kItemsPerCta, part_off, chunk_off, item_off, item_off + P + 1);
     TM_CHECK_LAUNCH();
     uint32_t routed = 0, chunks = 0;
     TM_CUDA(cudaMemcpyAsync(&routed, part_off + P, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -177,7 +178,7 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     if (rec_room < 256) throw Error(TM_ERR_CAPACITY, "no-allocation scratch exhausted before the hit records; split the batch");
     HitRec *recs = ar.take<HitRec>(rec_room - 32, "hit records");
     MatchArgs a{t.tile_words.p, t.tile_info.p, t.tile_keys.p, t.slot_key_off.p, t.part_tile_begin.p, part_count, part_off,
-                item_off, chunk_off, queue, queue + routed, slices, P, seg_tiles, counters, recs, (unsigned long long)(rec_room - 32), qkeys,
+                item_off, chunk_off, queue, queue + routed, slices, P, item_off + P + 1, counters, recs, (unsigned long long)(rec_room - 32), qkeys,
                 fpl_trip_cost(), nullptr, nullptr, nullptr};
     launch_match<false>(a, unsigned(sms) * 4, st);
     TM_CHECK_LAUNCH();
