@@ -26,7 +26,10 @@ constexpr int kSliceWords = kSliceRows * 8;  // 193 x 256 bits
 constexpr int kRouteThreads = 256;        // queries per routing CTA
 constexpr uint32_t kRouteParts = 64;      // partition masks per routing CTA
 constexpr uint32_t kGroupQueries = 8192;  // queries per count group: 256 words of a partition's routing row
-constexpr uint32_t kFillRanks = 2048;     // queue positions per queue-filling CTA (8 chunks)
+// Queue positions per queue-filling CTA (4 chunks; 20,011 queries on 125
+// partitions: 72 us with 2,048 positions, 59 with 1,024, 57 with 512, where
+// 65,536 on 382 take 345, 351 and 371).
+constexpr uint32_t kFillRanks = 1024;
 constexpr int kPlanThreads = 1024;
 
 // Words of one partition's routing row (a bit per query, whole CTAs).
@@ -205,7 +208,7 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, unsigned lane) {
 
 // Fills the partitions' queues from their routing rows (partitions
 // [p0, p0 + gridDim.x)): CTA (p, y) takes the queries of positions
-// [2048 y, 2048 y + 2048), finds them in the row (counts per group, then a
+// [1024 y, 1024 y + 1024), finds them in the row (counts per group, then a
 // prefix sum over a group's words), and per 256-query chunk writes the queue
 // records (words 0 .. 3 in one plane; words 4 and 5, the query id and a pad
 // in the other) and the chunk's bit-sliced masks: z[b * 8 + w] bit l is set when query 32 w + l of the chunk
