@@ -4,6 +4,7 @@
 // translation unit gets its own internal copy.
 #pragma once
 #include <algorithm>
+#include <type_traits>
 #include "match.cuh"
 
 namespace tmb {
@@ -420,7 +421,8 @@ struct MatchSmem {
     HitRec rec[kMatchWarps][kWarpRecs];                  // staged hit records per warp
     // candidate lists per warp: 1024 / T bytes for each of the T tiles it
     // selects for at once, the chunks' candidates in chunk order (query index
-    // in its chunk), padded to a multiple of 4
+    // in its chunk); trips read up to the next multiple of 4, what lies there
+    // is any query of the item and its hits are dropped
     uint8_t list[kMatchWarps][kItemQueries];
     uint4 tf[kMatchWarps][kWords][kTile / 4];            // a warp's tile: word k of filters 4 g .. 4 g + 3
     uint64_t full, empty;
@@ -568,8 +570,8 @@ __device__ __forceinline__ void test_queries(const uint4 (*tf)[kTile / 4], uint3
 //    words);
 // then, tile by tile, over the candidates of all chunks together (one pass
 // over the tile's filters for up to 1,024 queries: fuller passes and trips):
-//  * many candidates: candidate queries over the lanes (two per lane while
-//    more than 32 are left, then one), the tile's filters read from shared
+//  * many candidates, or an item of more than 512 queries: candidate queries
+//    over the lanes (two per lane while more than 32 are left, then one), the tile's filters read from shared
 //    memory (test_queries), the lane's hit mask over the tile built bit by
 //    bit;
 //  * few candidates: one filter per lane (the tile in registers), four
@@ -653,154 +655,168 @@ __global__ void __launch_bounds__(kMatchThreads, 4) k_match(MatchArgs a) {  // 4
             item_recs0 = w_recs;
         }
         // lanes per tile: the item's 32-query words, as a power of two
+        // (all lanes for more than 512 queries).  Wide items are compiled by
+        // themselves: with the lanes' roles known, the scan unrolled, no loop
+        // over tiles and only the lane-per-query path (few of their tiles
+        // have few candidates), 65,536 queries on ten million filters take
+        // 24.9 ms instead of 27.1.  More cases, or the second path, cost more
+        // in the instruction cache than they save: 500 queries, whose items
+        // have 4 to 16 words, went from 0.58 to 0.86 ms with a case for 16.
         const uint32_t words = (r.nq + 31) >> 5;
-        const uint32_t lg = words > 1 ? 32 - __clz(words - 1) : 0u, tiles = 32u >> lg;
-        const uint32_t wi = lane & ((1u << lg) - 1u), gi = lane >> lg;  // the lane's word, its tile of the step
-        const uint32_t last = lane | ((1u << lg) - 1u);                   // the last lane of its tile
-        // queries of the lane's word, and its slices
-        const uint32_t live = wi * 32 + 32 <= r.nq ? kFull : wi * 32 >= r.nq ? 0u : (1u << (r.nq - wi * 32)) - 1u;
-        const uint32_t *zl = a.slices + (size_t(r.zchunk) + (wi >> 3)) * kSliceWords + (wi & 7);
-        for (uint32_t t0 = r.tb + warp * tiles; t0 < r.te; t0 += kMatchWarps * tiles) {
-            const uint32_t tq = t0 + gi;
-            uint32_t cand = 0, tcount = 0;
-            if (tq < r.te && live) {  // words past the item's queries have no slices
-                const TileInfo ti = a.tile_info[tq];
-                tcount = ti.count;
-                const uint32_t lack =
-                    __ldg(&zl[(ti.sel[0] & 0xFFu) * 8]) | __ldg(&zl[((ti.sel[0] >> 8) & 0xFFu) * 8]) |
-                    __ldg(&zl[((ti.sel[0] >> 16) & 0xFFu) * 8]) | __ldg(&zl[(ti.sel[0] >> 24) * 8]) |
-                    __ldg(&zl[(ti.sel[1] & 0xFFu) * 8]) | __ldg(&zl[((ti.sel[1] >> 8) & 0xFFu) * 8]) |
-                    __ldg(&zl[((ti.sel[1] >> 16) & 0xFFu) * 8]) | __ldg(&zl[(ti.sel[1] >> 24) * 8]);
-                cand = ~lack & live;
-            }
-            if (COUNT) w_tiles += __popc(__ballot_sync(kFull, tq < r.te && wi == 0));  // lane 0 reports
-            // candidate lists (query index in its chunk, one byte each): a
-            // prefix sum over each tile's words places every lane's queries,
-            // from the word's highest down
-            const uint32_t cnt = __popc(cand);
-            uint32_t incl = cnt;
-            for (uint32_t o = 1; o < (1u << lg); o <<= 1) {
-                const uint32_t v = __shfl_up_sync(kFull, incl, o);
-                if (wi >= o) incl += v;
-            }
-            {
-                uint8_t *at = list + ((gi << lg) << 5) + incl;
-                if (lane == last) {
-                    // pad to a multiple of 4 (its hits are dropped)
-                    for (uint32_t x = incl; x & 3u; ++x) at[x - incl] = 0;
+        auto all_tiles = [&](auto wide) {
+            constexpr bool kWide = decltype(wide)::value;
+            const uint32_t lg = kWide ? 5u : words > 1 ? 32 - __clz(words - 1) : 0u, tiles = 32u >> lg;
+            const uint32_t wi = lane & ((1u << lg) - 1u), gi = lane >> lg;  // the lane's word, its tile of the step
+            const uint32_t last = lane | ((1u << lg) - 1u);                   // the last lane of its tile
+            // queries of the lane's word, and its slices
+            const uint32_t live = wi * 32 + 32 <= r.nq ? kFull : wi * 32 >= r.nq ? 0u : (1u << (r.nq - wi * 32)) - 1u;
+            const uint32_t *zl = a.slices + (size_t(r.zchunk) + (wi >> 3)) * kSliceWords + (wi & 7);
+            for (uint32_t t0 = r.tb + warp * tiles; t0 < r.te; t0 += kMatchWarps * tiles) {
+                const uint32_t tq = t0 + gi;
+                uint32_t cand = 0, tcount = 0;
+                if (kWide || tq < r.te) {
+                    const TileInfo ti = a.tile_info[tq];
+                    tcount = ti.count;
+                    if (live) {  // words past the item's queries have no slices
+                        const uint32_t lack =
+                            __ldg(&zl[(ti.sel[0] & 0xFFu) * 8]) | __ldg(&zl[((ti.sel[0] >> 8) & 0xFFu) * 8]) |
+                            __ldg(&zl[((ti.sel[0] >> 16) & 0xFFu) * 8]) | __ldg(&zl[(ti.sel[0] >> 24) * 8]) |
+                            __ldg(&zl[(ti.sel[1] & 0xFFu) * 8]) | __ldg(&zl[((ti.sel[1] >> 8) & 0xFFu) * 8]) |
+                            __ldg(&zl[((ti.sel[1] >> 16) & 0xFFu) * 8]) | __ldg(&zl[(ti.sel[1] >> 24) * 8]);
+                        cand = ~lack & live;
+                    }
                 }
-                while (cand) {
-                    const uint32_t bit = 31u - __clz(cand);
-                    cand ^= 1u << bit;
-                    *--at = uint8_t(wi * 32 + bit);
+                if (COUNT) w_tiles += __popc(__ballot_sync(kFull, tq < r.te && wi == 0));  // lane 0 reports
+                // candidate lists (query index in its chunk, one byte each): a
+                // prefix sum over each tile's words places every lane's queries,
+                // from the word's highest down
+                const uint32_t cnt = __popc(cand);
+                uint32_t incl = cnt;
+#pragma unroll
+                for (uint32_t o = 1; o < 32; o <<= 1) {
+                    if (!kWide && o >= (1u << lg)) break;
+                    const uint32_t v = __shfl_up_sync(kFull, incl, o);
+                    if (wi >= o) incl += v;
                 }
-            }
-            __syncwarp();
-            for (uint32_t todo = __ballot_sync(kFull, lane == last && incl != 0); todo; todo &= todo - 1) {
-                const uint32_t end = __ffs(todo) - 1, first = end & ~((1u << lg) - 1u);  // the tile's lanes
-                const uint32_t n = __shfl_sync(kFull, incl, end), count = __shfl_sync(kFull, tcount, first);
-                const uint32_t t = t0 + (end >> lg);
-                // list positions where chunks 1 .. kItemChunks - 1 begin: the
-                // candidate at position x is in chunk sum_c (x >= cb[c])
-                uint32_t cb[kItemChunks - 1];
+                {
+                    uint8_t *at = list + ((gi << lg) << 5) + incl;
+                    while (cand) {
+                        const uint32_t bit = 31u - __clz(cand);
+                        cand ^= 1u << bit;
+                        *--at = uint8_t(wi * 32 + bit);
+                    }
+                }
+                __syncwarp();
+                uint32_t todo = kWide ? 1u << 31 : __ballot_sync(kFull, lane == last && incl != 0);
+                for (; todo; todo = kWide ? 0u : todo & (todo - 1)) {
+                    const uint32_t end = kWide ? 31u : __ffs(todo) - 1, first = end & ~((1u << lg) - 1u);  // the tile's lanes
+                    const uint32_t n = __shfl_sync(kFull, incl, end), count = kWide ? tcount : __shfl_sync(kFull, tcount, first);
+                    if (kWide && n == 0) break;
+                    const uint32_t t = t0 + (end >> lg);
+                    // list positions where chunks 1 .. kItemChunks - 1 begin: the
+                    // candidate at position x is in chunk sum_c (x >= cb[c])
+                    uint32_t cb[kItemChunks - 1];
 #pragma unroll
-                for (int c = 0; c + 1 < kItemChunks; ++c) cb[c] = __shfl_sync(kFull, incl, min(first + 8 * c + 7, end));
-                auto query_at = [&](uint32_t x, uint32_t in_chunk) {
-                    uint32_t c = 0;
+                    for (int c = 0; c + 1 < kItemChunks; ++c) cb[c] = __shfl_sync(kFull, incl, min(first + 8 * c + 7, end));
+                    auto query_at = [&](uint32_t x, uint32_t in_chunk) {
+                        uint32_t c = 0;
 #pragma unroll
-                    for (int k = 0; k + 1 < kItemChunks; ++k) c += x >= cb[k] ? (uint32_t)kChunk : 0u;
-                    return c + in_chunk;
-                };
-                if (COUNT) w_cand += n;  // the warp's candidates (lane 0 reports)
-                const uint8_t *lst = list + (first << 5);
-                uint32_t f[kWords];
+                        for (int k = 0; k + 1 < kItemChunks; ++k) c += x >= cb[k] ? (uint32_t)kChunk : 0u;
+                        return c + in_chunk;
+                    };
+                    if (COUNT) w_cand += n;  // the warp's candidates (lane 0 reports)
+                    const uint8_t *lst = list + (first << 5);
+                    uint32_t f[kWords];
 #pragma unroll
-                for (int k = 0; k < kWords; ++k) f[k] = __ldg(&a.tile_words[(size_t(t) * kWords + k) * kTile + lane]);
-                const uint32_t vm = count >= 32u ? kFull : (1u << count) - 1u;  // lanes holding a filter
-                const uint32_t groups = (count + 3) >> 2;
-                const bool per_query = ((n + 31) >> 5) * (16u + 40u * groups) < ((n + 3) >> 2) * a.fpl_trip_cost;
-                if (per_query) {
+                    for (int k = 0; k < kWords; ++k) f[k] = __ldg(&a.tile_words[(size_t(t) * kWords + k) * kTile + lane]);
+                    const uint32_t vm = count >= 32u ? kFull : (1u << count) - 1u;  // lanes holding a filter
+                    const uint32_t groups = (count + 3) >> 2;
+                    const bool per_query = kWide || ((n + 31) >> 5) * (16u + 40u * groups) < ((n + 3) >> 2) * a.fpl_trip_cost;
+                    if (per_query) {
 #pragma unroll
-                    for (int k = 0; k < kWords; ++k) tfw[k * kTile + lane] = f[k];
-                    __syncwarp();
-                    uint32_t p0 = 0;
-                    for (; p0 + 32 < n; p0 += 64) {
-                        const uint32_t j0 = p0 + lane, j1 = j0 + 32;
-                        const uint32_t i0 = query_at(j0, lst[j0]), i1 = j1 < n ? query_at(j1, lst[j1]) : 0u;
-                        const uint4 lo[2] = {S.q_lo[i0], S.q_lo[i1]}, hi[2] = {S.q_hi[i0], S.q_hi[i1]};
-                        uint32_t m[2];
-                        test_queries<2>(S.tf[warp], groups, lo, hi, m);
-                        if (COUNT) {
-                            w_passes += 2;
-                            w_groups += 2 * groups;
-                            w_lanes += min(64u, n - p0);
+                        for (int k = 0; k < kWords; ++k) tfw[k * kTile + lane] = f[k];
+                        __syncwarp();
+                        uint32_t p0 = 0;
+                        for (; p0 + 32 < n; p0 += 64) {
+                            const uint32_t j0 = p0 + lane, j1 = j0 + 32;
+                            const uint32_t i0 = query_at(j0, lst[j0]), i1 = j1 < n ? query_at(j1, lst[j1]) : 0u;
+                            const uint4 lo[2] = {S.q_lo[i0], S.q_lo[i1]}, hi[2] = {S.q_hi[i0], S.q_hi[i1]};
+                            uint32_t m[2];
+                            test_queries<2>(S.tf[warp], groups, lo, hi, m);
+                            if (COUNT) {
+                                w_passes += 2;
+                                w_groups += 2 * groups;
+                                w_lanes += min(64u, n - p0);
+                            }
+                            stage(m[0] & vm, hi[0].z, t);
+                            stage(j1 < n ? m[1] & vm : 0u, hi[1].z, t);
                         }
-                        stage(m[0] & vm, hi[0].z, t);
-                        stage(j1 < n ? m[1] & vm : 0u, hi[1].z, t);
-                    }
-                    if (p0 < n) {
-                        const uint32_t j0 = p0 + lane, i0 = j0 < n ? query_at(j0, lst[j0]) : 0u;
-                        const uint4 lo[1] = {S.q_lo[i0]}, hi[1] = {S.q_hi[i0]};
-                        uint32_t m[1];
-                        test_queries<1>(S.tf[warp], groups, lo, hi, m);
-                        if (COUNT) {
-                            ++w_passes;
-                            w_groups += groups;
-                            w_lanes += n - p0;
-                            if (p0 == 0 && n <= 16) ++w_small;
+                        if (p0 < n) {
+                            const uint32_t j0 = p0 + lane, i0 = j0 < n ? query_at(j0, lst[j0]) : 0u;
+                            const uint4 lo[1] = {S.q_lo[i0]}, hi[1] = {S.q_hi[i0]};
+                            uint32_t m[1];
+                            test_queries<1>(S.tf[warp], groups, lo, hi, m);
+                            if (COUNT) {
+                                ++w_passes;
+                                w_groups += groups;
+                                w_lanes += n - p0;
+                                if (p0 == 0 && n <= 16) ++w_small;
+                            }
+                            stage(j0 < n ? m[0] & vm : 0u, hi[0].z, t);
                         }
-                        stage(j0 < n ? m[0] & vm : 0u, hi[0].z, t);
+                    } else {
+                        const bool lane_valid = lane < count;
+                        for (uint32_t j = 0; j < n; j += 4) {
+                            if (COUNT) ++w_trips;
+                            const uint32_t idx4 = *reinterpret_cast<const uint32_t *>(lst + j);
+                            const uint32_t ia = query_at(j, idx4 & 0xFFu), ib = query_at(j + 1, (idx4 >> 8) & 0xFFu);
+                            const uint32_t ic = query_at(j + 2, (idx4 >> 16) & 0xFFu), id = query_at(j + 3, idx4 >> 24);
+                            const uint4 p0 = S.q_lo[ia], p1 = S.q_hi[ia];
+                            const uint4 q0 = S.q_lo[ib], q1 = S.q_hi[ib];
+                            const uint4 r0 = S.q_lo[ic], r1 = S.q_hi[ic];
+                            const uint4 u0 = S.q_lo[id], u1 = S.q_hi[id];
+                            uint32_t x0 = f[0] & ~p0.x, x1 = f[0] & ~q0.x, x2 = f[0] & ~r0.x, x3 = f[0] & ~u0.x;
+                            x0 = andnot_or(f[1], p0.y, x0);
+                            x1 = andnot_or(f[1], q0.y, x1);
+                            x2 = andnot_or(f[1], r0.y, x2);
+                            x3 = andnot_or(f[1], u0.y, x3);
+                            x0 = andnot_or(f[2], p0.z, x0);
+                            x1 = andnot_or(f[2], q0.z, x1);
+                            x2 = andnot_or(f[2], r0.z, x2);
+                            x3 = andnot_or(f[2], u0.z, x3);
+                            x0 = andnot_or(f[3], p0.w, x0);
+                            x1 = andnot_or(f[3], q0.w, x1);
+                            x2 = andnot_or(f[3], r0.w, x2);
+                            x3 = andnot_or(f[3], u0.w, x3);
+                            x0 = andnot_or(f[4], p1.x, x0);
+                            x1 = andnot_or(f[4], q1.x, x1);
+                            x2 = andnot_or(f[4], r1.x, x2);
+                            x3 = andnot_or(f[4], u1.x, x3);
+                            x0 = andnot_or(f[5], p1.y, x0);
+                            x1 = andnot_or(f[5], q1.y, x1);
+                            x2 = andnot_or(f[5], r1.y, x2);
+                            x3 = andnot_or(f[5], u1.y, x3);
+                            // common case: no hit among the four (one min chain, one vote)
+                            if (!__any_sync(kFull, lane_valid && min(min(x0, x1), min(x2, x3)) == 0)) continue;
+                            // warp-uniform from here: one ballot per candidate gives the
+                            // tile's hit mask for that query; lane k < 4 stages record k
+                            // (what lies past the list is dropped)
+                            const uint32_t b0 = __ballot_sync(kFull, x0 == 0) & vm;
+                            const uint32_t b1 = __ballot_sync(kFull, x1 == 0) & vm;
+                            const uint32_t b2 = __ballot_sync(kFull, x2 == 0) & vm;
+                            const uint32_t b3 = __ballot_sync(kFull, x3 == 0) & vm;
+                            const uint32_t mine = lane == 0 ? b0 : lane == 1 ? b1 : lane == 2 ? b2 : b3;
+                            const uint32_t qid = lane == 0 ? p1.z : lane == 1 ? q1.z : lane == 2 ? r1.z : u1.z;
+                            stage(lane < 4 && j + lane < n ? mine : 0u, qid, t);
+                        }
                     }
-                } else {
-                    const bool lane_valid = lane < count;
-                    for (uint32_t j = 0; j < n; j += 4) {
-                        if (COUNT) ++w_trips;
-                        const uint32_t idx4 = *reinterpret_cast<const uint32_t *>(lst + j);
-                        const uint32_t ia = query_at(j, idx4 & 0xFFu), ib = query_at(j + 1, (idx4 >> 8) & 0xFFu);
-                        const uint32_t ic = query_at(j + 2, (idx4 >> 16) & 0xFFu), id = query_at(j + 3, idx4 >> 24);
-                        const uint4 p0 = S.q_lo[ia], p1 = S.q_hi[ia];
-                        const uint4 q0 = S.q_lo[ib], q1 = S.q_hi[ib];
-                        const uint4 r0 = S.q_lo[ic], r1 = S.q_hi[ic];
-                        const uint4 u0 = S.q_lo[id], u1 = S.q_hi[id];
-                        uint32_t x0 = f[0] & ~p0.x, x1 = f[0] & ~q0.x, x2 = f[0] & ~r0.x, x3 = f[0] & ~u0.x;
-                        x0 = andnot_or(f[1], p0.y, x0);
-                        x1 = andnot_or(f[1], q0.y, x1);
-                        x2 = andnot_or(f[1], r0.y, x2);
-                        x3 = andnot_or(f[1], u0.y, x3);
-                        x0 = andnot_or(f[2], p0.z, x0);
-                        x1 = andnot_or(f[2], q0.z, x1);
-                        x2 = andnot_or(f[2], r0.z, x2);
-                        x3 = andnot_or(f[2], u0.z, x3);
-                        x0 = andnot_or(f[3], p0.w, x0);
-                        x1 = andnot_or(f[3], q0.w, x1);
-                        x2 = andnot_or(f[3], r0.w, x2);
-                        x3 = andnot_or(f[3], u0.w, x3);
-                        x0 = andnot_or(f[4], p1.x, x0);
-                        x1 = andnot_or(f[4], q1.x, x1);
-                        x2 = andnot_or(f[4], r1.x, x2);
-                        x3 = andnot_or(f[4], u1.x, x3);
-                        x0 = andnot_or(f[5], p1.y, x0);
-                        x1 = andnot_or(f[5], q1.y, x1);
-                        x2 = andnot_or(f[5], r1.y, x2);
-                        x3 = andnot_or(f[5], u1.y, x3);
-                        // common case: no hit among the four (one min chain, one vote)
-                        if (!__any_sync(kFull, lane_valid && min(min(x0, x1), min(x2, x3)) == 0)) continue;
-                        // warp-uniform from here: one ballot per candidate gives the
-                        // tile's hit mask for that query; lane k < 4 stages record k
-                        // (list padding repeats a query and is dropped)
-                        const uint32_t b0 = __ballot_sync(kFull, x0 == 0) & vm;
-                        const uint32_t b1 = __ballot_sync(kFull, x1 == 0) & vm;
-                        const uint32_t b2 = __ballot_sync(kFull, x2 == 0) & vm;
-                        const uint32_t b3 = __ballot_sync(kFull, x3 == 0) & vm;
-                        const uint32_t mine = lane == 0 ? b0 : lane == 1 ? b1 : lane == 2 ? b2 : b3;
-                        const uint32_t qid = lane == 0 ? p1.z : lane == 1 ? q1.z : lane == 2 ? r1.z : u1.z;
-                        stage(lane < 4 && j + lane < n ? mine : 0u, qid, t);
-                    }
+                    __syncwarp();  // the tile buffer is rebuilt for the next tile
                 }
-                __syncwarp();  // the tile buffer is rebuilt for the next tile
+                __syncwarp();  // the lists are rebuilt for the next tiles
             }
-            __syncwarp();  // the lists are rebuilt for the next tiles
-        }
+        };
+        if (words > 16) all_tiles(std::true_type{});
+        else all_tiles(std::false_type{});
         __syncwarp();
         if (TIMED && lane == 0) {
             atomicAdd(&a.item_stats[2 * size_t(item)], (unsigned long long)(clock64() - item_c0));
