@@ -141,6 +141,14 @@ constexpr size_t kQueueAheadBytes = size_t(256) << 20;
 // partitions, twice.
 constexpr size_t kRowWords = size_t(64) << 18;
 
+// Hit records per query that a batch's buffer is made for at first.  A batch
+// that has more runs again with a larger buffer, at twice the time, which is
+// what the first batches of an engine did on ten million filters: there a
+// query makes 3,350 records (446,000 tiles), 690 on a million (44,000), 950 on
+// two million skewed ones (98,000).
+constexpr size_t kLeastRecords = 512, kMostRecords = 4608;
+size_t records_per_query(uint32_t n_tiles) { return std::min(kLeastRecords + n_tiles / 128, kMostRecords); }
+
 MatchScratch::~MatchScratch() {
     if (ev_begin) cudaEventDestroy(ev_begin);
     if (ev_end) cudaEventDestroy(ev_end);
@@ -239,8 +247,14 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     // route, queues (both again per window), plan, match, scan, readback
     bs.launches += windows * (windows > 1 ? 3 : 2) + 3 + scan_launches(nq) + (ahead ? 0u : 1u);
     // ---- match (regrow and re-run on pair overflow) ----
-    if (s.rec_cap_hint == 0) s.rec_cap_hint = size_t(nq) * 512 + (1u << 20);
-    s.recs.reserve(s.rec_cap_hint);
+    s.rec_cap_hint = std::max(s.rec_cap_hint, size_t(nq) * records_per_query(t.n_tiles) + (1u << 20));
+    try {
+        s.recs.reserve(s.rec_cap_hint);
+    } catch (const Error &e) {
+        if (e.status != TM_ERR_NOMEM) throw;
+        s.rec_cap_hint = size_t(nq) * kLeastRecords + (1u << 20);  // it grows with what the batch turns out to need
+        s.recs.reserve(s.rec_cap_hint);
+    }
     unsigned long long hc[4] = {0, 0, 0, 0};
     uint64_t total = 0;
     for (int attempt = 0;; ++attempt) {

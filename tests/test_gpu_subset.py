@@ -45,3 +45,25 @@ def test_candidates_per_tile(n, nf):
     q[at, 0] |= 1
     q[at[::3], 1] |= np.uint32(1 << (50 - 32))
     _check(f, ko, k, q, 65536, 128)
+
+
+def test_more_records_than_expected():
+    """Queries that match every filter make more hit records than the buffer is
+    made for at first: the batch runs again and is exact."""
+    import torch
+
+    from tagmatch_b200.tagmatch import read_device
+    f, ko, k = workload.generate_filters(200_000, 62)
+    nq = 300
+    with TagMatch() as tm:
+        tm.set_persistence(False)
+        tm.add_many(f, ko, k)
+        tm.consolidate(65536, 1)
+        dq = torch.full((nq, 6), -1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        for retries in (1, 1):  # the second call finds the buffer grown
+            po, pk, nk = tm.match_batch_device(dq.data_ptr(), nq)
+            assert tm.match_stats()["pair_retries"] == retries
+            assert np.array_equal(read_device(po, nq + 1, np.uint64), np.arange(nq + 1, dtype=np.uint64) * k.size)
+        last = read_device(pk + 4 * (nq - 1) * k.size, k.size, np.uint32)
+        assert np.array_equal(np.sort(last), np.sort(k))
