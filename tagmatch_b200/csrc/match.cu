@@ -79,6 +79,7 @@ MatchScratch &MatchScratch::operator=(MatchScratch &&o) noexcept {
     item_stats = std::move(o.item_stats);
     h_item_stats = std::move(o.h_item_stats);
     for (int i = 0; i < 2 * ScanScratch::kLevels; ++i) scr.levels[i] = std::move(o.scr.levels[i]);
+    side.swap(o.side);
     sm_count = o.sm_count;
     rec_cap_hint = o.rec_cap_hint;
     seg_tiles = o.seg_tiles;
@@ -197,7 +198,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     const uint32_t *order = ordered ? s.d_part_order.p : nullptr;
     s.part_off.reserve(size_t(P) + 1);
     s.chunk_off.reserve(size_t(P) + 1);
-    s.item_off.reserve(size_t(P) + 2);
+    s.item_off.reserve(size_t(P) + 4);
     // batches whose items are timed for the cost model take the tiles per item
     // as they are set: the model learns their effect
     const uint32_t least = least_seg(nq);
@@ -348,12 +349,12 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
         s.ukeys.reserve(std::max<uint64_t>(total, 1));
         // the offsets' buffer holds the list of long queries until the scan
         launch_unique_sort(s.keys.p, s.qoff.p, nq, s.ukeys.p, s.ucount.p, reinterpret_cast<uint32_t *>(s.uoff.p), t.max_key,
-                           s.sm_count, st);
+                           s.sm_count, st, &s.side);
         exclusive_scan<uint32_t, uint64_t>(s.ucount.p, s.uoff.p, nq, s.scr, st);
         // compact into s.keys (unique prefix of every segment is <= its length)
         k_compact<<<nq, 256, 0, st>>>(s.ukeys.p, s.qoff.p, s.uoff.p, nq, s.keys.p);
         TM_CHECK_LAUNCH();
-        bs.launches += 4 + scan_launches(nq);  // two sorts, compact, readback, scan
+        bs.launches += 5 + scan_launches(nq);  // list, two sorts, compact, readback, scan
     }
     uint64_t utotal = 0;
     std::memcpy(&utotal, read_back(s, s.uoff.p + nq, 2, nullptr, 0, nullptr, 0, st), sizeof(uint64_t));

@@ -40,6 +40,7 @@ struct MatchScratch {
     bool record_items = false;
     DevBuf<unsigned long long> item_stats;
     std::vector<unsigned long long> h_item_stats;
+    SideStream side;  // the long results of the sorting route
     ScanScratch scr;
     int sm_count = 0;
     size_t rec_cap_hint = 0;

@@ -128,8 +128,8 @@ __host__ __device__ inline uint32_t part_items(uint32_t count, uint32_t nt, uint
 // Offsets of the work plan from the partitions' counts, one CTA: queue
 // positions, 256-query chunks, and work items (groups of kItemChunks chunks
 // x tile segments), the items over queue positions (order: the partition at
-// each position; null: id order).  *seg_out: tiles per item, from seg_tiles
-// and the items wanted (0: seg_tiles as it is).
+// each position; null: id order).  seg_out: tiles per item, from seg_tiles
+// and the items wanted (0: seg_tiles as it is); queue positions; chunks.
 __global__ void __launch_bounds__(kPlanThreads) k_plan(const uint32_t *__restrict__ part_count,
                                                        const uint32_t *__restrict__ part_tile_begin,
                                                        const uint32_t *__restrict__ order, uint32_t n_parts,
@@ -188,7 +188,9 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(const uint32_t *__restric
         part_off[n_parts] = base[0];
         chunk_off[n_parts] = base[1];
         item_off[n_parts] = base[2];
-        *seg_out = seg;
+        seg_out[0] = seg;
+        seg_out[1] = base[0];
+        seg_out[2] = base[1];
     }
 }
 
@@ -1183,7 +1185,7 @@ __global__ void __launch_bounds__(kExpandThreads) k_unique_expand(const uint32_t
 // counts (a prefix sum over digits, then warps) and, within 32 keys, from
 // the lanes that hold the same digit.  Most results are short, and a small
 // block per query keeps many of them resident; the queries above
-// kSortSmallKeys keys are put on a list, and a second kernel gives them 1,024
+// kSortSmallKeys keys are on a list, and a kernel of their own gives them 1,024
 // threads each.  Both are bound by the shared-memory steps of the ranking:
 // 2,000 queries of 1,070 32-bit keys take 82 + 83 us (the few long results),
 // where one thread per stretch with 4-bit digits in global memory took 650.
@@ -1290,15 +1292,17 @@ __device__ __forceinline__ void sort_query(uint32_t *keys, uint64_t b, uint32_t 
 }
 
 // long_list: [0] number of long queries (zeroed by the caller), [1 ..] the queries.
+__global__ void k_long_list(const uint64_t *__restrict__ qoff, uint32_t nq, uint32_t *__restrict__ long_list) {
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < nq && qoff[q + 1] - qoff[q] > kSortSmallKeys) long_list[1 + atomicAdd(&long_list[0], 1u)] = q;
+}
+
 __global__ void __launch_bounds__(kSortSmallThreads) k_unique_sort(uint32_t *keys, const uint64_t *__restrict__ qoff,
                                                                    uint32_t *ukeys, uint32_t *__restrict__ ucount,
-                                                                   uint32_t *long_list, int key_bits) {
+                                                                   int key_bits) {
     const uint32_t q = blockIdx.x;
     const uint64_t b = qoff[q], n = qoff[q + 1] - b;  // a query's keys are counted in 32 bits
-    if (n > kSortSmallKeys) {
-        if (threadIdx.x == 0) long_list[1 + atomicAdd(&long_list[0], 1u)] = q;
-        return;
-    }
+    if (n > kSortSmallKeys) return;
     if (n == 0) {
         if (threadIdx.x == 0) ucount[q] = 0;
         return;
@@ -1354,19 +1358,26 @@ inline void launch_unique_expand(const uint32_t *bitmaps, const uint64_t *uoff, 
 }
 
 // Sorts every query's keys and leaves the different ones in ukeys[qoff ..).
-// long_list: scratch of nq + 1 words.
+// long_list: scratch of nq + 1 words.  The long queries are sorted beside the
+// others where the caller has a stream for them (2,000 queries of 1,070 keys:
+// the two kernels take 84 and 94 us, one after the other before).
 inline void launch_unique_sort(uint32_t *keys, const uint64_t *qoff, uint32_t nq, uint32_t *ukeys, uint32_t *ucount,
-                               uint32_t *long_list, uint32_t max_key, int sm_count, cudaStream_t st) {
+                               uint32_t *long_list, uint32_t max_key, int sm_count, cudaStream_t st,
+                               SideStream *side = nullptr) {
     int key_bits = 0;
     while (key_bits < 32 && (max_key >> key_bits)) ++key_bits;
     constexpr int small = kSortSmem<kSortSmallThreads, kSortSmallKeys>, large = kSortSmem<kSortLargeThreads, kSortLargeKeys>;
     TM_CUDA(cudaFuncSetAttribute(k_unique_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, large));
     TM_CUDA(cudaMemsetAsync(long_list, 0, sizeof(uint32_t), st));
-    k_unique_sort<<<nq, kSortSmallThreads, small, st>>>(keys, qoff, ukeys, ucount, long_list, key_bits);
+    k_long_list<<<blocks_for(nq, 256), 256, 0, st>>>(qoff, nq, long_list);
     TM_CHECK_LAUNCH();
-    k_unique_sort_long<<<std::min<uint32_t>(nq, uint32_t(sm_count)), kSortLargeThreads, large, st>>>(keys, qoff, ukeys, ucount,
-                                                                                                     long_list, key_bits);
+    cudaStream_t beside = side ? side->fork(st) : st;
+    k_unique_sort_long<<<std::min<uint32_t>(nq, uint32_t(sm_count)), kSortLargeThreads, large, beside>>>(
+        keys, qoff, ukeys, ucount, long_list, key_bits);
     TM_CHECK_LAUNCH();
+    k_unique_sort<<<nq, kSortSmallThreads, small, st>>>(keys, qoff, ukeys, ucount, key_bits);
+    TM_CHECK_LAUNCH();
+    if (side) side->join(st);
 }
 
 // Copies na words at a, nb at b, then nc at c, into mapped pinned host memory

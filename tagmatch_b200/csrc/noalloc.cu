@@ -123,23 +123,22 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
         TM_CUDA(cudaStreamSynchronize(st));
         return;
     }
-    unsigned long long *counters = ar.take<unsigned long long>(4, "counters");
+    unsigned long long *counters = ar.take<unsigned long long>(5, "counters");  // and the key total
+    uint32_t *qkeys = ar.take<uint32_t>(nq, "query key counts");
+    uint32_t *qcursor = ar.take<uint32_t>(nq, "query cursors");
     uint32_t *part_count = ar.take<uint32_t>(P, "partition counts");
+    // what starts at zero, cleared together
+    TM_CUDA(cudaMemsetAsync(counters, 0, size_t(reinterpret_cast<unsigned char *>(part_count + P) -
+                                                reinterpret_cast<unsigned char *>(counters)), st));
     uint32_t *part_off = ar.take<uint32_t>(size_t(P) + 1, "partition offsets");
     uint32_t *chunk_off = ar.take<uint32_t>(size_t(P) + 1, "plan");
-    uint32_t *item_off = ar.take<uint32_t>(size_t(P) + 2, "plan");
+    uint32_t *item_off = ar.take<uint32_t>(size_t(P) + 4, "plan");
     // block sums of a scan over at most kNoAllocMaxQueries
     constexpr size_t kScanBlocks = (kNoAllocMaxQueries + kScanTile - 1) / kScanTile;
     uint64_t *sums = ar.take<uint64_t>(kScanBlocks, "scan");
     uint64_t *offs = ar.take<uint64_t>(kScanBlocks + 1, "scan");
-    uint32_t *qkeys = ar.take<uint32_t>(nq, "query key counts");
-    uint32_t *qcursor = ar.take<uint32_t>(nq, "query cursors");
     uint64_t *qoff = ar.take<uint64_t>(size_t(nq) + 1, "query offsets");
     uint32_t *ucount = ar.take<uint32_t>(nq, "unique counts");
-    TM_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), st));
-    TM_CUDA(cudaMemsetAsync(part_count, 0, P * sizeof(uint32_t), st));
-    TM_CUDA(cudaMemsetAsync(qkeys, 0, nq * sizeof(uint32_t), st));
-    TM_CUDA(cudaMemsetAsync(qcursor, 0, nq * sizeof(uint32_t), st));
 
     // routing counts and the work plan; the routing rows lie in what the
     // queues leave free, as many partitions at a time as fit (the first
@@ -156,10 +155,10 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     k_plan<<<1, kPlanThreads, 0, st>>>(part_count, t.part_tile_begin.p, nullptr, P, seg_tiles, least_seg(nq),
                                        uint32_t(sms) * 4 * kItemsPerCta, part_off, chunk_off, item_off, item_off + P + 1);
     TM_CHECK_LAUNCH();
-    uint32_t routed = 0, chunks = 0;
-    TM_CUDA(cudaMemcpyAsync(&routed, part_off + P, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    TM_CUDA(cudaMemcpyAsync(&chunks, chunk_off + P, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    uint32_t plan[2] = {0, 0};  // routed pairs, chunks: k_plan's last words
+    TM_CUDA(cudaMemcpyAsync(plan, item_off + P + 2, sizeof(plan), cudaMemcpyDeviceToHost, st));
     TM_CUDA(cudaStreamSynchronize(st));
+    const uint32_t routed = plan[0], chunks = plan[1];
 
     uint4 *queue = ar.take<uint4>(size_t(std::max<uint32_t>(routed, 1)) * 2, "partition queues");
     uint32_t *slices = ar.take<uint32_t>(size_t(std::max<uint32_t>(chunks, 1)) * kSliceWords, "query slices");
@@ -182,9 +181,18 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
                 fpl_trip_cost(), nullptr, nullptr, nullptr};
     launch_match<false>(a, unsigned(sms) * 4, st);
     TM_CHECK_LAUNCH();
-    unsigned long long hc[3] = {0, 0, 0};
-    TM_CUDA(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, st));
+    // the record count and the key total come back together
+    uint64_t *key_off = unique ? qoff : d_out_offsets;
+    scan_fixed<uint32_t, uint64_t>(qkeys, key_off, nq, sums, offs, st);
+    struct {
+        unsigned long long counters[4];
+        uint64_t total;
+    } back;
+    TM_CUDA(cudaMemcpyAsync(counters + 4, key_off + nq, sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
+    TM_CUDA(cudaMemcpyAsync(&back, counters, sizeof(back), cudaMemcpyDeviceToHost, st));
     TM_CUDA(cudaStreamSynchronize(st));
+    const unsigned long long *hc = back.counters;
+    const uint64_t total = back.total;
     if (hc[2]) throw Error(TM_ERR_TIMEOUT, "match kernel: bounded wait for the query copy expired");
     if (hc[1] > rec_room - 32)
         throw Error(TM_ERR_CAPACITY, "no-allocation scratch too small for the " + std::to_string(hc[1]) +
@@ -192,11 +200,6 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
 
     // keys
     ar.trim(recs + hc[1]);
-    uint64_t *key_off = unique ? qoff : d_out_offsets;
-    scan_fixed<uint32_t, uint64_t>(qkeys, key_off, nq, sums, offs, st);
-    uint64_t total = 0;
-    TM_CUDA(cudaMemcpyAsync(&total, key_off + nq, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    TM_CUDA(cudaStreamSynchronize(st));
     if (!unique) {
         *n_keys = total;
         if (total > capacity)

@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace tmb {
@@ -118,6 +119,42 @@ private:
     };
     size_t total_ = 0;
     std::vector<Piece> pieces_;
+};
+
+// A stream for work beside the owner's: fork() makes it wait for what st holds
+// so far and returns it, join() makes st wait for it.  Created at first use
+// on the then current device.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t forked = nullptr, joined = nullptr;
+    SideStream() = default;
+    SideStream(const SideStream &) = delete;
+    SideStream &operator=(const SideStream &) = delete;
+    ~SideStream() { release(); }
+    void release() {
+        if (stream) cudaStreamDestroy(stream);
+        if (forked) cudaEventDestroy(forked);
+        if (joined) cudaEventDestroy(joined);
+        stream = nullptr;
+        forked = joined = nullptr;
+    }
+    void swap(SideStream &o) {
+        std::swap(stream, o.stream);
+        std::swap(forked, o.forked);
+        std::swap(joined, o.joined);
+    }
+    cudaStream_t fork(cudaStream_t st) {
+        if (!stream) TM_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        if (!forked) TM_CUDA(cudaEventCreateWithFlags(&forked, cudaEventDisableTiming));
+        if (!joined) TM_CUDA(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming));
+        TM_CUDA(cudaEventRecord(forked, st));
+        TM_CUDA(cudaStreamWaitEvent(stream, forked, 0));
+        return stream;
+    }
+    void join(cudaStream_t st) {
+        TM_CUDA(cudaEventRecord(joined, stream));
+        TM_CUDA(cudaStreamWaitEvent(st, joined, 0));
+    }
 };
 
 // Pinned host buffer (grow-only).
