@@ -26,21 +26,23 @@
 //                bit transposes of the query words);
 //   k_match      persistent CTAs take items from an atomic counter.  Each
 //                item's query records are staged into shared memory by bulk
-//                TMA copies (cp.async.bulk + mbarrier), one per chunk; the
-//                buffers are released by per-warp mbarrier arrivals.  A warp
-//                takes one tile of <= 32 filters at a time; the tile's AND
-//                mask selects candidate queries of all four chunks by
-//                OR-ing the slices of its bits (one 32-query word per lane);
-//                the candidates are tested either one per lane against the
-//                tile's filters broadcast from shared memory, or, when they
-//                are few, four at a time against the tile held one filter
-//                per lane (6 LOP3s per (query, filter) either way); each
-//                (query, tile) with a hit becomes a (query, tile, hit mask,
-//                key count) record, staged per warp in shared memory and
-//                flushed with one global atomic, and its key count is added
-//                to the query's total;
+//                TMA copies (cp.async.bulk + mbarrier); the buffers are
+//                released by per-warp mbarrier arrivals.  A warp selects the
+//                candidate queries of one tile of <= 32 filters (or of
+//                several, for items of few queries) by OR-ing the slices of
+//                bits that all the tile's filters hold, one 32-query word
+//                per lane; the candidates are tested either two or one per
+//                lane against the tile's filters broadcast from shared
+//                memory, or, when they are few, four at a time against the
+//                tile held one filter per lane (6 LOP3s per (query, filter)
+//                either way); each (query, tile) with a hit becomes a
+//                (query, tile, hit mask, key count) record, staged per warp
+//                in shared memory and flushed with one global atomic, which
+//                is when its keys are counted and added to the query's
+//                total;
 //   k_key_fill   after a prefix sum of the query totals: one cursor atomic
-//                per record; the runs of adjacent hit bits of a warp's 64
+//                per record (per query and block of records for batches of
+//                few queries); the runs of adjacent hit bits of a warp's 64
 //                records (one key range each) are numbered and copied 32 at
 //                a time by the whole warp;
 //   k_unique_*   match_unique: per-query bitmap, read out in order (small
@@ -95,7 +97,8 @@ MatchScratch &MatchScratch::operator=(MatchScratch &&o) noexcept {
 // Estimated cost of one 4-candidate trip of the subset test's
 // lane-per-filter loop, against which the lane-per-query pass is weighed
 // for each tile (TM_FPL_TRIP_COST overrides it; results do not depend on
-// it).  Measured on the config-1 step with 1,024-query work items: flat
+// it; items of more than 512 queries always take the pass).  Measured on
+// 524,288 queries and ten million filters with 1,024-query work items: flat
 // from 75 to 150, worse below (45: +9%).
 uint32_t fpl_trip_cost() {
     static const uint32_t v = [] {
