@@ -141,6 +141,10 @@ const uint32_t *read_back(MatchScratch &s, const void *a, uint32_t na, const voi
 // and the wait saved (it is paid by small batches: about 10 us of 180 for
 // one query).
 constexpr size_t kQueueAheadBytes = size_t(256) << 20;
+// match_unique's bitmaps take this much without a question (1 GiB); beyond, at
+// most twice what the batch's keys take: many queries with a few keys each
+// are sorted instead, which needs no more than the keys.
+constexpr size_t kBitmapWordsAnyway = size_t(1) << 28;
 // Largest routing matrix kept at once; larger ones are made in windows of
 // partitions, twice.
 constexpr size_t kRowWords = size_t(64) << 18;
@@ -341,9 +345,18 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     // ---- match_unique ----
     s.ucount.reserve(nq);
     s.uoff.reserve(size_t(nq) + 1);
-    if (unique_by_bitmap(t.max_key)) {
-        const uint32_t words = (t.max_key >> 5) + 1;
-        s.ukeys.reserve(size_t(nq) * bitmap_stride(words));
+    const uint32_t words = (t.max_key >> 5) + 1;
+    const size_t bitmap_words = size_t(nq) * bitmap_stride(words);
+    bool bitmaps = unique_by_bitmap(t.max_key) && bitmap_words <= std::max<size_t>(kBitmapWordsAnyway, 2 * total);
+    if (bitmaps) {
+        try {
+            s.ukeys.reserve(bitmap_words);
+        } catch (const Error &e) {
+            if (e.status != TM_ERR_NOMEM) throw;
+            bitmaps = false;
+        }
+    }
+    if (bitmaps) {
         launch_unique_mark(s.keys.p, s.qoff.p, nq, words, s.ukeys.p, s.ucount.p, s.sm_count, st);
         exclusive_scan<uint32_t, uint64_t>(s.ucount.p, s.uoff.p, nq, s.scr, st);
         launch_unique_expand(s.ukeys.p, s.uoff.p, nq, words, s.keys.p, st);

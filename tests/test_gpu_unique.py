@@ -66,3 +66,29 @@ def test_unique_shared_digits():
             off, keys = tm.match_batch(q, unique=True)
         eoff, ekeys = oracle.match(f, ko, k, q, unique=True)
         assert np.array_equal(off, eoff) and np.array_equal(keys, ekeys)
+
+
+@pytest.mark.parametrize("nq", [131_072, 140_000])
+def test_many_queries_with_few_small_keys(nq):
+    """16-bit keys on both sides of where the bitmaps of a batch (8 KB per
+    query) give way to sorting."""
+    import torch
+
+    from tagmatch_b200.tagmatch import read_device
+    keys = [np.array([7, 9, 65_535], dtype=np.uint32), np.array([1, 9, 30_000], dtype=np.uint32)]
+    with TagMatch() as tm:
+        tm.set_persistence(False)
+        tm.add(filter_from_bits([3]), keys[0])
+        tm.add(filter_from_bits([3, 4]), keys[1])
+        tm.consolidate(65536, 1)
+        q = np.tile(filter_from_bits([3, 4, 5]), (nq, 1))
+        q[1::2] = filter_from_bits([3])
+        q[::1000] = 0
+        dq = torch.from_numpy(q.view(np.int32)).cuda()
+        torch.cuda.synchronize()
+        po, pk, nk = tm.match_batch_device(dq.data_ptr(), nq, unique=True)
+        off, got = read_device(po, nq + 1, np.uint64), read_device(pk, nk, np.uint32)
+    both = np.array([1, 7, 9, 30_000, 65_535], dtype=np.uint32)
+    want = [np.zeros(0, np.uint32) if i % 1000 == 0 else keys[0] if i & 1 else both for i in range(nq)]
+    assert np.array_equal(np.diff(off.astype(np.int64)), [w.size for w in want])
+    assert np.array_equal(got, np.concatenate(want))
