@@ -194,21 +194,6 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(const uint32_t *__restric
     }
 }
 
-// 32 x 32 bit transpose over a warp: bit j of lane i <- bit i of lane j.
-// Five rounds exchange the off-diagonal blocks of 16, 8, .. 1 bits.
-__device__ __forceinline__ uint32_t warp_transpose(uint32_t x, unsigned lane) {
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
-        constexpr uint32_t kLow[5] = {0x55555555u, 0x33333333u, 0x0F0F0F0Fu, 0x00FF00FFu, 0x0000FFFFu};
-        const uint32_t low = kLow[s == 1 ? 0 : s == 2 ? 1 : s == 4 ? 2 : s == 8 ? 3 : 4];
-        const uint32_t y = __shfl_xor_sync(kFull, x, s);
-        const bool up = (lane & s) != 0;
-        const uint32_t keep = up ? ~low : low;
-        x = (x & keep) | (__funnelshift_l(y, y, up ? 32 - s : s) & ~keep);
-    }
-    return x;
-}
-
 // Fills the partitions' queues from their routing rows (partitions
 // [p0, p0 + gridDim.x)): CTA (p, y) takes the queries of positions
 // [1024 y, 1024 y + 1024), finds them in the row (counts per group, then a

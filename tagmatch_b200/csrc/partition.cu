@@ -387,19 +387,6 @@ __global__ void k_children(const Seg *__restrict__ segs, uint32_t n_act, const u
     }
 }
 
-// 32 x 32 bit transpose over a warp: bit j of lane i <- bit i of lane j.
-__device__ __forceinline__ uint32_t transpose32(uint32_t x, unsigned lane) {
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
-        const uint32_t low = s == 16 ? 0x0000FFFFu : s == 8 ? 0x00FF00FFu : s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
-        const uint32_t y = __shfl_xor_sync(kFull, x, s);
-        const bool up = (lane & s) != 0;
-        const uint32_t keep = up ? ~low : low;
-        x = (x & keep) | (__funnelshift_l(y, y, up ? 32 - s : s) & ~keep);
-    }
-    return x;
-}
-
 // Peels one range to its end (nonzero_mask_partitioning, partitioning.cc:
 // 230-250) in one CTA: while some bit is held by a part of the filters left,
 // those that hold the most frequent one (the first on ties) split off, behind
@@ -479,7 +466,7 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel(const Seg *__restrict__ s
             const uint32_t e = have ? list[g + lane] : 0u;
 #pragma unroll
             for (int k = 0; k < kWords; ++k) {
-                const uint32_t held = __popc(transpose32(have ? w0[size_t(e) * kWords + k] : 0u, lane));
+                const uint32_t held = __popc(warp_transpose(have ? w0[size_t(e) * kWords + k] : 0u, lane));
                 if (held) atomicSub(&s_cnt[k * 32 + lane], held);
             }
         }
@@ -628,7 +615,7 @@ __global__ void __launch_bounds__(32) k_split_small(uint32_t *__restrict__ words
             const bool have = g + lane < r.e;
             const uint32_t i = have ? S.at[g + lane] : 0u;
 #pragma unroll
-            for (int k = 0; k < kWords; ++k) f[k] += __popc(transpose32(have ? S.w[k][i] : 0u, lane));
+            for (int k = 0; k < kWords; ++k) f[k] += __popc(warp_transpose(have ? S.w[k][i] : 0u, lane));
         }
         unsigned long long best = ~0ull;
 #pragma unroll

@@ -64,6 +64,20 @@ __device__ __forceinline__ void add_if_zero(uint32_t &acc, uint32_t x, uint32_t 
     asm("{\n .reg .pred p;\n setp.eq.u32 p, %1, 0;\n @p add.u32 %0, %0, %2;\n}\n" : "+r"(acc) : "r"(x), "r"(v));
 }
 
+// 32 x 32 bit transpose over a warp: bit j of lane i <- bit i of lane j.
+// Five rounds exchange the off-diagonal blocks of 16, 8, .. 1 bits.
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t x, unsigned lane) {
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        const uint32_t low = s == 16 ? 0x0000FFFFu : s == 8 ? 0x00FF00FFu : s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
+        const uint32_t y = __shfl_xor_sync(kFull, x, s);
+        const bool up = (lane & s) != 0;
+        const uint32_t keep = up ? ~low : low;
+        x = (x & keep) | (__funnelshift_l(y, y, up ? 32 - s : s) & ~keep);
+    }
+    return x;
+}
+
 __device__ __forceinline__ bool subset6(const uint32_t *f, const uint32_t *q) {
     uint32_t a = f[0] & ~q[0];
     a = andnot_or(f[1], q[1], a);
