@@ -83,7 +83,8 @@ MatchScratch &MatchScratch::operator=(MatchScratch &&o) noexcept {
     for (int i = 0; i < 2 * ScanScratch::kLevels; ++i) scr.levels[i] = std::move(o.scr.levels[i]);
     side.swap(o.side);
     sm_count = o.sm_count;
-    rec_cap_hint = o.rec_cap_hint;
+    rec_history = o.rec_history;
+    bitmaps_refused = o.bitmaps_refused;
     seg_tiles = o.seg_tiles;
     profile = o.profile;
     if (ev_begin) cudaEventDestroy(ev_begin);
@@ -149,13 +150,7 @@ constexpr size_t kBitmapWordsAnyway = size_t(1) << 28;
 // partitions, twice.
 constexpr size_t kRowWords = size_t(64) << 18;
 
-// Hit records per query that a batch's buffer is made for at first.  A batch
-// that has more runs again with a larger buffer, at twice the time, which is
-// what the first batches of an engine did on ten million filters: there a
-// query makes 3,350 records (446,000 tiles), 690 on a million (44,000), 950 on
-// two million skewed ones (98,000).
-constexpr size_t kLeastRecords = 512, kMostRecords = 4608;
-size_t records_per_query(uint32_t n_tiles) { return std::min(kLeastRecords + n_tiles / 128, kMostRecords); }
+static_assert(sizeof(HitRec) == kRecordBytes, "the record buffer is sized in records");
 
 MatchScratch::~MatchScratch() {
     if (ev_begin) cudaEventDestroy(ev_begin);
@@ -255,14 +250,11 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     // route, queues (both again per window), plan, match, scan, readback
     bs.launches += windows * (windows > 1 ? 3 : 2) + 3 + scan_launches(nq) + (ahead ? 0u : 1u);
     // ---- match (regrow and re-run on pair overflow) ----
-    s.rec_cap_hint = std::max(s.rec_cap_hint, size_t(nq) * records_per_query(t.n_tiles) + (1u << 20));
-    try {
-        s.recs.reserve(s.rec_cap_hint);
-    } catch (const Error &e) {
-        if (e.status != TM_ERR_NOMEM) throw;
-        s.rec_cap_hint = size_t(nq) * kLeastRecords + (1u << 20);  // it grows with what the batch turns out to need
-        s.recs.reserve(s.rec_cap_hint);
-    }
+    reserve_records(s.recs, s.rec_history, nq, t.n_tiles, [] {
+        size_t free_bytes = 0, all_bytes = 0;
+        TM_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes));
+        return free_bytes;
+    });
     unsigned long long hc[4] = {0, 0, 0, 0};
     uint64_t total = 0;
     for (int attempt = 0;; ++attempt) {
@@ -316,11 +308,11 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
         }
         if (hc[1] <= s.recs.cap) break;
         if (attempt >= 3) throw Error(TM_ERR_INTERNAL, "hit record buffer regrowth did not converge");
-        s.rec_cap_hint = size_t(hc[1] + hc[1] / 4 + 1024);
-        s.recs.reserve(s.rec_cap_hint);
+        s.recs.reserve(size_t(hc[1] + hc[1] / 4 + 1024));
         bs.retries++;
     }
     bs.records = hc[1];
+    s.rec_history.seen(nq, hc[1]);
     if (s.record_items) {
         s.h_item_stats.resize(2 * size_t(items));
         if (items)
@@ -347,15 +339,8 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     s.uoff.reserve(size_t(nq) + 1);
     const uint32_t words = (t.max_key >> 5) + 1;
     const size_t bitmap_words = size_t(nq) * bitmap_stride(words);
-    bool bitmaps = unique_by_bitmap(t.max_key) && bitmap_words <= std::max<size_t>(kBitmapWordsAnyway, 2 * total);
-    if (bitmaps) {
-        try {
-            s.ukeys.reserve(bitmap_words);
-        } catch (const Error &e) {
-            if (e.status != TM_ERR_NOMEM) throw;
-            bitmaps = false;
-        }
-    }
+    const bool bitmaps = unique_by_bitmap(t.max_key) && bitmap_words <= std::max<size_t>(kBitmapWordsAnyway, 2 * total) &&
+                         reserve_bitmaps(s.ukeys, bitmap_words, s.bitmaps_refused);
     if (bitmaps) {
         launch_unique_mark(s.keys.p, s.qoff.p, nq, words, s.ukeys.p, s.ucount.p, s.sm_count, st);
         exclusive_scan<uint32_t, uint64_t>(s.ucount.p, s.uoff.p, nq, s.scr, st);

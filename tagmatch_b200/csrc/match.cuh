@@ -3,6 +3,7 @@
 #pragma once
 #include <cstdint>
 #include "partition.cuh"
+#include "scratch_size.hpp"
 
 namespace tmb {
 
@@ -43,7 +44,8 @@ struct MatchScratch {
     SideStream side;  // the long results of the sorting route
     ScanScratch scr;
     int sm_count = 0;
-    size_t rec_cap_hint = 0;
+    RecordHistory rec_history;
+    size_t bitmaps_refused = ~size_t(0);  // words of match_unique bitmaps that were not to be had
     uint32_t seg_tiles = kSegTiles;  // tiles per work item
     // optional CUDA-event timing of the subset-test kernel
     bool profile = false;

@@ -1,0 +1,88 @@
+// How large the matcher's optional or guessed device buffers are made: plain
+// rules over sizes, apart from the device so that they can be run without one.
+#pragma once
+#include <algorithm>
+#include <cstddef>
+#include <cstdint>
+
+namespace tmb {
+
+constexpr size_t kRecordBytes = 16;               // one hit record
+constexpr size_t kSpareRecords = size_t(1) << 20;  // of a first buffer, beside those per query
+// Hit records per query that a buffer is made for ahead of its first batch.
+// A batch that has more runs again with a larger buffer, at twice the time,
+// which is what the first batches of an engine did on ten million filters:
+// there a query makes 3,350 records (446,000 tiles), 690 on a million (44,000),
+// 950 on two million skewed ones (98,000).
+constexpr size_t kLeastRecords = 512, kMostRecords = 4608;
+constexpr size_t records_per_query(uint32_t n_tiles) {
+    return kLeastRecords + n_tiles / 128 < kMostRecords ? kLeastRecords + n_tiles / 128 : kMostRecords;
+}
+// A guess may take this share of the device memory that is free with the
+// buffer given back: the keys, whose size is known and must be had, come after.
+constexpr size_t kGuessShare = 8;
+
+// What the batches of one scratch have shown of its table's hit records.
+struct RecordHistory {
+    uint32_t n_tiles = 0;                  // the table they were matched on
+    uint64_t queries = 0, records = 0;     // seen
+    size_t ceiling = ~size_t(0);           // records that a guess may not exceed any more
+
+    void seen(uint32_t nq, uint64_t n) {
+        queries += nq;
+        records += n;
+        if (queries > (uint64_t(1) << 20)) {  // later batches count more
+            queries /= 2;
+            records /= 2;
+        }
+    }
+    // Records expected of nq queries: the table's guess, which weighs as much
+    // as 64 queries, and what was seen, with a margin of a quarter.
+    size_t expected(uint32_t nq, uint32_t tiles) {
+        if (tiles != n_tiles) {
+            *this = RecordHistory();
+            n_tiles = tiles;
+        }
+        const double guess = double(records_per_query(tiles));
+        const double per_query = (64.0 * guess + 1.25 * double(records)) / (64.0 + double(queries));
+        return size_t(double(nq) * std::min(guess, per_query));
+    }
+};
+
+// Makes the record buffer ready for a batch: never smaller than it is (at
+// first kLeastRecords a query and the spare ones), larger where the batch is
+// expected to need it and a share of the free memory allows.  What was refused
+// once, by that share or by the allocator, is not tried again: every further
+// try would free the buffer that serves, fail, and make the small one again,
+// with the subset test run twice after it (65,536 queries without matches on
+// ten million filters with 3 GiB free: 2,970 us or more for every call, 170
+// since).
+// free_bytes() is asked only when the buffer would grow.
+template <class Buf, class FreeBytes>
+void reserve_records(Buf &recs, RecordHistory &h, uint32_t nq, uint32_t n_tiles, FreeBytes free_bytes) {
+    const size_t held = recs.p ? recs.cap : 0;
+    const size_t least = held ? held : size_t(nq) * kLeastRecords + kSpareRecords;
+    size_t want = std::min(h.expected(nq, n_tiles), h.ceiling);
+    if (want > least) {
+        const size_t room = (free_bytes() / kRecordBytes + held) / kGuessShare;
+        if (want > room) h.ceiling = want = room;
+    }
+    if (want > least) {
+        if (recs.try_reserve(want)) return;
+        h.ceiling = least;
+    }
+    recs.reserve(least);
+}
+
+// Makes room for match_unique's bitmaps; false when there is none.  The size
+// that was refused is not tried again (refused: kept beside the buffer).
+template <class Buf>
+bool reserve_bitmaps(Buf &buf, size_t words, size_t &refused) {
+    if (buf.p && words <= buf.cap) return true;
+    if (words >= refused) return false;
+    if (buf.try_reserve(words)) return true;
+    refused = words;
+    return false;
+}
+
+}  // namespace tmb

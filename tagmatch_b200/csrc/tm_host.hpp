@@ -70,24 +70,37 @@ struct DevBuf {
     // Grows by at least half the current capacity, so a slowly growing
     // demand reallocates (and frees, which synchronises the device) rarely.
     void reserve(size_t n) {
-        if (n <= cap && p) return;
-        if (p) n = std::max(n, cap + cap / 2);
-        release();
-        size_t bytes = (n ? n : 1) * sizeof(T);
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e != cudaSuccess) {
-            p = nullptr;
-            cap = 0;
-            cudaGetLastError();
+        size_t bytes = 0;
+        const cudaError_t e = grow(n, bytes);
+        if (e != cudaSuccess)
             throw Error(-5, cuda_msg(e, "cudaMalloc", __FILE__, __LINE__) + " bytes=" + std::to_string(bytes));
-        }
-        cap = n ? n : 1;
+    }
+    // reserve() that reports a refusal, which leaves the buffer empty.
+    bool try_reserve(size_t n) {
+        size_t bytes = 0;
+        return grow(n, bytes) == cudaSuccess;
     }
     void release() {
         if (p && owned) cudaFree(p);
         forget();
     }
     T *get() const { return p; }
+
+private:
+    cudaError_t grow(size_t n, size_t &bytes) {
+        if (n <= cap && p) return cudaSuccess;
+        if (p) n = std::max(n, cap + cap / 2);
+        release();
+        bytes = (n ? n : 1) * sizeof(T);
+        const cudaError_t e = cudaMalloc(&p, bytes);
+        if (e != cudaSuccess) {
+            forget();
+            cudaGetLastError();
+            return e;
+        }
+        cap = n ? n : 1;
+        return e;
+    }
 };
 
 // One device allocation cut into 256-byte aligned pieces, for calls that need

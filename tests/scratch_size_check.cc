@@ -1,0 +1,116 @@
+// The matcher's buffer size rules over an allocator with a limit, no device.
+#include "../tagmatch_b200/csrc/scratch_size.hpp"
+#include <cstdio>
+#include <cstdlib>
+
+#define CHECK(x)                                                   \
+    do {                                                           \
+        if (!(x)) {                                                \
+            std::printf("%s:%d: %s\n", __FILE__, __LINE__, #x);    \
+            std::exit(1);                                          \
+        }                                                          \
+    } while (0)
+
+// A buffer like the device's: growing frees first, and may be refused.
+struct Device {
+    size_t free_bytes;
+    int allocations = 0, refusals = 0;
+};
+struct Buf {
+    Device &dev;
+    size_t element;
+    void *p = nullptr;
+    size_t cap = 0;
+    bool try_reserve(size_t n) {
+        if (p && n <= cap) return true;
+        if (p) n = std::max(n, cap + cap / 2);
+        dev.free_bytes += cap * element;
+        p = nullptr;
+        cap = 0;
+        if (n * element > dev.free_bytes) return ++dev.refusals, false;
+        dev.free_bytes -= n * element;
+        ++dev.allocations;
+        p = this;
+        cap = n;
+        return true;
+    }
+    void reserve(size_t n) { CHECK(try_reserve(n)); }
+};
+
+static void batch(Buf &b, tmb::RecordHistory &h, uint32_t nq, uint32_t tiles, uint64_t records, int *runs = nullptr) {
+    tmb::reserve_records(b, h, nq, tiles, [&] { return b.dev.free_bytes; });
+    if (records > b.cap) {
+        b.reserve(records + records / 4 + 1024);
+        if (runs) ++*runs;
+    }
+    h.seen(nq, records);
+}
+
+int main() {
+    const size_t GiB = size_t(1) << 30;
+    const uint32_t tiles = 446000, nq = 65536;  // ten million filters
+    for (uint64_t per_query : {0, 100, 3350}) {
+        for (size_t free_gib : {3, 5, 8, 20, 170}) {
+            Device dev{free_gib * GiB};
+            Buf b{dev, tmb::kRecordBytes};
+            tmb::RecordHistory h;
+            if (per_query * nq * 5 / 4 * tmb::kRecordBytes > free_gib * GiB) continue;  // does not fit at all
+            int runs = 0;
+            batch(b, h, nq, tiles, per_query * nq, &runs);
+            // a guess takes no more than its share; what is needed is had
+            CHECK(dev.refusals == 0);
+            if (!runs) CHECK(b.cap * tmb::kRecordBytes <= std::max(free_gib * GiB / tmb::kGuessShare, (nq * size_t(512) + (1u << 20)) * 16));
+            const int allocations = dev.allocations;
+            const size_t cap = b.cap;
+            for (int i = 0; i < 50; ++i) batch(b, h, nq, tiles, per_query * nq, &runs);
+            CHECK(dev.allocations == allocations && b.cap == cap && dev.refusals == 0);
+            CHECK(runs == (allocations > 1 ? 1 : 0));
+            // a smaller batch leaves the buffer
+            batch(b, h, 1, tiles, per_query);
+            CHECK(b.cap == cap);
+            // with memory to spare the first batch does not run twice
+            if (free_gib == 170) CHECK(runs == 0);
+        }
+    }
+    {   // a guess that the allocator refuses all the same is made once
+        Device dev{3 * GiB};
+        Buf b{dev, tmb::kRecordBytes};
+        tmb::RecordHistory h;
+        auto all_free = [] { return size_t(170) << 30; };
+        tmb::reserve_records(b, h, nq, tiles, all_free);
+        CHECK(dev.refusals == 1 && b.cap == nq * size_t(512) + (1u << 20));
+        for (int i = 0; i < 5; ++i) tmb::reserve_records(b, h, nq, tiles, all_free);
+        CHECK(dev.refusals == 1 && dev.allocations == 1);
+    }
+    {   // small batches first: later ones are sized by what was seen, not by
+        // the table alone, and one query's records are no measure
+        Device dev{170 * GiB};
+        Buf b{dev, tmb::kRecordBytes};
+        tmb::RecordHistory h;
+        for (int i = 0; i < 20; ++i) batch(b, h, 1000, tiles, 1000 * 20);
+        batch(b, h, 4 * nq, tiles, size_t(4) * nq * 20);
+        CHECK(b.cap * 16 < GiB);
+        tmb::RecordHistory one;
+        one.seen(1, 400000);
+        CHECK(one.expected(nq, tiles) <= size_t(nq) * tmb::kMostRecords);
+    }
+    {   // another table starts over
+        tmb::RecordHistory h;
+        h.expected(1, tiles);
+        h.seen(100000, 0);
+        h.ceiling = 5;
+        CHECK(h.expected(1000, 128 * 200) == 1000 * 712 && h.ceiling == ~size_t(0));
+    }
+    {   // refused bitmaps are not asked for again, smaller ones are
+        Device dev{GiB};
+        Buf b{dev, 4};
+        size_t refused = ~size_t(0);
+        for (int i = 0; i < 5; ++i) {
+            CHECK(!tmb::reserve_bitmaps(b, GiB / 2, refused));
+            b.reserve(1000);  // the sorting route's buffer
+        }
+        CHECK(dev.refusals == 1 && dev.allocations == 1);
+        CHECK(tmb::reserve_bitmaps(b, GiB / 8, refused) && tmb::reserve_bitmaps(b, GiB / 8, refused) && dev.allocations == 2);
+    }
+    std::puts("ok");
+}
