@@ -193,7 +193,9 @@ int tm_set_flush_mode(tm_engine *e, int mode);
 int tm_set_serving_results(tm_engine *e, int where);
 /* Device-memory budget per lane for a batch's queues, hit records and keys; the
  * number of queries admitted into one batch is capped by it (estimated
- * from the bytes per query of recent batches).  Default 16 GiB. */
+ * from the bytes per query of recent batches), and buffers made larger than
+ * the batch is known to need, and match_unique's bitmaps, take at most a part
+ * of it.  Default 16 GiB. */
 int tm_set_memory_budget(tm_engine *e, uint64_t bytes);
 
 /* partitioning::balanced_partitioning(fib, masks) -- partitioning.cc:361-411,

@@ -687,7 +687,7 @@ void Engine::run_pieces(Device &d, Lane &ln, std::vector<Piece> &pieces, bool un
         TM_CUDA(cudaStreamSynchronize(ln.stream));
         dkeys_out = dkeys;
         // running estimate of device bytes per query (queues, hit records, keys)
-        const uint64_t bytes = bs.routed * (kQueueWords * 4) + bs.records * sizeof(HitRec) + nk * 4 * (unique ? 3 : 1);
+        const uint64_t bytes = bs.routed * (kQueueWords * 4) + bs.records * sizeof(HitRec) + bs.key_bytes;
         const uint64_t bpq = std::max<uint64_t>(1024, bytes / std::max<uint32_t>(nq, 1));
         bytes_per_query_.store((bytes_per_query_.load() * 3 + bpq) / 4);
     } catch (const Error &e) {
@@ -836,6 +836,7 @@ void Engine::prepare(MatchScratch &s, uint32_t nq, bool serving) {
     s.record_items = sched_.recording();
     if (learned_order_.load()) s.part_order = sched_.order();
     else s.part_order.clear();
+    s.budget = serving ? size_t(memory_budget_.load()) : 0;
     if (serving) {
         // the learned serving mode also picks each batch's tiles per work
         // item (small batches want more, smaller items); otherwise the

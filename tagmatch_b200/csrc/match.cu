@@ -86,6 +86,7 @@ MatchScratch &MatchScratch::operator=(MatchScratch &&o) noexcept {
     rec_history = o.rec_history;
     bitmaps_refused = o.bitmaps_refused;
     seg_tiles = o.seg_tiles;
+    budget = o.budget;
     profile = o.profile;
     if (ev_begin) cudaEventDestroy(ev_begin);
     if (ev_end) cudaEventDestroy(ev_end);
@@ -142,10 +143,6 @@ const uint32_t *read_back(MatchScratch &s, const void *a, uint32_t na, const voi
 // and the wait saved (it is paid by small batches: about 10 us of 180 for
 // one query).
 constexpr size_t kQueueAheadBytes = size_t(256) << 20;
-// match_unique's bitmaps take this much without a question (1 GiB); beyond, at
-// most twice what the batch's keys take: many queries with a few keys each
-// are sorted instead, which needs no more than the keys.
-constexpr size_t kBitmapWordsAnyway = size_t(1) << 28;
 // Largest routing matrix kept at once; larger ones are made in windows of
 // partitions, twice.
 constexpr size_t kRowWords = size_t(64) << 18;
@@ -236,7 +233,8 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
         bs.items = items;
     };
     size_t queue_len = size_t(nq) * P, slice_len = size_t(P) * blocks_for(nq, kChunk);
-    const bool ahead = !s.record_items && queue_len * kQueueWords * 4 + slice_len * kSliceWords * 4 <= kQueueAheadBytes;
+    const bool ahead = !s.record_items && queue_len * kQueueWords * 4 + slice_len * kSliceWords * 4 <=
+                                              std::min(kQueueAheadBytes, budget_share(s.budget, kQueueBudgetShare));
     if (!ahead) {
         host_plan(read_back(s, part_count, P, nullptr, 0, nullptr, 0, st));
         queue_len = bs.routed;
@@ -250,7 +248,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     // route, queues (both again per window), plan, match, scan, readback
     bs.launches += windows * (windows > 1 ? 3 : 2) + 3 + scan_launches(nq) + (ahead ? 0u : 1u);
     // ---- match (regrow and re-run on pair overflow) ----
-    reserve_records(s.recs, s.rec_history, nq, t.n_tiles, [] {
+    reserve_records(s.recs, s.rec_history, nq, t.n_tiles, s.budget, [] {
         size_t free_bytes = 0, all_bytes = 0;
         TM_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes));
         return free_bytes;
@@ -324,6 +322,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     bs.launches += 1 + (2 + scan_launches(nq)) * uint32_t(bs.retries);
     bs.pairs = hc[3];
     s.keys.reserve(std::max<uint64_t>(total, 1));
+    bs.key_bytes = total * 4;
     launch_key_fill(t, s.recs.p, counters, hc[1], s.qoff.p, qcursor, nq, s.keys.p, s.sm_count, st);
     if (!unique) {
         TM_CUDA(cudaStreamSynchronize(st));
@@ -339,8 +338,9 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     s.uoff.reserve(size_t(nq) + 1);
     const uint32_t words = (t.max_key >> 5) + 1;
     const size_t bitmap_words = size_t(nq) * bitmap_stride(words);
-    const bool bitmaps = unique_by_bitmap(t.max_key) && bitmap_words <= std::max<size_t>(kBitmapWordsAnyway, 2 * total) &&
+    const bool bitmaps = unique_by_bitmap(t.max_key) && bitmaps_allowed(bitmap_words * 4, total * 4, s.budget) &&
                          reserve_bitmaps(s.ukeys, bitmap_words, s.bitmaps_refused);
+    bs.key_bytes += bitmaps ? bitmap_words * 4 : total * 4;
     if (bitmaps) {
         launch_unique_mark(s.keys.p, s.qoff.p, nq, words, s.ukeys.p, s.ucount.p, s.sm_count, st);
         exclusive_scan<uint32_t, uint64_t>(s.ucount.p, s.uoff.p, nq, s.scr, st);

@@ -47,6 +47,7 @@ struct MatchScratch {
     RecordHistory rec_history;
     size_t bitmaps_refused = ~size_t(0);  // words of match_unique bitmaps that were not to be had
     uint32_t seg_tiles = kSegTiles;  // tiles per work item
+    size_t budget = 0;               // bytes that a batch's buffers are to stay within (0: not bounded)
     // optional CUDA-event timing of the subset-test kernel
     bool profile = false;
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
@@ -64,6 +65,7 @@ struct BatchStats {
     uint64_t pairs = 0;    // matching (query, filter) pairs
     uint64_t records = 0;  // hit records ((query, tile) with at least one match)
     uint64_t keys = 0;     // output keys
+    uint64_t key_bytes = 0;  // device memory of the keys: before match_unique, and its bitmaps or second buffer
     int retries = 0;       // pair-buffer regrowths
     float match_ms = 0.f;  // subset-test kernel time (profiling on)
     uint64_t dense = 0;    // sum over partitions of routed queries x partition size

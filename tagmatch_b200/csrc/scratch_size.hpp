@@ -21,6 +21,13 @@ constexpr size_t records_per_query(uint32_t n_tiles) {
 // A guess may take this share of the device memory that is free with the
 // buffer given back: the keys, whose size is known and must be had, come after.
 constexpr size_t kGuessShare = 8;
+// What a budget (bytes, 0: none) leaves to a buffer that may take 1 / share of
+// it: a batch's guesses and conveniences must leave room for its records and
+// keys, which the number of queries admitted is reckoned from.
+constexpr size_t budget_share(size_t budget, size_t share) { return budget ? budget / share : ~size_t(0); }
+constexpr size_t kGuessBudgetShare = 2;   // hit records ahead of the batch
+constexpr size_t kQueueBudgetShare = 4;   // queues allocated before they are counted
+constexpr size_t kBitmapBudgetShare = 4;  // match_unique's bitmaps
 
 // What the batches of one scratch have shown of its table's hit records.
 struct RecordHistory {
@@ -51,18 +58,19 @@ struct RecordHistory {
 
 // Makes the record buffer ready for a batch: never smaller than it is (at
 // first kLeastRecords a query and the spare ones), larger where the batch is
-// expected to need it and a share of the free memory allows.  What was refused
-// once, by that share or by the allocator, is not tried again: every further
+// expected to need it and a share of the free memory, and of the budget,
+// allows.  What was refused once, by that share or by the allocator, is not tried again: every further
 // try would free the buffer that serves, fail, and make the small one again,
 // with the subset test run twice after it (65,536 queries without matches on
 // ten million filters with 3 GiB free: 2,970 us or more for every call, 170
 // since).
 // free_bytes() is asked only when the buffer would grow.
 template <class Buf, class FreeBytes>
-void reserve_records(Buf &recs, RecordHistory &h, uint32_t nq, uint32_t n_tiles, FreeBytes free_bytes) {
+void reserve_records(Buf &recs, RecordHistory &h, uint32_t nq, uint32_t n_tiles, size_t budget, FreeBytes free_bytes) {
     const size_t held = recs.p ? recs.cap : 0;
     const size_t least = held ? held : size_t(nq) * kLeastRecords + kSpareRecords;
     size_t want = std::min(h.expected(nq, n_tiles), h.ceiling);
+    want = std::min(want, budget_share(budget, kGuessBudgetShare) / kRecordBytes);
     if (want > least) {
         const size_t room = (free_bytes() / kRecordBytes + held) / kGuessShare;
         if (want > room) h.ceiling = want = room;
@@ -72,6 +80,16 @@ void reserve_records(Buf &recs, RecordHistory &h, uint32_t nq, uint32_t n_tiles,
         h.ceiling = least;
     }
     recs.reserve(least);
+}
+
+// Whether match_unique's bitmaps may take their memory: up to 1 GiB without a
+// question, beyond that at most twice what the batch's keys take (many queries
+// with a few keys each are sorted instead, which needs no more than the keys),
+// and under a budget never more than its share or than sorting would take.
+constexpr size_t kBitmapBytesAnyway = size_t(1) << 30;
+constexpr bool bitmaps_allowed(size_t bitmap_bytes, size_t key_bytes, size_t budget) {
+    return bitmap_bytes <= std::max(kBitmapBytesAnyway, 2 * key_bytes) &&
+           bitmap_bytes <= std::max(key_bytes, budget_share(budget, kBitmapBudgetShare));
 }
 
 // Makes room for match_unique's bitmaps; false when there is none.  The size

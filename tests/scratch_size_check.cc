@@ -37,8 +37,9 @@ struct Buf {
     void reserve(size_t n) { CHECK(try_reserve(n)); }
 };
 
-static void batch(Buf &b, tmb::RecordHistory &h, uint32_t nq, uint32_t tiles, uint64_t records, int *runs = nullptr) {
-    tmb::reserve_records(b, h, nq, tiles, [&] { return b.dev.free_bytes; });
+static void batch(Buf &b, tmb::RecordHistory &h, uint32_t nq, uint32_t tiles, uint64_t records, int *runs = nullptr,
+                  size_t budget = 0) {
+    tmb::reserve_records(b, h, nq, tiles, budget, [&] { return b.dev.free_bytes; });
     if (records > b.cap) {
         b.reserve(records + records / 4 + 1024);
         if (runs) ++*runs;
@@ -77,9 +78,9 @@ int main() {
         Buf b{dev, tmb::kRecordBytes};
         tmb::RecordHistory h;
         auto all_free = [] { return size_t(170) << 30; };
-        tmb::reserve_records(b, h, nq, tiles, all_free);
+        tmb::reserve_records(b, h, nq, tiles, 0, all_free);
         CHECK(dev.refusals == 1 && b.cap == nq * size_t(512) + (1u << 20));
-        for (int i = 0; i < 5; ++i) tmb::reserve_records(b, h, nq, tiles, all_free);
+        for (int i = 0; i < 5; ++i) tmb::reserve_records(b, h, nq, tiles, 0, all_free);
         CHECK(dev.refusals == 1 && dev.allocations == 1);
     }
     {   // small batches first: later ones are sized by what was seen, not by
@@ -101,6 +102,21 @@ int main() {
         h.ceiling = 5;
         CHECK(h.expected(1000, 128 * 200) == 1000 * 712 && h.ceiling == ~size_t(0));
     }
+    for (size_t budget : {size_t(1) << 20, GiB / 4, 16 * GiB}) {  // a lane's budget bounds the guess, not what is needed
+        Device dev{170 * GiB};
+        Buf b{dev, tmb::kRecordBytes};
+        tmb::RecordHistory h;
+        const uint32_t n = uint32_t(std::max<size_t>(1, std::min<size_t>(nq, budget / (64 << 10))));
+        batch(b, h, n, tiles, size_t(n) * 20, nullptr, budget);
+        CHECK(b.cap * 16 <= std::max(budget / 2, (n * size_t(512) + (1u << 20)) * 16));
+        batch(b, h, n, tiles, size_t(n) * 5000, nullptr, budget);
+        CHECK(b.cap >= size_t(n) * 5000);
+        // bitmaps: a quarter of the budget, or what sorting would take
+        CHECK(tmb::bitmaps_allowed(budget / 4, 0, budget) == (budget / 4 <= GiB));
+        CHECK(!tmb::bitmaps_allowed(budget / 4 + 1, 0, budget));
+        CHECK(tmb::bitmaps_allowed(budget / 4 + 1, budget / 4 + 1, budget));
+    }
+    CHECK(tmb::bitmaps_allowed(GiB, 0, 0) && !tmb::bitmaps_allowed(GiB + 1, 0, 0) && tmb::bitmaps_allowed(3 * GiB, 3 * GiB / 2, 0));
     {   // refused bitmaps are not asked for again, smaller ones are
         Device dev{GiB};
         Buf b{dev, 4};
