@@ -555,6 +555,18 @@ struct SplitSmem {
 constexpr float kVisitCost = 212.f, kCandCost = 1.4f, kTestCost = 0.28f;
 constexpr int kCostBits = 4;
 
+// -log2 of the chance that a query holds a bit of the split weight.  Never
+// below zero, nor the zero with a sign that -log2f(1.f) is (a bit that three in
+// four filters hold has a weight that 1.f - weight rounds away): tile_cost
+// compares the values as integers, where that one is above all others.  With
+// it, a tag that all filters share let any neighbours be put together that 32
+// filters hold (a million filters with one: 41,928 tiles instead of 46,400;
+// 8,192 queries 502 us instead of 481, 500 queries 150 instead of 156).
+__device__ __forceinline__ float scarcity(float weight) {
+    const float held = 1.f - weight;
+    return held < 1.f ? -log2f(fmaxf(held, 1e-6f)) : 0.f;
+}
+
 // Cost of a tile whose members' AND is `all`, beside the visit; uniform over
 // the warp.  scarce: -log2 of the chance that a query holds bit 32 k + lane.
 __device__ __forceinline__ float tile_cost(const uint32_t (&all)[kWords], uint32_t count, const float (&scarce)[kWords],
@@ -670,7 +682,7 @@ __global__ void __launch_bounds__(32) k_split_small(uint32_t *__restrict__ words
     // than another visit
     float scarce[kWords];
 #pragma unroll
-    for (int k = 0; k < kWords; ++k) scarce[k] = -log2f(fmaxf(1.f - weight[k], 1e-6f));
+    for (int k = 0; k < kWords; ++k) scarce[k] = scarcity(weight[k]);
     uint32_t cur_b = 0, cur_and[kWords] = {0, 0, 0, 0, 0, 0};
     float cur_cost = 0.f;
     for (uint32_t b = 0, e; b < n; b = e) {
