@@ -25,7 +25,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 CUDA_SOURCES = ["partition.cu", "match.cu", "noalloc.cu", "sched.cu", "engine.cu", "capi.cu", "facade.cu"]
 HEADERS = ["tm_device.cuh", "tm_host.hpp", "scan.cuh", "partition.cuh", "match.cuh", "match_kernels.cuh", "scratch_size.hpp",
-           "sched.cuh", "engine.cuh"]
+           "sched.cuh", "threads.hpp", "engine.cuh"]
 
 LIB = os.path.join(HERE, "libtagmatch_b200.so")
 WORKLOAD_LIB = os.path.join(HERE, "libtm_workload.so")

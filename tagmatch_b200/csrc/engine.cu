@@ -1,5 +1,6 @@
 // TagMatch engine implementation.
 #include "engine.cuh"
+#include "threads.hpp"
 #include <algorithm>
 #include <chrono>
 #include <cstdio>
@@ -102,56 +103,6 @@ bool read_db(const std::string &fn, std::vector<Entry> &out, std::map<FilterKey,
         if (!e.keys.empty()) out.push_back(std::move(e));
     }
     return true;
-}
-
-unsigned worker_threads() { return std::max(1u, std::min(32u, std::thread::hardware_concurrency())); }
-
-// Runs f(0) .. f(n - 1), each on a thread of its own (one alone on the
-// caller's).  An exception of f (memory) is thrown again here.
-template <class F>
-void on_threads(unsigned n, F f) {
-    if (n == 1) {
-        f(0u);
-        return;
-    }
-    std::vector<std::exception_ptr> failed(n);
-    std::vector<std::thread> ts;
-    for (unsigned t = 0; t < n; ++t)
-        ts.emplace_back([&, t] {
-            try {
-                f(t);
-            } catch (...) {
-                failed[t] = std::current_exception();
-            }
-        });
-    for (auto &x : ts) x.join();
-    for (auto &e : failed)
-        if (e) std::rethrow_exception(e);
-}
-
-// Sorts v with cmp on all hardware threads: sorted chunks, then pairwise
-// merges.
-template <class T, class Cmp>
-void parallel_sort(std::vector<T> &v, Cmp cmp) {
-    const size_t n = v.size();
-    const unsigned th = worker_threads();
-    if (n < (size_t(1) << 16) || th == 1) {
-        std::sort(v.begin(), v.end(), cmp);
-        return;
-    }
-    std::vector<size_t> b(th + 1);
-    for (unsigned i = 0; i <= th; ++i) b[i] = n * i / th;
-    std::vector<std::thread> ts;
-    for (unsigned i = 0; i < th; ++i) ts.emplace_back([&, i] { std::sort(v.begin() + b[i], v.begin() + b[i + 1], cmp); });
-    for (auto &t : ts) t.join();
-    for (unsigned w = 1; w < th; w *= 2) {
-        ts.clear();
-        for (unsigned i = 0; i + w < th; i += 2 * w) {
-            const size_t lo = b[i], mid = b[i + w], hi = b[std::min(i + 2 * w, th)];
-            ts.emplace_back([&, lo, mid, hi] { std::inplace_merge(v.begin() + lo, v.begin() + mid, v.begin() + hi, cmp); });
-        }
-        for (auto &t : ts) t.join();
-    }
 }
 
 bool write_db(const std::string &fn, const std::vector<Entry> &fib) {
