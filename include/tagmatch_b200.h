@@ -261,7 +261,8 @@ int tm_mlp_loss_grad(const float *params, const float *features, const float *ta
 /* Tiles per work item of the subset test (what tm_autotune chooses;
  * default 128): each work item is a group of four consecutive 256-query
  * chunks of a partition against this many of its tiles (up to 32 filters
- * each); batches that would make too few items for the device take fewer.
+ * each); batches that would make too few items for the device take fewer,
+ * but for those recorded for the cost model or served with its choice.
  * No reference counterpart.  Results do not depend on it. */
 int tm_set_tiles_per_item(tm_engine *e, uint32_t seg_tiles);
 uint32_t tm_get_tiles_per_item(const tm_engine *e);

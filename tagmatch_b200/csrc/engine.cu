@@ -794,6 +794,7 @@ void Engine::prepare(MatchScratch &s, uint32_t nq, bool serving) {
         // engine's (autotuned) value
         const uint32_t best = flush_mode_.load() == kFlushLearned ? sched_.best_seg(nq) : 0u;
         s.seg_tiles = best ? best : seg_tiles_;
+        s.seg_exact = best != 0;
     }
 }
 

@@ -86,6 +86,7 @@ MatchScratch &MatchScratch::operator=(MatchScratch &&o) noexcept {
     rec_history = o.rec_history;
     bitmaps_refused = o.bitmaps_refused;
     seg_tiles = o.seg_tiles;
+    seg_exact = o.seg_exact;
     budget = o.budget;
     profile = o.profile;
     if (ev_begin) cudaEventDestroy(ev_begin);
@@ -199,9 +200,10 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     s.chunk_off.reserve(size_t(P) + 1);
     s.item_off.reserve(size_t(P) + 4);
     // batches whose items are timed for the cost model take the tiles per item
-    // as they are set: the model learns their effect
+    // as they are set, the model learns their effect; and so do those for
+    // which it chose them
     const uint32_t least = least_seg(nq);
-    const uint32_t want_items = s.record_items ? 0 : uint32_t(s.sm_count) * 4 * kItemsPerCta;
+    const uint32_t want_items = s.record_items || s.seg_exact ? 0 : uint32_t(s.sm_count) * 4 * kItemsPerCta;
     k_plan<<<1, kPlanThreads, 0, st>>>(part_count, t.part_tile_begin.p, order, P, s.seg_tiles, least, want_items, s.part_off.p,
                                        s.chunk_off.p, s.item_off.p, s.item_off.p + P + 1);
     TM_CHECK_LAUNCH();

@@ -47,6 +47,7 @@ struct MatchScratch {
     RecordHistory rec_history;
     size_t bitmaps_refused = ~size_t(0);  // words of match_unique bitmaps that were not to be had
     uint32_t seg_tiles = kSegTiles;  // tiles per work item
+    bool seg_exact = false;          // seg_tiles as it is, however few items that makes
     size_t budget = 0;               // bytes that a batch's buffers are to stay within (0: not bounded)
     // optional CUDA-event timing of the subset-test kernel
     bool profile = false;
