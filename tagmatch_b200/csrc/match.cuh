@@ -16,12 +16,12 @@ struct MatchScratch {
     // hit records, [2] error flags, [3] pairs), [nq] key totals, [nq] key
     // cursors, [P] queries per partition, [P][groups] the same per group
     DevBuf<uint32_t> zeroed;
-    DevBuf<uint32_t> rows;        // routing matrix: [P][nq / 32] bits
+    DevBuf<uint32_t> rows;        // routing matrix of a window of partitions: a bit per query, in rows of whole 256 queries
     DevBuf<uint32_t> part_off;    // [P + 1]
     DevBuf<uint4> queue;          // two planes of [routed]
     DevBuf<uint32_t> item_off;    // [P + 1] work items per partition (prefix)
     DevBuf<uint32_t> chunk_off;   // [P + 1] 256-query chunks per partition (prefix)
-    DevBuf<uint32_t> slices;      // [chunks][192][8] bit-sliced "lacks bit" masks
+    DevBuf<uint32_t> slices;      // [chunks][192 + 1][8] bit-sliced "lacks bit" masks, then a row of zeros
     DevBuf<unsigned long long> work;  // optional kernel work counters
     DevBuf<uint16_t> keys16;          // keys narrowed for the host transfer
     DevBuf<HitRec> recs;          // hit records of the subset test

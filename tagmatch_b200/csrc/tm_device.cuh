@@ -78,20 +78,6 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, unsigned lane) {
     return x;
 }
 
-__device__ __forceinline__ bool subset6(const uint32_t *f, const uint32_t *q) {
-    uint32_t a = f[0] & ~q[0];
-    a = andnot_or(f[1], q[1], a);
-    a = andnot_or(f[2], q[2], a);
-    a = andnot_or(f[3], q[3], a);
-    a = andnot_or(f[4], q[4], a);
-    a = andnot_or(f[5], q[5], a);
-    return a == 0;
-}
-
-__device__ __forceinline__ int bit_of(const uint32_t *f, unsigned b) {
-    return (f[b >> 5] >> (b & 31)) & 1;
-}
-
 }  // namespace tmb
 
 // Status codes (TM_OK, TM_ERR_*) come from the C ABI header.
