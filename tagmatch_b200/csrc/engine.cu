@@ -915,8 +915,12 @@ constexpr double kDirectFraction = 0.1;
 // Batches of at most this many keys go to a pinned buffer directly, as 32-bit
 // values: one copy at the link's rate, where the narrowing kernel, a copy of
 // half the bytes and then the widening by one or two threads follow one
-// another (3,000 queries, 7.7 M keys: 2.24 ms per call narrowed, 1.03
-// direct).  Larger batches overlap the three stages with other batches.
+// another.  That holds for one batch as for many that overlap.  Direct against
+// a tenth direct (ms per call, 65,536 queries a batch): one batch of 12.5 M
+// keys 1.4 and 2.6, of 25 M 2.4 and 4.8; six of 12.6 M 6.2 and 10.0, of 17 M
+// 8.2 and 12.9, of 25 M 11.9 and 14.3.  The line is on the safe side: direct
+// was still ahead with 43 M (four batches 13.8 and 14.0) and 75 M keys, but its
+// lead shrinks, and larger batches have the share that adapts to the host.
 constexpr uint64_t kDirectKeys = uint64_t(1) << 24;
 // smallest batch of match_host's final, halving batches
 constexpr uint64_t kTailBatch = 4096;
