@@ -325,7 +325,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     bs.pairs = hc[3];
     s.keys.reserve(std::max<uint64_t>(total, 1));
     bs.key_bytes = total * 4;
-    launch_key_fill(t, s.recs.p, counters, hc[1], s.qoff.p, qcursor, nq, s.keys.p, s.sm_count, st);
+    launch_key_fill(t, s.recs.p, counters, hc[1], total, s.qoff.p, qcursor, nq, s.keys.p, s.sm_count, st);
     if (!unique) {
         TM_CUDA(cudaStreamSynchronize(st));
         *d_offsets = s.qoff.p;

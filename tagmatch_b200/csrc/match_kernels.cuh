@@ -855,10 +855,14 @@ constexpr int kFillCtas = 6;     // resident per SM, at least (register budget)
 constexpr int kFillThreads = 256;
 constexpr int kFillWarps = kFillThreads / 32;
 constexpr int kFillStep = 32 * kFillPerLane;  // records per warp step
-// The block variant of the gather: records per block, and the most queries
+// The block variant of the gather: most records per block, and the most queries
 // of a batch that takes it (4 bytes of shared memory each).
 constexpr uint32_t kFillBlockRecs = 2048;
 constexpr uint32_t kFillBlockQueries = 2048;
+// Keys per record from which the gather is the one that looks for long runs,
+// and keys of a batch of 32 runs from which it copies them one by one.
+constexpr uint32_t kLongRecord = 32;
+constexpr uint32_t kLongBatch = 32 * 128;
 
 // Owners of 32 consecutive positions p0 + lane, when lane i owns a non-empty
 // stretch that begins at `start` (increasing with i; live: the lane has one):
@@ -885,17 +889,26 @@ __device__ __forceinline__ uint32_t owner_of(uint32_t start, bool live, uint32_t
 // key j, the run that owns it), so the stores coalesce and a record with
 // several runs costs no extra pass over the warp.
 //
-// BLOCK: a CTA takes kFillBlockRecs consecutive records, sums their keys per
+// BLOCK: a CTA takes block_recs consecutive records, sums their keys per
 // query in shared memory and reserves each query's keys with one global
 // atomic.  Atomics on one address follow one another, and in a batch of few
 // queries the heaviest holds a good part of all records: 500 queries of the
 // ten-million table (1.8 M records) took 272 us, six times the time per
 // record of a batch of 20,011.
-template <bool BLOCK>
+//
+// LONG: batches of 32 runs of kLongBatch keys or more are copied run by run,
+// four loads in flight, where 32 keys of all runs at a time wait for each load.
+// 20,000 queries with one run each, us: runs of 100 keys 137 as short ones and
+// 142 as long ones, of 150 159 and 125, of 400 256 and 150, of 2,000 927 and
+// 323.  An instantiation of its own for tables with that many keys per record:
+// the code beside the short way costs batches of short runs 0.3 to 0.6% of
+// their whole time.
+template <bool BLOCK, bool LONG>
 __global__ void __launch_bounds__(kFillThreads, kFillCtas) k_key_fill(
     const HitRec *__restrict__ recs, const unsigned long long *__restrict__ counters,
     const uint32_t *__restrict__ slot_key_off, const TileKeys *__restrict__ tile_keys, const uint32_t *__restrict__ tkeys,
-    const uint64_t *__restrict__ qoff, uint32_t *__restrict__ qcursor, uint32_t nq, uint32_t *__restrict__ out) {
+    const uint64_t *__restrict__ qoff, uint32_t *__restrict__ qcursor, uint32_t nq, uint32_t block_recs,
+    uint32_t *__restrict__ out) {
     extern __shared__ uint32_t s_cur[];  // BLOCK: [nq] the block's cursor per query
     // per warp and record of the step: tile, hit mask, keys, runs of the
     // lane's earlier records; and the record's first output position
@@ -975,6 +988,24 @@ __global__ void __launch_bounds__(kFillThreads, kFillCtas) k_key_fill(
             const uint32_t kin = warp_incl_scan(len);
             const uint32_t keys = __shfl_sync(kFull, kin, 31);
             const uint32_t start = kin - len;
+            if (LONG && keys >= kLongBatch) {
+                for (uint32_t runs = __ballot_sync(kFull, len != 0); runs; runs &= runs - 1) {
+                    const uint32_t ro = __ffs(runs) - 1;
+                    const uint32_t n_run = __shfl_sync(kFull, len, ro);
+                    const uint32_t *from = tkeys + __shfl_sync(kFull, src, ro);
+                    uint32_t *to = out + __shfl_sync(kFull, d, ro);
+                    uint32_t k = lane;
+                    for (; k + 96 < n_run; k += 128) {
+                        const uint32_t v0 = from[k], v1 = from[k + 32], v2 = from[k + 64], v3 = from[k + 96];
+                        to[k] = v0;
+                        to[k + 32] = v1;
+                        to[k + 64] = v2;
+                        to[k + 96] = v3;
+                    }
+                    for (; k < n_run; k += 32) to[k] = from[k];
+                }
+                continue;
+            }
             src -= start;
             d -= start;
             for (uint32_t j0 = 0; j0 < keys; j0 += 32) {
@@ -988,9 +1019,9 @@ __global__ void __launch_bounds__(kFillThreads, kFillCtas) k_key_fill(
         __syncwarp();  // the shared entries are rewritten by the next step
     };
     if constexpr (BLOCK) {
-        for (unsigned long long b0 = (unsigned long long)blockIdx.x * kFillBlockRecs; b0 < n;
-             b0 += (unsigned long long)gridDim.x * kFillBlockRecs) {
-            const unsigned long long b1 = min(n, b0 + kFillBlockRecs);
+        for (unsigned long long b0 = (unsigned long long)blockIdx.x * block_recs; b0 < n;
+             b0 += (unsigned long long)gridDim.x * block_recs) {
+            const unsigned long long b1 = min(n, b0 + block_recs);
             for (uint32_t q = threadIdx.x; q < nq; q += kFillThreads) s_cur[q] = 0;
             __syncthreads();
             for (unsigned long long i = b0 + threadIdx.x; i < b1; i += kFillThreads) {
@@ -1014,19 +1045,25 @@ __global__ void __launch_bounds__(kFillThreads, kFillCtas) k_key_fill(
     }
 }
 
-// Gathers the keys of n_recs records of nq queries (qcursor zeroed).
+// Gathers the `keys` keys of n_recs records of nq queries (qcursor zeroed).
 inline void launch_key_fill(const DevTable &t, const HitRec *recs, const unsigned long long *counters,
-                            unsigned long long n_recs, const uint64_t *qoff, uint32_t *qcursor, uint32_t nq, uint32_t *out,
-                            int sm_count, cudaStream_t st) {
+                            unsigned long long n_recs, uint64_t keys, const uint64_t *qoff, uint32_t *qcursor, uint32_t nq,
+                            uint32_t *out, int sm_count, cudaStream_t st) {
     const unsigned most = unsigned(sm_count) * 16;
+    const bool longer = keys >= kLongRecord * n_recs;
     if (nq <= kFillBlockQueries) {
-        const unsigned grid = std::max(1u, std::min(blocks_for(n_recs, kFillBlockRecs), most));
-        k_key_fill<true><<<grid, kFillThreads, nq * sizeof(uint32_t), st>>>(recs, counters, t.slot_key_off.p, t.tile_keys.p,
-                                                                           t.keys.p, qoff, qcursor, nq, out);
+        // few records are spread over the SMs, a warp's step of them each at
+        // least: they may have thousands of keys each (2,048 queries with a run
+        // of 400 keys each: 688 us in one block of 2,048 records, 116 so)
+        const unsigned long long per_sm = (n_recs + sm_count - 1) / sm_count;
+        const uint32_t block_recs = std::min(kFillBlockRecs, blocks_for(std::max(per_sm, 1ull), kFillStep) * kFillStep);
+        const unsigned grid = std::max(1u, std::min(blocks_for(n_recs, block_recs), most));
+        (longer ? k_key_fill<true, true> : k_key_fill<true, false>)<<<grid, kFillThreads, nq * sizeof(uint32_t), st>>>(
+            recs, counters, t.slot_key_off.p, t.tile_keys.p, t.keys.p, qoff, qcursor, nq, block_recs, out);
     } else {
         const unsigned grid = std::max(1u, std::min(blocks_for(n_recs, kFillThreads * kFillPerLane), most));
-        k_key_fill<false><<<grid, kFillThreads, 0, st>>>(recs, counters, t.slot_key_off.p, t.tile_keys.p, t.keys.p, qoff,
-                                                         qcursor, nq, out);
+        (longer ? k_key_fill<false, true> : k_key_fill<false, false>)<<<grid, kFillThreads, 0, st>>>(
+            recs, counters, t.slot_key_off.p, t.tile_keys.p, t.keys.p, qoff, qcursor, nq, 0, out);
     }
     TM_CHECK_LAUNCH();
 }

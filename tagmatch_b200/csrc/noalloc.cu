@@ -204,7 +204,7 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
         *n_keys = total;
         if (total > capacity)
             throw Error(TM_ERR_CAPACITY, "output key buffer too small: " + std::to_string(total) + " keys needed");
-        launch_key_fill(t, recs, counters, hc[1], d_out_offsets, qcursor, nq, d_out_keys, sms, st);
+        launch_key_fill(t, recs, counters, hc[1], total, d_out_offsets, qcursor, nq, d_out_keys, sms, st);
         TM_CUDA(cudaStreamSynchronize(st));
         return;
     }
@@ -221,7 +221,7 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     const size_t second_bytes = bitmap ? bitmap_bytes : key_bytes;
     uint32_t *second = second_bytes <= rec_bytes ? reinterpret_cast<uint32_t *>(recs)
                                                  : ar.take<uint32_t>(second_bytes / sizeof(uint32_t), "match_unique keys");
-    launch_key_fill(t, recs, counters, hc[1], qoff, qcursor, nq, keys, sms, st);
+    launch_key_fill(t, recs, counters, hc[1], total, qoff, qcursor, nq, keys, sms, st);
     if (bitmap) {
         launch_unique_mark(keys, qoff, nq, words, second, ucount, sms, st);
     } else {
