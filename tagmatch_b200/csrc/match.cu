@@ -148,6 +148,12 @@ constexpr size_t kQueueAheadBytes = size_t(256) << 20;
 // partitions, twice.
 constexpr size_t kRowWords = size_t(64) << 18;
 
+size_t free_device_bytes() {
+    size_t free_bytes = 0, all_bytes = 0;
+    TM_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes));
+    return free_bytes;
+}
+
 static_assert(sizeof(HitRec) == kRecordBytes, "the record buffer is sized in records");
 
 MatchScratch::~MatchScratch() {
@@ -250,11 +256,7 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     // route, queues (both again per window), plan, match, scan, readback
     bs.launches += windows * (windows > 1 ? 3 : 2) + 3 + scan_launches(nq) + (ahead ? 0u : 1u);
     // ---- match (regrow and re-run on pair overflow) ----
-    reserve_records(s.recs, s.rec_history, nq, t.n_tiles, s.budget, [] {
-        size_t free_bytes = 0, all_bytes = 0;
-        TM_CUDA(cudaMemGetInfo(&free_bytes, &all_bytes));
-        return free_bytes;
-    });
+    reserve_records(s.recs, s.rec_history, nq, t.n_tiles, s.budget, free_device_bytes);
     unsigned long long hc[4] = {0, 0, 0, 0};
     uint64_t total = 0;
     for (int attempt = 0;; ++attempt) {
@@ -340,11 +342,11 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     s.uoff.reserve(size_t(nq) + 1);
     const uint32_t words = (t.max_key >> 5) + 1;
     const size_t bitmap_words = size_t(nq) * bitmap_stride(words);
-    const bool bitmaps = unique_by_bitmap(t.max_key) && bitmaps_allowed(bitmap_words * 4, total * 4, s.budget) &&
-                         reserve_bitmaps(s.ukeys, bitmap_words, s.bitmaps_refused);
+    const bool bitmaps = unique_by_bitmap(t.max_key, nq, total) && bitmaps_allowed(bitmap_words * 4, total * 4, s.budget) &&
+                         reserve_bitmaps(s.ukeys, bitmap_words, s.bitmaps_refused, free_device_bytes);
     bs.key_bytes += bitmaps ? bitmap_words * 4 : total * 4;
     if (bitmaps) {
-        launch_unique_mark(s.keys.p, s.qoff.p, nq, words, s.ukeys.p, s.ucount.p, s.sm_count, st);
+        launch_unique_mark(s.keys.p, s.qoff.p, nq, total, words, s.ukeys.p, s.ucount.p, s.sm_count, st);
         exclusive_scan<uint32_t, uint64_t>(s.ucount.p, s.uoff.p, nq, s.scr, st);
         launch_unique_expand(s.ukeys.p, s.uoff.p, nq, words, s.keys.p, st);
         bs.launches += 3 + scan_launches(nq);  // mark, expand, readback, scan

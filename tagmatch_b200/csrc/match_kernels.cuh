@@ -1072,9 +1072,9 @@ inline void launch_key_fill(const DevTable &t, const HitRec *recs, const unsigne
 // match_unique
 // ---------------------------------------------------------------------------
 // Two routes.  Keys of a small space [0, 32 * words) are marked in a bitmap
-// per query, which is then read out in order; others are sorted.
+// per query, which is then read out in order; others, and few keys in a space
+// that is not so small, are sorted.
 constexpr uint32_t kBitmapMaxWords = 12288;  // 48 KB of shared memory
-constexpr int kExpandThreads = 256;
 
 // Words between two queries' bitmaps (16-byte rows).
 __host__ __device__ inline uint32_t bitmap_stride(uint32_t words) { return (words + 3u) & ~3u; }
@@ -1142,16 +1142,17 @@ __global__ void __launch_bounds__(1024) k_unique_mark(const uint32_t *__restrict
 }
 
 // Reads a query's bitmap out in order into its place of the result (one CTA
-// per query).  Warp w takes words [w * per, (w + 1) * per), 64 at a time,
+// per query, of as many warps as the bitmap has rounds, eight at most).  Warp w
+// takes words [w * per, (w + 1) * per), 64 at a time,
 // two per lane: a prefix sum over the lanes' popcounts places each lane's
 // keys in a per-warp buffer (11-bit positions in the round's 2,048), which
 // the warp then writes out 32 consecutive keys per store.
-__global__ void __launch_bounds__(kExpandThreads) k_unique_expand(const uint32_t *__restrict__ bitmaps,
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) k_unique_expand(const uint32_t *__restrict__ bitmaps,
                                                                   const uint64_t *__restrict__ uoff, uint32_t words,
                                                                   uint32_t *__restrict__ out) {
-    constexpr int kWarps = kExpandThreads / 32;
-    __shared__ uint16_t s_stage[kWarps][2048];
-    __shared__ uint32_t s_sum[kWarps];
+    __shared__ uint16_t s_stage[WARPS][2048];
+    __shared__ uint32_t s_sum[WARPS];
     const uint32_t q = blockIdx.x;
     const uint64_t o = uoff[q];
     if (uoff[q + 1] == o) return;
@@ -1159,7 +1160,7 @@ __global__ void __launch_bounds__(kExpandThreads) k_unique_expand(const uint32_t
     const uint32_t rows = bitmap_stride(words) >> 1;
     const uint2 *bm = reinterpret_cast<const uint2 *>(bitmaps) + size_t(q) * rows;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t per = ((rows + kWarps - 1) / kWarps + 31) & ~31u;
+    const uint32_t per = ((rows + WARPS - 1) / WARPS + 31) & ~31u;
     const uint32_t r0 = min(rows, warp * per), r1 = min(rows, r0 + per);
     uint32_t c = 0;
     for (uint32_t r = r0 + lane; r < r1; r += 32) {
@@ -1171,7 +1172,7 @@ __global__ void __launch_bounds__(kExpandThreads) k_unique_expand(const uint32_t
     __syncthreads();
     uint32_t *d = out + o;
 #pragma unroll
-    for (int k = 0; k < kWarps; ++k)
+    for (int k = 0; k < WARPS; ++k)
         if (k < int(warp)) d += s_sum[k];
     uint16_t *stage = s_stage[warp];
     for (uint32_t r = r0; r < r1; r += 32) {
@@ -1313,6 +1314,21 @@ __device__ __forceinline__ void sort_query(uint32_t *keys, uint64_t b, uint32_t 
     if (tid == 0) *ucount = total;
 }
 
+// At most 32 keys, one per lane of a warp: each different key's place is the
+// number of different keys below it (140,000 queries of 2 keys: 397 us a call,
+// 955 with the block's passes over 16-bit keys).
+__device__ __forceinline__ void sort_few(const uint32_t *keys, uint32_t n, uint32_t *ukeys, uint32_t *ucount, unsigned lane) {
+    const uint32_t k = lane < n ? keys[lane] : 0u;
+    const uint32_t live = __ballot_sync(kFull, lane < n);
+    const uint32_t same = __match_any_sync(kFull, k) & live;
+    const bool first = lane < n && lane == (unsigned)__ffs(same) - 1u;
+    const uint32_t firsts = __ballot_sync(kFull, first);
+    uint32_t at = 0;
+    for (uint32_t m = firsts; m; m &= m - 1) at += __shfl_sync(kFull, k, __ffs(m) - 1) < k ? 1u : 0u;
+    if (first) ukeys[at] = k;
+    if (lane == 0) *ucount = __popc(firsts);
+}
+
 // long_list: [0] number of long queries (zeroed by the caller), [1 ..] the queries.
 __global__ void k_long_list(const uint64_t *__restrict__ qoff, uint32_t nq, uint32_t *__restrict__ long_list) {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1325,8 +1341,8 @@ __global__ void __launch_bounds__(kSortSmallThreads) k_unique_sort(uint32_t *key
     const uint32_t q = blockIdx.x;
     const uint64_t b = qoff[q], n = qoff[q + 1] - b;  // a query's keys are counted in 32 bits
     if (n > kSortSmallKeys) return;
-    if (n == 0) {
-        if (threadIdx.x == 0) ucount[q] = 0;
+    if (n <= 32) {
+        if (threadIdx.x < 32) sort_few(keys + b, uint32_t(n), ukeys + b, &ucount[q], threadIdx.x);
         return;
     }
     sort_query<kSortSmallThreads, kSortSmallKeys>(keys, b, uint32_t(n), ukeys, &ucount[q], key_bits);
@@ -1361,21 +1377,44 @@ __global__ void k_compact(const uint32_t *__restrict__ ukeys, const uint64_t *__
     for (; i < n; i += blockDim.x) out[dst + i] = ukeys[src + i];
 }
 
-// Whether match_unique marks bitmaps: the key space fits one.
-inline bool unique_by_bitmap(uint32_t max_key) { return (max_key >> 5) + 1 <= kBitmapMaxWords; }
+// Whether match_unique marks bitmaps: the key space fits one, and what they
+// move is worth it.  A bitmap's way out and back costs by its words, sorting
+// by the keys, and a warp's sort of up to 32 keys next to nothing.  Calls of
+// 20,000 queries (us, bitmaps and sorted): 2 keys each in 256 words 148 and
+// 160, in 1,024 194 and 159, in 2,048 228 and 158; 50 keys in 1,024 228 and
+// 261; 100 in 2,048 302 and 286, 200 313 and 324; 500 in 4,096 480 and 497;
+// 500 in 6,250 606 and 495, 1,000 682 and 735; 1,000 in 10,938 941 and 742,
+// 2,000 1,080 and 1,210.  Bitmaps of up to 32 MB stay in L2: 2,000 queries
+// of 50 keys in 2,048 words 113 and 117.
+inline bool unique_by_bitmap(uint32_t max_key, uint32_t nq, uint64_t keys) {
+    const uint64_t words = (max_key >> 5) + 1, all_words = nq * words;
+    if (words > kBitmapMaxWords) return false;
+    if (words < 1024 || all_words < (uint64_t(8) << 20)) return true;
+    if (keys <= uint64_t(nq) * 32) return false;
+    return words < 2048 || keys * (words < 4096 ? 20 : 8) >= all_words;
+}
 
-inline void launch_unique_mark(const uint32_t *keys, const uint64_t *qoff, uint32_t nq, uint32_t words, uint32_t *bitmaps,
-                               uint32_t *ucount, int sm_count, cudaStream_t st) {
+inline void launch_unique_mark(const uint32_t *keys, const uint64_t *qoff, uint32_t nq, uint64_t n_keys, uint32_t words,
+                               uint32_t *bitmaps, uint32_t *ucount, int sm_count, cudaStream_t st) {
     // the bitmap and the count may together exceed the default 48 KB
     TM_CUDA(cudaFuncSetAttribute(k_unique_mark, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBitmapMaxWords * 4)));
-    const unsigned threads = nq <= 4u * unsigned(sm_count) ? 1024 : 256;
+    // no more threads than have four stores of the bitmap's words or two
+    // loads of four keys each to make (140,000 queries of 100 keys in 32 words,
+    // with the read-out's: 669 us a call with 256 and eight warps, 320 so)
+    unsigned threads = nq <= 4u * unsigned(sm_count) ? 1024 : 256;
+    const uint64_t busy = std::max<uint64_t>(bitmap_stride(words) / 16, n_keys / nq / 8);
+    while (threads > 32 && threads / 2 >= busy) threads /= 2;
     k_unique_mark<<<nq, threads, bitmap_stride(words) * 4, st>>>(keys, qoff, words, bitmaps, ucount);
     TM_CHECK_LAUNCH();
 }
 
 inline void launch_unique_expand(const uint32_t *bitmaps, const uint64_t *uoff, uint32_t nq, uint32_t words, uint32_t *out,
                                  cudaStream_t st) {
-    k_unique_expand<<<nq, kExpandThreads, 0, st>>>(bitmaps, uoff, words, out);
+    // a warp for each round of 64 words
+    if (words > 256) k_unique_expand<8><<<nq, 256, 0, st>>>(bitmaps, uoff, words, out);
+    else if (words > 128) k_unique_expand<4><<<nq, 128, 0, st>>>(bitmaps, uoff, words, out);
+    else if (words > 64) k_unique_expand<2><<<nq, 64, 0, st>>>(bitmaps, uoff, words, out);
+    else k_unique_expand<1><<<nq, 32, 0, st>>>(bitmaps, uoff, words, out);
     TM_CHECK_LAUNCH();
 }
 

@@ -217,13 +217,13 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     const uint32_t words = (t.max_key >> 5) + 1;
     const size_t bitmap_bytes = size_t(nq) * bitmap_stride(words) * sizeof(uint32_t);
     const size_t key_bytes = std::max<uint64_t>(total, 1) * sizeof(uint32_t), rec_bytes = hc[1] * sizeof(HitRec);
-    const bool bitmap = unique_by_bitmap(t.max_key) && bitmap_bytes <= std::max(rec_bytes, ar.left());
+    const bool bitmap = unique_by_bitmap(t.max_key, nq, total) && bitmap_bytes <= std::max(rec_bytes, ar.left());
     const size_t second_bytes = bitmap ? bitmap_bytes : key_bytes;
     uint32_t *second = second_bytes <= rec_bytes ? reinterpret_cast<uint32_t *>(recs)
                                                  : ar.take<uint32_t>(second_bytes / sizeof(uint32_t), "match_unique keys");
     launch_key_fill(t, recs, counters, hc[1], total, qoff, qcursor, nq, keys, sms, st);
     if (bitmap) {
-        launch_unique_mark(keys, qoff, nq, words, second, ucount, sms, st);
+        launch_unique_mark(keys, qoff, nq, total, words, second, ucount, sms, st);
     } else {
         launch_unique_sort(keys, qoff, nq, second, ucount, reinterpret_cast<uint32_t *>(d_out_offsets), t.max_key, sms, st);
     }

@@ -82,23 +82,24 @@ void reserve_records(Buf &recs, RecordHistory &h, uint32_t nq, uint32_t n_tiles,
     recs.reserve(least);
 }
 
-// Whether match_unique's bitmaps may take their memory: up to 1 GiB without a
-// question, beyond that at most twice what the batch's keys take (many queries
-// with a few keys each are sorted instead, which needs no more than the keys),
-// and under a budget never more than its share or than sorting would take.
-constexpr size_t kBitmapBytesAnyway = size_t(1) << 30;
+// Whether a budget allows match_unique's bitmaps: never more than its share, or
+// than sorting, which takes a second buffer for the keys, would take.
 constexpr bool bitmaps_allowed(size_t bitmap_bytes, size_t key_bytes, size_t budget) {
-    return bitmap_bytes <= std::max(kBitmapBytesAnyway, 2 * key_bytes) &&
-           bitmap_bytes <= std::max(key_bytes, budget_share(budget, kBitmapBudgetShare));
+    return bitmap_bytes <= std::max(key_bytes, budget_share(budget, kBitmapBudgetShare));
 }
 
-// Makes room for match_unique's bitmaps; false when there is none.  The size
-// that was refused is not tried again (refused: kept beside the buffer).
-template <class Buf>
-bool reserve_bitmaps(Buf &buf, size_t words, size_t &refused) {
+// Makes room for match_unique's bitmaps (words of 4 bytes); false when there is
+// none: they may take 1 GiB, or a share of the free memory, and sorting does
+// without.  A size that was refused is not tried again (refused: kept beside
+// the buffer).
+constexpr size_t kBitmapBytesAnyway = size_t(1) << 30;
+template <class Buf, class FreeBytes>
+bool reserve_bitmaps(Buf &buf, size_t words, size_t &refused, FreeBytes free_bytes) {
     if (buf.p && words <= buf.cap) return true;
     if (words >= refused) return false;
-    if (buf.try_reserve(words)) return true;
+    const size_t held = buf.p ? buf.cap : 0;
+    if ((words * 4 <= kBitmapBytesAnyway || words * 4 <= (free_bytes() + held * 4) / kGuessShare) && buf.try_reserve(words))
+        return true;
     refused = words;
     return false;
 }

@@ -112,21 +112,36 @@ int main() {
         batch(b, h, n, tiles, size_t(n) * 5000, nullptr, budget);
         CHECK(b.cap >= size_t(n) * 5000);
         // bitmaps: a quarter of the budget, or what sorting would take
-        CHECK(tmb::bitmaps_allowed(budget / 4, 0, budget) == (budget / 4 <= GiB));
+        CHECK(tmb::bitmaps_allowed(budget / 4, 0, budget));
         CHECK(!tmb::bitmaps_allowed(budget / 4 + 1, 0, budget));
         CHECK(tmb::bitmaps_allowed(budget / 4 + 1, budget / 4 + 1, budget));
     }
-    CHECK(tmb::bitmaps_allowed(GiB, 0, 0) && !tmb::bitmaps_allowed(GiB + 1, 0, 0) && tmb::bitmaps_allowed(3 * GiB, 3 * GiB / 2, 0));
+    CHECK(tmb::bitmaps_allowed(100 * GiB, 0, 0));
     {   // refused bitmaps are not asked for again, smaller ones are
         Device dev{GiB};
         Buf b{dev, 4};
         size_t refused = ~size_t(0);
+        auto free_bytes = [&] { return dev.free_bytes; };
         for (int i = 0; i < 5; ++i) {
-            CHECK(!tmb::reserve_bitmaps(b, GiB / 2, refused));
+            CHECK(!tmb::reserve_bitmaps(b, GiB / 4 + 1, refused, free_bytes));  // by the share
             b.reserve(1000);  // the sorting route's buffer
         }
-        CHECK(dev.refusals == 1 && dev.allocations == 1);
-        CHECK(tmb::reserve_bitmaps(b, GiB / 8, refused) && tmb::reserve_bitmaps(b, GiB / 8, refused) && dev.allocations == 2);
+        CHECK(dev.refusals == 0 && dev.allocations == 1);
+        dev.free_bytes -= GiB / 2;
+        for (int i = 0; i < 5; ++i) {
+            CHECK(!tmb::reserve_bitmaps(b, GiB / 4, refused, free_bytes));  // by the allocator
+            b.reserve(1000);
+        }
+        CHECK(dev.refusals == 1 && dev.allocations == 2);
+        CHECK(tmb::reserve_bitmaps(b, GiB / 16, refused, free_bytes) && tmb::reserve_bitmaps(b, GiB / 16, refused, free_bytes));
+        CHECK(dev.allocations == 3);
+    }
+    {   // more than 1 GiB where the device has it
+        Device dev{170 * GiB};
+        Buf b{dev, 4};
+        size_t refused = ~size_t(0);
+        CHECK(tmb::reserve_bitmaps(b, 5 * GiB, refused, [&] { return dev.free_bytes; }) && b.cap == 5 * GiB);
+        CHECK(!tmb::reserve_bitmaps(b, 6 * GiB, refused, [&] { return dev.free_bytes; }) && b.cap == 5 * GiB);
     }
     std::puts("ok");
 }

@@ -44,15 +44,17 @@ def _check(lists, q, want):
             assert np.array_equal(out[: keys.size].view(np.uint32), keys) and (out[keys.size:] == -1).all()
 
 
-@pytest.mark.parametrize("nq", [1, 1300, 1350, 1358, 1360, 1362, 1363, 1364, 1365, 1366, 1500, 4096])
+@pytest.mark.parametrize("nq", [1, 682, 683, 1100, 1130, 1138, 1140, 1141, 1142, 1143, 1144, 1146, 1150, 1300, 1500])
 def test_bitmaps_larger_than_the_array(nq):
-    """Key space 393,216: bitmaps of 48 KB, of which the array holds 1,365 and
-    less than that beside the rest of the call's scratch."""
-    a, b = np.array([0, 70_000, 393_215], dtype=np.uint32), np.array([5, 70_000, 393_214], dtype=np.uint32)
+    """Key space 393,216 and 1,600 or 3,190 keys per query: bitmaps of 48 KB, of
+    which the array holds some 1,200 beside the keys and the rest."""
+    rng = np.random.default_rng(7)
+    a, b = (np.unique(np.concatenate([rng.choice(393_216, size=1600, replace=False), e])).astype(np.uint32)
+            for e in ([0, 393_215], [5, 70_000]))
     q = np.tile(filter_from_bits([3, 4, 5]), (nq, 1))
     q[1::2] = filter_from_bits([3])
     q[5::100] = 0
-    both = np.array([0, 5, 70_000, 393_214, 393_215], dtype=np.uint32)
+    both = np.union1d(a, b)
     want = [np.zeros(0, np.uint32) if i % 100 == 5 else a if i & 1 else both for i in range(nq)]
     _check([(filter_from_bits([3]), a), (filter_from_bits([3, 4]), b)], q, want)
 
