@@ -85,6 +85,8 @@ MatchScratch &MatchScratch::operator=(MatchScratch &&o) noexcept {
     sm_count = o.sm_count;
     rec_history = o.rec_history;
     bitmaps_refused = o.bitmaps_refused;
+    ahead_refused = o.ahead_refused;
+    row_words = o.row_words;
     seg_tiles = o.seg_tiles;
     seg_exact = o.seg_exact;
     budget = o.budget;
@@ -144,9 +146,6 @@ const uint32_t *read_back(MatchScratch &s, const void *a, uint32_t na, const voi
 // and the wait saved (it is paid by small batches: about 10 us of 180 for
 // one query).
 constexpr size_t kQueueAheadBytes = size_t(256) << 20;
-// Largest routing matrix kept at once; larger ones are made in windows of
-// partitions, twice.
-constexpr size_t kRowWords = size_t(64) << 18;
 
 size_t free_device_bytes() {
     size_t free_bytes = 0, all_bytes = 0;
@@ -191,8 +190,13 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
     unsigned long long *counters = reinterpret_cast<unsigned long long *>(s.zeroed.p);
     uint32_t *qkeys = s.zeroed.p + 8, *qcursor = qkeys + nq, *part_count = qcursor + nq, *group_count = part_count + P;
     TM_CUDA(cudaMemsetAsync(s.zeroed.p, 0, n_zero * sizeof(uint32_t), st));
-    const uint32_t window = route_window(P, nq, kRowWords), windows = (P + window - 1) / window;
+    uint32_t window = route_window(P, nq, s.row_words);
+    while (window > 32 && !s.rows.try_reserve(size_t(window) * route_row_words(nq))) {
+        s.row_words /= 2;  // smaller windows where the device is short of memory
+        window = route_window(P, nq, s.row_words);
+    }
     s.rows.reserve(size_t(window) * route_row_words(nq));
+    const uint32_t windows = (P + window - 1) / window;
     for (uint32_t p0 = 0; p0 < P; p0 += window)
         launch_route(true, d_queries, nq, t, p0, std::min(P, p0 + window), s.rows.p, part_count, group_count, st);
     // ---- plan: queue positions, chunks and work items ----
@@ -241,8 +245,10 @@ void match_batch(const DevTable &t, const uint32_t *d_queries, uint32_t nq, bool
         bs.items = items;
     };
     size_t queue_len = size_t(nq) * P, slice_len = size_t(P) * blocks_for(nq, kChunk);
-    const bool ahead = !s.record_items && queue_len * kQueueWords * 4 + slice_len * kSliceWords * 4 <=
-                                              std::min(kQueueAheadBytes, budget_share(s.budget, kQueueBudgetShare));
+    const bool ahead = !s.record_items &&
+                       reserve_ahead(s.queue, queue_len * 2, s.slices, slice_len * kSliceWords,
+                                     queue_len * kQueueWords * 4 + slice_len * kSliceWords * 4,
+                                     std::min(kQueueAheadBytes, budget_share(s.budget, kQueueBudgetShare)), s.ahead_refused);
     if (!ahead) {
         host_plan(read_back(s, part_count, P, nullptr, 0, nullptr, 0, st));
         queue_len = bs.routed;

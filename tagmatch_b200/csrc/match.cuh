@@ -7,6 +7,10 @@
 
 namespace tmb {
 
+// Largest routing matrix kept at once; larger ones are made in windows of
+// partitions, twice.
+constexpr size_t kRowWords = size_t(64) << 18;
+
 constexpr int kSegTiles = 128;  // default tiles per work item (tm_autotune may change it)
 
 // Device scratch for one in-flight batch (grow-only).
@@ -45,7 +49,10 @@ struct MatchScratch {
     ScanScratch scr;
     int sm_count = 0;
     RecordHistory rec_history;
-    size_t bitmaps_refused = ~size_t(0);  // words of match_unique bitmaps that were not to be had
+    // sizes that were not to be had: words of match_unique's bitmaps, bytes of
+    // queues by their bound; and the words that the routing rows may take
+    size_t bitmaps_refused = ~size_t(0), ahead_refused = ~size_t(0);
+    size_t row_words = kRowWords;
     uint32_t seg_tiles = kSegTiles;  // tiles per work item
     bool seg_exact = false;          // seg_tiles as it is, however few items that makes
     size_t budget = 0;               // bytes that a batch's buffers are to stay within (0: not bounded)

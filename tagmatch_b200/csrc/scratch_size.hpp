@@ -82,6 +82,19 @@ void reserve_records(Buf &recs, RecordHistory &h, uint32_t nq, uint32_t n_tiles,
     recs.reserve(least);
 }
 
+// Makes the queues and slices ready by their bound, which saves the wait for
+// their exact sizes: when that takes no more than `limit` bytes and can be had.
+// False: they are to be made by their exact sizes, which may fit where the
+// bound does not.  A refused size is not tried again.
+template <class Queue, class Slices>
+bool reserve_ahead(Queue &queue, size_t queue_len, Slices &slices, size_t slice_len, size_t bytes, size_t limit, size_t &refused) {
+    if (bytes > limit || bytes >= refused) return false;
+    if (queue.try_reserve(queue_len) && slices.try_reserve(slice_len)) return true;
+    queue.release();  // what it got would be missing beside
+    refused = bytes;
+    return false;
+}
+
 // Whether a budget allows match_unique's bitmaps: never more than its share, or
 // than sorting, which takes a second buffer for the keys, would take.
 constexpr bool bitmaps_allowed(size_t bitmap_bytes, size_t key_bytes, size_t budget) {

@@ -24,9 +24,7 @@ struct Buf {
     bool try_reserve(size_t n) {
         if (p && n <= cap) return true;
         if (p) n = std::max(n, cap + cap / 2);
-        dev.free_bytes += cap * element;
-        p = nullptr;
-        cap = 0;
+        release();
         if (n * element > dev.free_bytes) return ++dev.refusals, false;
         dev.free_bytes -= n * element;
         ++dev.allocations;
@@ -35,6 +33,11 @@ struct Buf {
         return true;
     }
     void reserve(size_t n) { CHECK(try_reserve(n)); }
+    void release() {
+        dev.free_bytes += cap * element;
+        p = nullptr;
+        cap = 0;
+    }
 };
 
 static void batch(Buf &b, tmb::RecordHistory &h, uint32_t nq, uint32_t tiles, uint64_t records, int *runs = nullptr,
@@ -142,6 +145,20 @@ int main() {
         size_t refused = ~size_t(0);
         CHECK(tmb::reserve_bitmaps(b, 5 * GiB, refused, [&] { return dev.free_bytes; }) && b.cap == 5 * GiB);
         CHECK(!tmb::reserve_bitmaps(b, 6 * GiB, refused, [&] { return dev.free_bytes; }) && b.cap == 5 * GiB);
+    }
+    {   // queues by their bound: refused once, then by their exact sizes
+        const size_t MiB = size_t(1) << 20;
+        Device dev{150 * MiB};
+        Buf queue{dev, 16}, slices{dev, 4};
+        size_t refused = ~size_t(0);
+        for (int i = 0; i < 5; ++i) {
+            CHECK(!tmb::reserve_ahead(queue, 8 * MiB, slices, 10 * MiB, 168 * MiB, 256 * MiB, refused));
+            queue.reserve(MiB);
+            slices.reserve(MiB);
+        }
+        CHECK(dev.refusals == 1);
+        CHECK(tmb::reserve_ahead(queue, 4 * MiB, slices, 10 * MiB, 104 * MiB, 256 * MiB, refused));
+        CHECK(!tmb::reserve_ahead(queue, 4 * MiB, slices, 10 * MiB, 104 * MiB, 100 * MiB, refused));
     }
     std::puts("ok");
 }
