@@ -211,8 +211,8 @@ void match_batch_noalloc(const DevTable &t, const uint32_t *d_queries, uint32_t 
     // match_unique: keys into one arena buffer; the bitmaps, or the sorting
     // route's second key buffer, into another (the hit records' space when
     // it is large enough: they are no longer read once the keys are filled).
-    // Bitmaps that fit nowhere leave the sorting route, whose buffer is as
-    // long as the keys.
+    // Bitmaps that fit nowhere, or that few keys make not worth it, leave the
+    // sorting route, whose buffer is as long as the keys.
     uint32_t *keys = ar.take<uint32_t>(std::max<uint64_t>(total, 1), "match_unique keys");
     const uint32_t words = (t.max_key >> 5) + 1;
     const size_t bitmap_bytes = size_t(nq) * bitmap_stride(words) * sizeof(uint32_t);

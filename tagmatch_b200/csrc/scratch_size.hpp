@@ -59,12 +59,12 @@ struct RecordHistory {
 // Makes the record buffer ready for a batch: never smaller than it is (at
 // first kLeastRecords a query and the spare ones), larger where the batch is
 // expected to need it and a share of the free memory, and of the budget,
-// allows.  What was refused once, by that share or by the allocator, is not tried again: every further
-// try would free the buffer that serves, fail, and make the small one again,
-// with the subset test run twice after it (65,536 queries without matches on
-// ten million filters with 3 GiB free: 2,970 us or more for every call, 170
-// since).
-// free_bytes() is asked only when the buffer would grow.
+// allows.  What was refused once, by that share or by the allocator, is not
+// tried again: every further try would free the buffer that serves, fail, and
+// make the small one again, with the subset test run twice after it (65,536
+// queries without matches on ten million filters with 3 GiB free: 2,970 us or
+// more for every call, 170 since).  free_bytes() is asked only when the buffer
+// would grow.
 template <class Buf, class FreeBytes>
 void reserve_records(Buf &recs, RecordHistory &h, uint32_t nq, uint32_t n_tiles, size_t budget, FreeBytes free_bytes) {
     const size_t held = recs.p ? recs.cap : 0;
